@@ -23,7 +23,8 @@ void launch_reset_count(const Dev &d, cudaStream_t st);
 void launch_persson(const Dev &d, cudaStream_t st);
 void launch_flags_from_host(const Dev &d, cudaStream_t st, const int *flags);
 void launch_weno(const Dev &d, cudaStream_t st);
-void launch_weno_warp(const Dev &d, cudaStream_t st);
+void launch_weno_block(const Dev &d, cudaStream_t st);
+cudaError_t set_kernel_limits();
 void launch_weno_commit(const Dev &d, cudaStream_t st);
 void launch_corner(const Dev &d, cudaStream_t st);
 void launch_node(const Dev &d, cudaStream_t st);
@@ -398,7 +399,7 @@ static void enqueue_step_fast(lag2d_handle *h, int itime, const StageRec *rec = 
       cudaMemcpyAsync(rec->vs + slot * rec->np, d.vs, rec->np * sizeof(double), cudaMemcpyDeviceToDevice, h->st);
     }
     run(h, "persson", [&] { launch_reset_count(d, h->st); launch_fast_persson(d, h->st); }, 2);
-    run(h, "weno", [&] { launch_weno_warp(d, h->st); launch_weno_commit(d, h->st); }, 2);
+    run(h, "weno", [&] { launch_weno_block(d, h->st); launch_weno_commit(d, h->st); }, 2);
     if (src_launches(d)) run(h, "src", [&] { src_pass(h, d); });
     run(h, "corner", [&] { corner_pass(h, d); }, corner_launches(h, d));
     run(h, "node", [&] { launch_fast_node(d, h->st); });
@@ -535,6 +536,10 @@ int lag2d_create(const lag2d_mesh *m, const lag2d_config *c, lag2d_handle **out)
   if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess) {
     delete h;
     return fail(LAG2D_ECUDA, "cudaStreamCreate failed");
+  }
+  if (cudaError_t e = set_kernel_limits()) {
+    lag2d_destroy(h);
+    return fail(LAG2D_ECUDA, std::string("kernel attributes: ") + cudaGetErrorString(e));
   }
   const int nq = m->nquad, np = m->npoin;
   // ---- connectivity
@@ -909,7 +914,10 @@ int lag2d_rhs(lag2d_handle *h, int itime, double *rhsel, int *flags) {
   if (flags) {
     CK(cudaMemcpyAsync(h->flags_dev, d.flag, d.ncell * sizeof(int), cudaMemcpyDeviceToDevice, h->st));
   }
-  run(h, "weno", [&] { launch_weno(d, h->st); launch_weno_commit(d, h->st); }, 2);
+  run(h, "weno", [&] {
+    if (ex) launch_weno(d, h->st); else launch_weno_block(d, h->st);
+    launch_weno_commit(d, h->st);
+  }, 2);
   if (ex) {
     run(h, "corner", [&] { launch_tri_corner(d, h->st); launch_corner(d, h->st); }, 1 + (d.ntria > 0));
     run(h, "node", [&] { launch_node(d, h->st); });
@@ -971,7 +979,7 @@ int lag2d_weno_linear(lag2d_handle *h, int transpose, const double *in, double *
   if (r) return r;
   // Persson marks and the reconstruction at the handle's state (not committed)
   run(h, "persson", [&] { launch_reset_count(d, h->st); launch_fast_persson(d, h->st); }, 2);
-  run(h, "weno", [&] { launch_weno_warp(d, h->st); });
+  run(h, "weno", [&] { launch_weno_block(d, h->st); });
   const int cap = std::max(1, std::min(d.nquad, 16384));
   double *vbuf = nullptr, *obuf = nullptr, *wbuf = nullptr;
   int *wslot = nullptr, *overflow = nullptr;
@@ -1211,7 +1219,7 @@ struct AdjWork {
         launch_fast_geom(ds, h->st, 0);
         launch_reset_count(ds, h->st);
         launch_fast_persson(ds, h->st);
-        launch_weno_warp(ds, h->st);
+        launch_weno_block(ds, h->st);
         launch_weno_swap(ds, h->st);
         // stage 1 reads x^n directly: its reverse folds the coordinate adjoints
         // in; the U^n fold waits for the WENO transpose (in the gather)

@@ -615,52 +615,64 @@ __global__ void __launch_bounds__(64) k_weno(Dev d) { b_weno(d, blockIdx.x * blo
 
 // Copy the reconstructions into the stage state once every read of the
 // pre-limit state is done (the reference's unknr copy, WENO.f90:6096).
-__host__ __device__ void b_weno_commit(const Dev &d, int t) {
-  if (stopped(d) || t >= *d.wcount) return;
-  const int iq = d.wlist[t];
-  const int e = iq + d.ntria;
-  if (d.flag[e] != 2) return;
-  for (int q = 0; q < 4; q++)
-    for (int k = 1; k < 6; k++) d.Us[(q * NDEG + k) * d.ncell + e] = d.Uw[(q * 5 + (k - 1)) * d.nquad + iq];
+__global__ void k_weno_commit(Dev d) {
+  if (stopped(d)) return;
+  const int n = 20 * *d.wcount;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int t = i / 20, v = i - 20 * t, q = v / 5, k = v - 5 * q + 1;
+    const int iq = d.wlist[t], e = iq + d.ntria;
+    if (d.flag[e] == 2) d.Us[(q * NDEG + k) * (size_t)d.ncell + e] = d.Uw[v * (size_t)d.nquad + iq];
+  }
 }
-__global__ void k_weno_commit(Dev d) { b_weno_commit(d, blockIdx.x * blockDim.x + threadIdx.x); }
 // Exchange the replaced moments between the state and the reconstruction
 // buffer (the adjoint's reverse stage switches the recorded stage input
 // between its values before and after WENO this way, in place).
 __global__ void k_weno_swap(Dev d) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= *d.wcount) return;
-  const int iq = d.wlist[t];
-  const int e = iq + d.ntria;
-  if (d.flag[e] != 2) return;
-  for (int q = 0; q < 4; q++)
-    for (int k = 1; k < 6; k++) {
-      double *a = d.Us + (q * NDEG + k) * (size_t)d.ncell + e, *b = d.Uw + (q * 5 + (k - 1)) * (size_t)d.nquad + iq;
-      const double v = *a;
-      *a = *b;
-      *b = v;
-    }
+  const int n = 20 * *d.wcount;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int t = i / 20, v = i - 20 * t, q = v / 5, k = v - 5 * q + 1;
+    const int iq = d.wlist[t], e = iq + d.ntria;
+    if (d.flag[e] != 2) continue;
+    double *a = d.Us + (q * NDEG + k) * (size_t)d.ncell + e, *b = d.Uw + v * (size_t)d.nquad + iq;
+    const double x = *a;
+    *a = *b;
+    *b = x;
+  }
 }
 
 // ---------------------------------------------------------------------------
-// The same WENO reconstruction with one warp per troubled quad (the optimised
-// step's version).  The per-item arithmetic is b_weno's; the independent
-// items run on different lanes: the 216 stencil DOFs, the 81 stencil nodes,
-// the 225 stencil quadrature points, the 9 stencil cells' local geometry and
-// L2 projections, the 8 candidate stencils and the 4 faces, with the data
-// between phases in shared memory.  Lane 0 combines the faces in order and
-// writes the result.  Blocks of one warp loop over the troubled list.
+// The same WENO reconstruction with one block per troubled quad (the optimised
+// step's version).  A stage of a blast has tens of troubled quads, so the
+// kernel's time is the time of one quad: what bounds it is the length of the
+// dependent chain, not bandwidth or arithmetic.  Every sum, 5x5 entry and
+// 5x5 inverse of the reconstruction is therefore a thread's item of its own
+// (216 stencil DOFs, 225 quadrature points, 480 sums over 25 points, 10 and 8
+// inverses held in registers), with the data between phases in shared memory.
+// Sums that do not depend on the candidate stencil are taken once per stencil
+// cell: the mean and derivative rows of the target's basis serve all
+// candidates that contain the cell, and the derivative rows' right-hand sides
+// come from the cell's own mass matrix.  The physical mass centres of the nine
+// cells and the target's frame are computed here, for these cells only.
+// Sedov 128^2, 40 troubled quads a stage: 430 us a launch with one warp
+// per quad and one lane per stencil cell, 27 us this way.
 // ---------------------------------------------------------------------------
+constexpr int kWenoThreads = 256;
 struct WenoShared {
-  double unkrl[9][4][6];
-  double xpqi[9][9][2], xpql[9][9][2], rhogi[9];
-  double rhodj[9][25], xl[9][25], yl[9][25];
+  double unkrl[9][4][6];                    // stencil DOFs, velocities rotated
+  double xpqi[9][9][2], xpql[9][9][2];      // stencil nodes: initial, current rotated
+  double geo[9][5];                         // rc, sc, g19, g20, g21
+  double rhogi[9], mass[9], dxc[9];
+  double rhodj[225], xl[225], yl[225];      // per point s*25 + ig
+  double bq[225][5], bo[225][5], bt[225][5];  // cell basis, local basis, target's local basis
   double geopl[9][5];
-  double unkpl[9][4][6];
-  double mtbbq[25], mtbbi[25];
+  double bb[9][25], bbq[9][25], bbqi[9][25], bbi[25];
+  double rhsl[9][4][6], unkpl[9][4][6];
+  double mrow[9][5], drow[9][2][5], hrow[9][2][5], rh[9][2][4];
+  double mat[8][25], matinv[8][25], rhsls[4][4][5];
   double unksl[9][4][6];
-  double unkf[4][4][6];
-  int fvalid[4];
+  double qinvm[4][16], qmat[4][16], os[4][9], wsum[4][4][6], fch[4][4][6], unkf[4][4][6];
+  double phy[4][6], rhsuk[4][6], out[4][6];
+  int cell[9], fvalid[4];
 };
 
 // The reconstruction's linear factors at a given state, for its adjoint: with
@@ -683,343 +695,471 @@ struct WenoFactors {
   double mp[4];
   int ifprj;
 };
+__constant__ int cIelst1[4][7] = {{1, 2, 5, 6, 9, 8, 3}, {1, 3, 2, 7, 6, 9, 5}, {1, 4, 3, 8, 7, 6, 5}, {1, 5, 4, 9, 8, 7, 3}};
+__constant__ int cIelst2[4][4] = {{1, 2, 6, 9}, {1, 3, 6, 7}, {1, 4, 8, 7}, {1, 5, 8, 9}};
 
+// 5 x 5 inverse, column-major, Gauss-Jordan with partial pivoting (inv_small
+// with every index known at compile time: the matrices stay in registers)
+__device__ __forceinline__ void inv5(const double *a, double *b) {
+  double t[5][5], e[5][5];  // [column][row]
+#pragma unroll
+  for (int j = 0; j < 5; j++)
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+      t[j][i] = a[i + 5 * j];
+      e[j][i] = i == j ? 1.0 : 0.0;
+    }
+#pragma unroll
+  for (int k = 0; k < 5; k++) {
+    int piv = k;
+    double big = fabs(t[k][k]);
+#pragma unroll
+    for (int i = k + 1; i < 5; i++)
+      if (fabs(t[k][i]) > big) { big = fabs(t[k][i]); piv = i; }
+#pragma unroll
+    for (int i = k + 1; i < 5; i++) {
+      const bool sw = piv == i;
+#pragma unroll
+      for (int j = 0; j < 5; j++) {
+        const double x = t[j][k], y = t[j][i];
+        t[j][k] = sw ? y : x;
+        t[j][i] = sw ? x : y;
+        const double u = e[j][k], v = e[j][i];
+        e[j][k] = sw ? v : u;
+        e[j][i] = sw ? u : v;
+      }
+    }
+    const double dd = 1.0 / t[k][k];
+#pragma unroll
+    for (int j = 0; j < 5; j++) { t[j][k] *= dd; e[j][k] *= dd; }
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+      if (i == k) continue;
+      const double f = t[k][i];
+#pragma unroll
+      for (int j = 0; j < 5; j++) {
+        t[j][i] -= f * t[j][k];
+        e[j][i] -= f * e[j][k];
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 5; j++)
+#pragma unroll
+    for (int i = 0; i < 5; i++) b[i + 5 * j] = e[j][i];
+}
+
+// row km (0..8) of Hermite stencil is, moment k (0..4), and its right-hand side
+__device__ __forceinline__ double weno_hrow(const WenoShared &S, int is, int km, int k) {
+  if (km < 3) return S.mrow[cIelst2[is][km + 1] - 1][k];
+  return S.drow[cIelst2[is][(km - 3) / 2 + 1] - 1][(km - 3) & 1][k];
+}
+__device__ __forceinline__ double weno_hrhs(const WenoShared &S, int is, int km, int q) {
+  if (km < 3) return S.unkpl[cIelst2[is][km + 1] - 1][q][0] - S.unkpl[0][q][0];
+  return S.rh[cIelst2[is][(km - 3) / 2 + 1] - 1][(km - 3) & 1][q];
+}
+
+// Reconstructs troubled-list entry t with the whole block; every thread of the
+// block calls it (the early return is block-uniform).  With FACT the factors
+// go to F and nothing is written to the state.
 template <bool FACT>
-__device__ void weno_warp_cell_t(const Dev &d, int t, WenoShared &S, WenoFactors *F) {
-  const int lane = threadIdx.x & 31;
+__device__ bool weno_block_cell(const Dev &d, int t, WenoShared &S, WenoFactors *F) {
+  const int tid = threadIdx.x;
   const int iq = d.wlist[t];
   const int ielem = iq + d.ntria;
-  int ielaj[9];
-  for (int k = 0; k < 9; k++) ielaj[k] = d.stencil[k * d.nquad + iq];
-  if (ielaj[0] == -2 && lane == 0 && !FACT) atomic_or(&d.sc_dev->status, ST_STENCIL);
-  if (ielaj[0] < 0) return;  // boundary cell: the reference leaves it (WENO.f90:7704)
-  const int ielst1[4][7] = {{1, 2, 5, 6, 9, 8, 3}, {1, 3, 2, 7, 6, 9, 5},
-                            {1, 4, 3, 8, 7, 6, 5}, {1, 5, 4, 9, 8, 7, 3}};
-  const int ielst2[4][4] = {{1, 2, 6, 9}, {1, 3, 6, 7}, {1, 4, 8, 7}, {1, 5, 8, 9}};
-  double mp[4];
-  for (int k = 0; k < 4; k++) mp[k] = d.mapmt[k * d.ncell + ielem];
-  const double dxcl = sqrt(d.vol[ielem]), dycl = dxcl;
-
-  // stencil DOFs (velocities rotated to the local frame) and stencil nodes
-  for (int e = lane; e < 216; e += 32) {
-    const int s = e / 24, q = (e / 6) % 4, k = e % 6;
-    S.unkrl[s][q][k] = Uget(d, d.Us, k, q, ielaj[s]);
+  const int first = d.stencil[iq];
+  if (first < 0) {  // boundary cell: the reference leaves it (WENO.f90:7704)
+    if (first == -2 && tid == 0 && !FACT) atomic_or(&d.sc_dev->status, ST_STENCIL);
+    return false;
   }
-  for (int e = lane; e < 81; e += 32) {
-    const int s = e / 9, k = e % 9;
-    const int p = d.ipq[k * d.nquad + (ielaj[s] - d.ntria)];
+  const size_t nc = d.ncell, nq = d.nquad;
+  // the velocity-aligned frame of the target
+  double mp[4] = {0.0, 0.0, 0.0, 0.0};
+  {
+    const double ma = d.Us[6 * nc + ielem], mb = d.Us[12 * nc + ielem];
+    const double nrm = sqrt(ma * ma + mb * mb);
+    if (nrm > 1.0e-10) {
+      mp[0] = ma / nrm;
+      mp[2] = mb / nrm;
+      mp[1] = -mb / nrm;
+      mp[3] = ma / nrm;
+    }
+  }
+  if (tid < 216) {
+    const int s = tid / 24, v = tid - 24 * s;
+    const int je = d.stencil[s * nq + iq];
+    S.unkrl[s][v / 6][v % 6] = d.Us[v * nc + je];
+    if (v == 0) S.cell[s] = je;
+    if (v == 1) S.mass[s] = d.mass[je];
+    if (v == 2) S.dxc[s] = sqrt(d.vol[je]);
+    if (v == 3) { S.geo[s][0] = d.rc[je]; S.geo[s][1] = d.sc[je]; }
+    if (v == 4) { S.geo[s][2] = d.g19[je]; S.geo[s][3] = d.g20[je]; S.geo[s][4] = d.g21[je]; }
+  }
+  if (tid < 81) {
+    const int s = tid / 9, k = tid - 9 * s;
+    const int jq = d.stencil[s * nq + iq] - d.ntria;
+    const int p = d.ipq[k * nq + jq];
     S.xpqi[s][k][0] = d.x0[p];
     S.xpqi[s][k][1] = d.y0[p];
     double x = d.xs[p], y = d.ys[p];
     vec_local(mp, x, y);
     S.xpql[s][k][0] = x;
     S.xpql[s][k][1] = y;
+  } else if (tid >= 96 && tid < 105) {
+    // physical mass centre from the time-invariant mass-weighted shape moments
+    const int s = tid - 96;
+    const int je = d.stencil[s * nq + iq], jq = je - d.ntria;
+    double xmc = 0.0, ymc = 0.0;
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      const int p = d.ipq[k * nq + jq];
+      const double w = d.wmom[k * nq + jq];
+      xmc += w * d.xs[p];
+      ymc += w * d.ys[p];
+    }
+    const double masel = d.mass[je];
+    double xc = xmc / masel, yc = ymc / masel;
+    vec_local(mp, xc, yc);
+    S.geopl[s][0] = xc;
+    S.geopl[s][1] = yc;
+  } else if (tid >= 128 && tid < 132) {
+    // characteristic matrices of the interior faces
+    const int a = tid - 128;
+    const int jelem = d.esq[a * nq + iq];
+    S.fvalid[a] = jelem >= 0;
+    if (jelem >= 0) {
+      const int pa = d.ipq[a * nq + iq], pb = d.ipq[((a + 1) & 3) * nq + iq];
+      const double dtx = d.xs[pb] - d.xs[pa], dty = d.ys[pb] - d.ys[pa];
+      const double dlgt = sqrt(dtx * dtx + dty * dty);
+      double dnx = dty / dlgt, dny = -dtx / dlgt;
+      vec_local(mp, dnx, dny);
+      double ul[4], ur[4];
+      for (int q = 0; q < 4; q++) { ul[q] = d.Us[q * 6 * nc + ielem]; ur[q] = d.Us[q * 6 * nc + jelem]; }
+      vec_local(mp, ul[1], ul[2]);
+      vec_local(mp, ur[1], ur[2]);
+      matrix_prj2(d.gamlg, S.qmat[a], S.qinvm[a], dnx, dny, ul, ur);
+    }
   }
-  __syncwarp();
-  for (int e = lane; e < 54; e += 32) {
-    const int s = e / 6, k = e % 6;
-    vec_local(mp, S.unkrl[s][1][k], S.unkrl[s][2][k]);
+  __syncthreads();
+  if (tid < 54) {
+    vec_local(mp, S.unkrl[tid / 6][1][tid % 6], S.unkrl[tid / 6][2][tid % 6]);
+  } else if (tid >= 64 && tid < 73) {
+    const int s = tid - 64;
+    double shp[9], xc, yc;
+    shp9v(S.geo[s][0], S.geo[s][1], shp);
+    map9(S.xpqi[s], shp, xc, yc);
+    S.rhogi[s] = rho_initial(d, S.cell[s], xc, yc);
   }
-  if (lane < 9) {
-    const int jelem = ielaj[lane];
-    double shp[9], xcrho, ycrho;
-    shp9v(d.rc[jelem], d.sc[jelem], shp);
-    map9(S.xpqi[lane], shp, xcrho, ycrho);
-    S.rhogi[lane] = rho_initial(d, jelem, xcrho, ycrho);
-  }
-  __syncwarp();
+  __syncthreads();
   // quadrature points of the stencil cells (weno_points)
-  for (int e = lane; e < 225; e += 32) {
-    const int s = e / 25, ig = e % 25;
+  if (tid < 225) {
+    const int s = tid / 25, ig = tid - 25 * s;
     const double r = cQ.g25[ig][0], sp = cQ.g25[ig][1], wi = cQ.w25[ig];
     double shp[9], dr[9], ds[9];
     shp9v(r, sp, shp);
     shp9d(r, sp, dr, ds);
-    Jac j = jac9(S.xpqi[s], dr, ds);
-    const double djacoi = wi * (j.xr * j.ys - j.yr * j.xs);
+    const Jac j = jac9(S.xpqi[s], dr, ds);
     double xg, yg;
     map9(S.xpql[s], shp, xg, yg);
-    S.rhodj[s][ig] = S.rhogi[s] * djacoi;
-    S.xl[s][ig] = xg;
-    S.yl[s][ig] = yg;
+    S.rhodj[tid] = S.rhogi[s] * (wi * (j.xr * j.ys - j.yr * j.xs));
+    S.xl[tid] = xg;
+    S.yl[tid] = yg;
+    S.bo[tid][0] = (xg - S.geopl[s][0]) / S.dxc[s];
+    S.bo[tid][1] = (yg - S.geopl[s][1]) / S.dxc[s];
+    const double b1 = r - S.geo[s][0], b2 = sp - S.geo[s][1];
+    S.bq[tid][0] = b1;
+    S.bq[tid][1] = b2;
+    S.bq[tid][2] = 0.5 * b1 * b1 - S.geo[s][2];
+    S.bq[tid][3] = 0.5 * b2 * b2 - S.geo[s][3];
+    S.bq[tid][4] = b1 * b2 - S.geo[s][4];
   }
-  __syncwarp();
-  // getgeophy_local_Taylor, then getunknp_local_Taylor, one stencil cell per lane
-  if (lane < 9) {
-    const int s = lane, jelem = ielaj[s];
-    double xclj = d.geoph[jelem], yclj = d.geoph[d.ncell + jelem];
-    vec_local(mp, xclj, yclj);
-    const double dxclj = sqrt(d.vol[jelem]), dyclj = dxclj;
-    const double masel = d.mass[jelem];
-    double v1 = 0.0, v2 = 0.0, v3 = 0.0;
-    for (int ig = 0; ig < 25; ig++) {
-      double b2 = (S.xl[s][ig] - xclj) / dxclj, b3 = (S.yl[s][ig] - yclj) / dyclj;
-      v1 = v1 + S.rhodj[s][ig] * b2 * b2;
-      v2 = v2 + S.rhodj[s][ig] * b3 * b3;
-      v3 = v3 + S.rhodj[s][ig] * b2 * b3;
-    }
-    v1 = v1 / masel; v2 = v2 / masel; v3 = v3 / masel;
-    double gp[5] = {xclj, yclj, 0.5 * v1, 0.5 * v2, v3};
-    for (int k = 0; k < 5; k++) S.geopl[s][k] = gp[k];
-    const double rcj = d.rc[jelem], scj = d.sc[jelem];
-    double bb[25], bbq[25], bbi[25], bbqi[25];
-    for (int i = 0; i < 25; i++) { bb[i] = 0.0; bbq[i] = 0.0; }
-    for (int ig = 0; ig < 25; ig++) {
-      double r = cQ.g25[ig][0], s_ = cQ.g25[ig][1];
-      double bq[6], bqpl[3], bqol[6];
-      bq[0] = 1.0; bq[1] = (r - rcj) / 1.0; bq[2] = (s_ - scj) / 1.0;
-      bq[3] = 0.5 * bq[1] * bq[1] - d.g19[jelem];
-      bq[4] = 0.5 * bq[2] * bq[2] - d.g20[jelem];
-      bq[5] = bq[1] * bq[2] - d.g21[jelem];
-      bqpl[0] = 1.0; bqpl[1] = (S.xl[s][ig] - xclj) / dxclj; bqpl[2] = (S.yl[s][ig] - yclj) / dyclj;
-      basis_orthg1(bqpl, &gp[2], bqol);
-      for (int i = 1; i < 6; i++)
-        for (int j = 1; j < 6; j++) {
-          bb[(i - 1) + 5 * (j - 1)] = bb[(i - 1) + 5 * (j - 1)] + S.rhodj[s][ig] * bq[i] * bqol[j];
-          bbq[(i - 1) + 5 * (j - 1)] = bbq[(i - 1) + 5 * (j - 1)] + S.rhodj[s][ig] * bqol[i] * bqol[j];
-        }
-    }
-    double rhs[6][4];
-    for (int i = 0; i < 6; i++) for (int q = 0; q < 4; q++) rhs[i][q] = 0.0;
-    for (int i = 1; i < 6; i++)
-      for (int j = 1; j < 6; j++)
-        for (int q = 0; q < 4; q++) rhs[i][q] = rhs[i][q] + S.unkrl[s][q][j] * bb[(j - 1) + 5 * (i - 1)];
-    inv_small(5, bbq, bbqi);
-    inv_small(5, bb, bbi);
-    double up[4][6];
-    for (int q = 0; q < 4; q++) for (int k = 0; k < 6; k++) up[q][k] = 0.0;
-    for (int i = 1; i < 6; i++)
-      for (int j = 1; j < 6; j++)
-        for (int q = 0; q < 4; q++) up[q][i] = up[q][i] + rhs[j][q] * bbqi[(j - 1) + 5 * (i - 1)];
-    for (int q = 0; q < 4; q++) up[q][0] = S.unkrl[s][q][0];
-    for (int q = 0; q < 4; q++) for (int k = 0; k < 6; k++) S.unkpl[s][q][k] = up[q][k];
-    if (s == 0)
-      for (int i = 0; i < 25; i++) { S.mtbbq[i] = bbq[i]; S.mtbbi[i] = bbi[i]; }
-    if (FACT) {
-      // up[i] = sum_m unkrl[m] sum_j bb[(m-1)+5(j-1)] bbqi[(j-1)+5(i-1)]
-      for (int m = 1; m < 6; m++)
-        for (int i = 1; i < 6; i++) {
-          double acc = 0.0;
-          for (int j = 1; j < 6; j++) acc += bb[(m - 1) + 5 * (j - 1)] * bbqi[(j - 1) + 5 * (i - 1)];
-          F->T[s][(m - 1) * 5 + (i - 1)] = acc;
-        }
-    }
+  __syncthreads();
+  // getgeophy_local_Taylor: second moments of each cell about its centre
+  if (tid < 27) {
+    const int s = tid / 3, m = tid - 3 * s;
+    const int i = m == 1 ? 1 : 0, j = m == 0 ? 0 : 1;
+    double v = 0.0;
+#pragma unroll
+    for (int ig = 0; ig < 25; ig++) v += S.rhodj[s * 25 + ig] * S.bo[s * 25 + ig][i] * S.bo[s * 25 + ig][j];
+    v /= S.mass[s];
+    S.geopl[s][2 + m] = m == 2 ? v : 0.5 * v;
   }
-  __syncwarp();
-  // candidate polynomials: 1 central (lane 8) + 4 Lagrangian (lanes 0-3) + 4 Hermite (lanes 4-7)
-  const double xmcl = S.geopl[0][0], ymcl = S.geopl[0][1];
-  if (lane < 9) {
-    const int isten = lane < 8 ? lane + 1 : 0;
-    double us[4][6];
-    for (int q = 0; q < 4; q++) for (int k = 0; k < 6; k++) us[q][k] = 0.0;
-    for (int q = 0; q < 4; q++) us[q][0] = S.unkpl[0][q][0];
-    if (isten == 0) {
-      for (int k = 0; k < 6; k++) for (int q = 0; q < 4; q++) us[q][k] = S.unkpl[0][q][k];
-    } else if (isten <= 4) {
-      const int is = isten - 1;
-      double matlg[25], rhslg[20], matin[25];
-      for (int i = 0; i < 25; i++) matlg[i] = 0.0;
-      for (int i = 0; i < 20; i++) rhslg[i] = 0.0;
-      for (int ies = 0; ies < 5; ies++) {
-        int sl = ielst1[is][ies + 1] - 1;
-        double masej = d.mass[ielaj[sl]];
-        for (int ig = 0; ig < 25; ig++) {
-          double bqplj[3], bqolj[6];
-          bqplj[0] = 1.0; bqplj[1] = (S.xl[sl][ig] - xmcl) / dxcl; bqplj[2] = (S.yl[sl][ig] - ymcl) / dycl;
-          basis_orthg1(bqplj, &S.geopl[0][2], bqolj);
-          for (int k = 0; k < 5; k++) matlg[ies + 5 * k] = matlg[ies + 5 * k] + S.rhodj[sl][ig] * bqolj[k + 1] / masej;
-        }
-        for (int q = 0; q < 4; q++) rhslg[q + 4 * ies] = S.unkpl[sl][q][0] - S.unkpl[0][q][0];
-      }
-      inv_small(5, matlg, matin);
-      if (FACT)
-        for (int i = 0; i < 25; i++) F->matL[is][i] = matin[i];
-      for (int k = 1; k < 6; k++)
-        for (int ies = 0; ies < 5; ies++)
-          for (int q = 0; q < 4; q++) us[q][k] = us[q][k] + matin[(k - 1) + 5 * ies] * rhslg[q + 4 * ies];
+  __syncthreads();
+  if (tid < 225) {
+    const int s = tid / 25;
+    const double b2 = S.bo[tid][0], b3 = S.bo[tid][1];
+    S.bo[tid][2] = 0.5 * b2 * b2 - S.geopl[s][2];
+    S.bo[tid][3] = 0.5 * b3 * b3 - S.geopl[s][3];
+    S.bo[tid][4] = b2 * b3 - S.geopl[s][4];
+    const double t2 = (S.xl[tid] - S.geopl[0][0]) / S.dxc[0], t3 = (S.yl[tid] - S.geopl[0][1]) / S.dxc[0];
+    S.bt[tid][0] = t2;
+    S.bt[tid][1] = t3;
+    S.bt[tid][2] = 0.5 * t2 * t2 - S.geopl[0][2];
+    S.bt[tid][3] = 0.5 * t3 * t3 - S.geopl[0][3];
+    S.bt[tid][4] = t2 * t3 - S.geopl[0][4];
+  }
+  __syncthreads();
+  // sums over the 25 points: bb (225), bbq (135, symmetric), mean rows (40)
+  // and derivative rows (80) of the target's basis on the neighbours
+  for (int it = tid; it < 480; it += kWenoThreads) {
+    int s, i, j;
+    const double *x, *y;
+    if (it < 225) {
+      s = it / 25;
+      i = (it % 25) % 5;
+      j = (it % 25) / 5;
+      x = &S.bq[s * 25][i];
+      y = &S.bo[s * 25][j];
+    } else if (it < 360) {
+      const int e = (it - 225) % 15;
+      s = (it - 225) / 15;
+      j = e < 1 ? 0 : e < 3 ? 1 : e < 6 ? 2 : e < 10 ? 3 : 4;
+      i = e - j * (j + 1) / 2;
+      x = &S.bo[s * 25][i];
+      y = &S.bo[s * 25][j];
+    } else if (it < 400) {
+      s = 1 + (it - 360) / 5;
+      i = (it - 360) % 5;
+      j = 0;
+      x = &S.bt[s * 25][i];
+      y = nullptr;
     } else {
-      const int is = isten - 5;
-      double mathm[45], rhshm[36], matls[25], rhsls[20], matin[25];
-      for (int i = 0; i < 45; i++) mathm[i] = 0.0;
-      for (int i = 0; i < 36; i++) rhshm[i] = 0.0;
-      for (int ies = 0; ies < 3; ies++) {
-        int sl = ielst2[is][ies + 1] - 1;
-        int jelem = ielaj[sl];
-        double masej = d.mass[jelem];
-        double dxclj = sqrt(d.vol[jelem]), dyclj = dxclj;
-        double xclj = S.geopl[sl][0], yclj = S.geopl[sl][1];
-        for (int ig = 0; ig < 25; ig++) {
-          double bqplj[3], bqol[6], bqolj[6];
-          bqplj[0] = 1.0; bqplj[1] = (S.xl[sl][ig] - xmcl) / dxcl; bqplj[2] = (S.yl[sl][ig] - ymcl) / dycl;
-          basis_orthg1(bqplj, &S.geopl[0][2], bqol);
-          for (int k = 0; k < 5; k++) mathm[ies + 9 * k] = mathm[ies + 9 * k] + S.rhodj[sl][ig] * bqol[k + 1] / masej;
-          bqplj[0] = 1.0; bqplj[1] = (S.xl[sl][ig] - xclj) / dxclj; bqplj[2] = (S.yl[sl][ig] - yclj) / dyclj;
-          basis_orthg1(bqplj, &S.geopl[sl][2], bqolj);
-          int ieshm = 3 + 2 * ies;
-          for (int k = 1; k < 6; k++) {
-            mathm[ieshm + 9 * (k - 1)] = mathm[ieshm + 9 * (k - 1)] + S.rhodj[sl][ig] * bqol[k] * bqolj[1] / masej;
-            mathm[ieshm + 1 + 9 * (k - 1)] =
-                mathm[ieshm + 1 + 9 * (k - 1)] + S.rhodj[sl][ig] * bqol[k] * bqolj[2] / masej;
-          }
-          for (int k = 1; k < 6; k++)
-            for (int q = 0; q < 4; q++) {
-              rhshm[q + 4 * ieshm] =
-                  rhshm[q + 4 * ieshm] + S.rhodj[sl][ig] * bqolj[k] * bqolj[1] * S.unkpl[sl][q][k] / masej;
-              rhshm[q + 4 * (ieshm + 1)] =
-                  rhshm[q + 4 * (ieshm + 1)] + S.rhodj[sl][ig] * bqolj[k] * bqolj[2] * S.unkpl[sl][q][k] / masej;
-            }
-          if (FACT)
-            for (int k = 1; k < 6; k++) {
-              F->H[is][ies][0][k - 1] = (ig == 0 ? 0.0 : F->H[is][ies][0][k - 1]) +
-                                        S.rhodj[sl][ig] * bqolj[k] * bqolj[1] / masej;
-              F->H[is][ies][1][k - 1] = (ig == 0 ? 0.0 : F->H[is][ies][1][k - 1]) +
-                                        S.rhodj[sl][ig] * bqolj[k] * bqolj[2] / masej;
-            }
-        }
-        for (int q = 0; q < 4; q++) rhshm[q + 4 * ies] = S.unkpl[sl][q][0] - S.unkpl[0][q][0];
-      }
-      for (int i = 0; i < 25; i++) matls[i] = 0.0;
-      for (int i = 0; i < 20; i++) rhsls[i] = 0.0;
-      for (int im = 0; im < 5; im++)
-        for (int jm = 0; jm < 5; jm++)
-          for (int km = 0; km < 9; km++) matls[im + 5 * jm] = matls[im + 5 * jm] + mathm[km + 9 * im] * mathm[km + 9 * jm];
-      for (int q = 0; q < 4; q++)
-        for (int im = 0; im < 5; im++)
-          for (int km = 0; km < 9; km++) rhsls[q + 4 * im] = rhsls[q + 4 * im] + mathm[km + 9 * im] * rhshm[q + 4 * km];
-      inv_small(5, matls, matin);
-      if (FACT)
-        for (int k = 1; k < 6; k++)
-          for (int km = 0; km < 9; km++) {
-            double acc = 0.0;
-            for (int im = 0; im < 5; im++) acc += matin[(k - 1) + 5 * im] * mathm[km + 9 * im];
-            F->G[is][k - 1][km] = acc;
-          }
-      for (int k = 1; k < 6; k++)
-        for (int ies = 0; ies < 5; ies++)
-          for (int q = 0; q < 4; q++) us[q][k] = us[q][k] + matin[(k - 1) + 5 * ies] * rhsls[q + 4 * ies];
+      const int e = (it - 400) % 10;
+      s = 1 + (it - 400) / 10;
+      i = e % 5;
+      j = e / 5;
+      x = &S.bt[s * 25][i];
+      y = &S.bo[s * 25][j];
     }
-    for (int q = 0; q < 4; q++) for (int k = 0; k < 6; k++) S.unksl[isten][q][k] = us[q][k];
+    double acc = 0.0;
+    if (y) {
+#pragma unroll 5
+      for (int ig = 0; ig < 25; ig++) acc += S.rhodj[s * 25 + ig] * x[5 * ig] * y[5 * ig];
+    } else {
+#pragma unroll 5
+      for (int ig = 0; ig < 25; ig++) acc += S.rhodj[s * 25 + ig] * x[5 * ig];
+    }
+    if (it < 225) S.bb[s][i + 5 * j] = acc;
+    else if (it < 360) { S.bbq[s][i + 5 * j] = acc; S.bbq[s][j + 5 * i] = acc; }
+    else if (it < 400) S.mrow[s][i] = acc / S.mass[s];
+    else S.drow[s][j][i] = acc / S.mass[s];
   }
-  __syncwarp();
-  // weno_cell_Taylor: characteristic WENO per interior face (lanes 0-3)
-  const int isten = 9;
-  const double epsil = 1.0e-6;
-  const double dxc = sqrt(d.vol[ielem]), dyc = dxc;
-  if (lane < 4) {
-    const int ies = lane;
-    const int mapfe[4][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}};
-    const int jelem = d.esq[ies * d.nquad + iq];
-    S.fvalid[ies] = jelem >= 0;
-    if (jelem >= 0) {
-      const int pa = d.ipq[mapfe[ies][0] * d.nquad + iq], pb = d.ipq[mapfe[ies][1] * d.nquad + iq];
-      double dtx = d.xs[pb] - d.xs[pa];
-      double dty = d.ys[pb] - d.ys[pa];
-      double dlgt = sqrt(dtx * dtx + dty * dty);
-      double dnx = dty / dlgt, dny = -dtx / dlgt;
-      vec_local(mp, dnx, dny);
-      double ul[4], ur[4];
-      for (int q = 0; q < 4; q++) { ul[q] = Uget(d, d.Us, 0, q, ielem); ur[q] = Uget(d, d.Us, 0, q, jelem); }
-      vec_local(mp, ul[1], ul[2]);
-      vec_local(mp, ur[1], ur[2]);
-      double qmat[16], qinvm[16];
-      matrix_prj2(d.gamlg, qmat, qinvm, dnx, dny, ul, ur);
-      double weigh[9][4], weigt[4] = {0.0, 0.0, 0.0, 0.0}, os1[9];
-      for (int is = 0; is < isten; is++) {
-        double mx = 0.0;
-        for (int k = 0; k < 4; k++) {
-          double c1 = 0.0, c2 = 0.0;
-          for (int q = 0; q < 4; q++) {
-            c1 = c1 + qinvm[k + 4 * q] * S.unksl[is][q][1];
-            c2 = c2 + qinvm[k + 4 * q] * S.unksl[is][q][2];
-          }
-          double t1 = c1 / dxc, t2 = c2 / dyc;
-          double os = t1 * t1 + t2 * t2;
-          if (k == 0 || os > mx) mx = os;
-        }
-        os1[is] = mx;
+  __syncthreads();
+  // getunknp_local_Taylor: local projections
+  if (tid < 10) {
+    if (tid < 9) inv5(S.bbq[tid], S.bbqi[tid]);
+    else inv5(S.bb[0], S.bbi);
+  } else if (tid >= 32 && tid < 212) {
+    const int e = tid - 32, s = e / 20, q = (e % 20) / 5, i = e % 5;
+    double acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < 5; j++) acc += S.unkrl[s][q][j + 1] * S.bb[s][j + 5 * i];
+    S.rhsl[s][q][i + 1] = acc;
+  } else if (tid >= 212 && tid < 220) {
+    const int s = 1 + tid - 212;
+    const double im = 1.0 / S.mass[s];
+#pragma unroll
+    for (int k = 0; k < 5; k++) { S.hrow[s][0][k] = S.bbq[s][k] * im; S.hrow[s][1][k] = S.bbq[s][k + 5] * im; }
+  }
+  __syncthreads();
+  if (tid < 180) {
+    const int s = tid / 20, q = (tid % 20) / 5, i = tid % 5;
+    double acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < 5; j++) acc += S.rhsl[s][q][j + 1] * S.bbqi[s][j + 5 * i];
+    S.unkpl[s][q][i + 1] = acc;
+  } else if (tid < 216) {
+    const int s = (tid - 180) / 4, q = (tid - 180) % 4;
+    S.unkpl[s][q][0] = S.unkrl[s][q][0];
+  }
+  __syncthreads();
+  // candidate matrices: 4 Lagrangian, 4 Hermite normal matrices (and the
+  // right-hand sides of the derivative rows)
+  if (tid < 64) {
+    const int s = 1 + tid / 8, row = (tid >> 2) & 1, q = tid & 3;
+    double acc = 0.0;
+#pragma unroll
+    for (int k = 0; k < 5; k++) acc += S.hrow[s][row][k] * S.unkpl[s][q][k + 1];
+    S.rh[s][row][q] = acc;
+  }
+  for (int it = tid; it < 200; it += kWenoThreads) {
+    const int is = (it % 100) / 25, e = it % 25;
+    if (it < 100) {
+      S.mat[is][e] = S.mrow[cIelst1[is][e % 5 + 1] - 1][e / 5];
+    } else {
+      double acc = 0.0;
+#pragma unroll
+      for (int km = 0; km < 9; km++) acc += weno_hrow(S, is, km, e % 5) * weno_hrow(S, is, km, e / 5);
+      S.mat[4 + is][e] = acc;
+    }
+  }
+  __syncthreads();
+  if (tid < 8) {
+    inv5(S.mat[tid], S.matinv[tid]);
+  } else if (tid >= 32 && tid < 112) {
+    const int is = (tid - 32) / 20, q = ((tid - 32) % 20) / 5, im = (tid - 32) % 5;
+    double acc = 0.0;
+#pragma unroll
+    for (int km = 0; km < 9; km++) acc += weno_hrow(S, is, km, im) * weno_hrhs(S, is, km, q);
+    S.rhsls[is][q][im] = acc;
+  }
+  __syncthreads();
+  // candidate polynomials: central, Lagrangian, Hermite
+  if (tid < 216) {
+    const int c = tid / 24, q = (tid % 24) / 6, k = tid % 6;
+    double v;
+    if (k == 0) v = S.unkpl[0][q][0];
+    else if (c == 0) v = S.unkpl[0][q][k];
+    else {
+      v = 0.0;
+#pragma unroll
+      for (int ies = 0; ies < 5; ies++) {
+        const double r = c <= 4 ? S.unkpl[cIelst1[c - 1][ies + 1] - 1][q][0] - S.unkpl[0][q][0] : S.rhsls[c - 5][q][ies];
+        v += S.matinv[c - 1][(k - 1) + 5 * ies] * r;
       }
-      double weigl0 = .2, weigl1 = 0.8 / (isten - 1.0);
-      for (int is = 0; is < isten; is++)
+    }
+    S.unksl[c][q][k] = v;
+  }
+  __syncthreads();
+  // weno_cell_Taylor: characteristic WENO per interior face
+  if (tid < 36) {
+    const int a = tid / 9, is = tid - 9 * a;
+    double mx = 0.0;
+    if (S.fvalid[a]) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        double c1 = 0.0, c2 = 0.0;
+#pragma unroll
         for (int q = 0; q < 4; q++) {
-          double tt = epsil + os1[is];
-          weigh[is][q] = (is == 0 ? weigl0 : weigl1) / (tt * tt);
+          c1 += S.qinvm[a][k + 4 * q] * S.unksl[is][q][1];
+          c2 += S.qinvm[a][k + 4 * q] * S.unksl[is][q][2];
         }
-      for (int q = 0; q < 4; q++)
-        for (int is = 0; is < isten; is++) weigt[q] = weigt[q] + weigh[is][q];
-      for (int is = 0; is < isten; is++)
-        for (int q = 0; q < 4; q++) weigh[is][q] = weigh[is][q] / weigt[q];
-      if (FACT) {
-        for (int i = 0; i < 16; i++) { F->qinvm[ies][i] = qinvm[i]; F->qmat[ies][i] = qmat[i]; }
-        for (int is = 0; is < isten; is++)
-          for (int q = 0; q < 4; q++) F->wgt[ies][is][q] = weigh[is][q];
+        const double t1 = c1 / S.dxc[0], t2 = c2 / S.dxc[0];
+        const double os = t1 * t1 + t2 * t2;
+        if (k == 0 || os > mx) mx = os;
       }
-      double fch[4][6];
-      for (int q = 0; q < 4; q++) for (int k = 0; k < 6; k++) fch[q][k] = 0.0;
-      for (int is = 0; is < isten; is++)
-        for (int kq = 0; kq < 4; kq++)
-          for (int k = 0; k < 6; k++) {
-            double ch = 0.0;
-            for (int q = 0; q < 4; q++) ch = ch + qinvm[kq + 4 * q] * S.unksl[is][q][k];
-            fch[kq][k] = fch[kq][k] + weigh[is][kq] * ch;
-          }
-      double uf[4][6];
-      for (int q = 0; q < 4; q++) for (int k = 0; k < 6; k++) uf[q][k] = 0.0;
-      for (int kq = 0; kq < 4; kq++)
-        for (int k = 1; k < 6; k++)
-          for (int q = 0; q < 4; q++) uf[q][k] = uf[q][k] + qmat[q + 4 * kq] * fch[kq][k];
-      for (int q = 0; q < 4; q++) for (int k = 0; k < 6; k++) S.unkf[ies][q][k] = uf[q][k];
     }
+    // one weight per candidate: the indicator is the maximum over the fields
+    const double tt = 1.0e-6 + mx;
+    S.os[a][is] = (is == 0 ? .2 : 0.8 / 8.0) / (tt * tt);
   }
-  __syncwarp();
+  __syncthreads();
+  if (tid < 80) {
+    const int a = tid / 20, q = (tid % 20) / 5, k = tid % 5 + 1;
+    double w = 0.0, acc = 0.0;
+#pragma unroll
+    for (int is = 0; is < 9; is++) w += S.os[a][is];
+#pragma unroll
+    for (int is = 0; is < 9; is++) acc += (S.os[a][is] / w) * S.unksl[is][q][k];
+    S.wsum[a][q][k] = acc;
+  }
   if (FACT) {
-    if (lane == 0) {
-      int ifprj = 0;
-      for (int a = 0; a < 4; a++) ifprj += S.fvalid[a];
-      F->ifprj = ifprj;
+    // the factors, each item by itself
+    if (tid < 225) {
+      const int s = tid / 25, m = (tid % 25) / 5, i = tid % 5;
+      double acc = 0.0;
+#pragma unroll
+      for (int j = 0; j < 5; j++) acc += S.bb[s][m + 5 * j] * S.bbqi[s][j + 5 * i];
+      F->T[s][m * 5 + i] = acc;
+    }
+    if (tid < 100) F->matL[tid / 25][tid % 25] = S.matinv[tid / 25][tid % 25];
+    if (tid < 180) {
+      const int is = tid / 45, k = (tid % 45) / 9, km = tid % 9;
+      double acc = 0.0;
+#pragma unroll
+      for (int im = 0; im < 5; im++) acc += S.matinv[4 + is][k + 5 * im] * weno_hrow(S, is, km, im);
+      F->G[is][k][km] = acc;
+    }
+    if (tid < 120) {
+      const int is = tid / 30, ies = (tid % 30) / 10, row = (tid % 10) / 5, k = tid % 5;
+      F->H[is][ies][row][k] = S.hrow[cIelst2[is][ies + 1] - 1][row][k];
+    }
+    if (tid < 64) {
+      F->qinvm[tid / 16][tid % 16] = S.qinvm[tid / 16][tid % 16];
+      F->qmat[tid / 16][tid % 16] = S.qmat[tid / 16][tid % 16];
+    }
+    if (tid < 36) {
+      const int a = tid / 9, is = tid % 9;
+      double w = 0.0;
+#pragma unroll
+      for (int i = 0; i < 9; i++) w += S.os[a][i];
+      for (int q = 0; q < 4; q++) F->wgt[a][is][q] = S.os[a][is] / w;
+    }
+    if (tid < 25) {
+      const int j = tid / 5, i = tid % 5;
+      double acc = 0.0;
+#pragma unroll
+      for (int m = 0; m < 5; m++) acc += S.bbq[0][j + 5 * m] * S.bbi[m + 5 * i];
+      F->B[j][i] = acc;
+    }
+    if (tid == 0) {
+      F->ifprj = S.fvalid[0] + S.fvalid[1] + S.fvalid[2] + S.fvalid[3];
       for (int k = 0; k < 4; k++) F->mp[k] = mp[k];
-      for (int j = 1; j < 6; j++)
-        for (int i = 1; i < 6; i++) {
-          double acc = 0.0;
-          for (int m = 1; m < 6; m++) acc += S.mtbbq[(j - 1) + 5 * (m - 1)] * S.mtbbi[(m - 1) + 5 * (i - 1)];
-          F->B[j - 1][i - 1] = acc;
-        }
+    }
+    __syncthreads();
+    return true;
+  }
+  __syncthreads();
+  // characteristic projection of the weighted candidate and back
+  const int a20 = tid / 20, q20 = (tid % 20) / 5, k20 = tid % 5 + 1;
+  if (tid < 80 && S.fvalid[a20]) {
+    double acc = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) acc += S.qinvm[a20][q20 + 4 * q] * S.wsum[a20][q][k20];
+    S.fch[a20][q20][k20] = acc;
+  }
+  __syncthreads();
+  if (tid < 80 && S.fvalid[a20]) {
+    double acc = 0.0;
+#pragma unroll
+    for (int kq = 0; kq < 4; kq++) acc += S.qmat[a20][q20 + 4 * kq] * S.fch[a20][kq][k20];
+    S.unkf[a20][q20][k20] = acc;
+  }
+  __syncthreads();
+  // face average, inverse L2 projection back to the target's Taylor basis, un-rotate
+  if (tid < 32) {
+    const int q = tid / 5, k = tid % 5 + 1;
+    if (tid < 20) {
+      const double weigf = 1.0 / (S.fvalid[0] + S.fvalid[1] + S.fvalid[2] + S.fvalid[3]);
+      double acc = 0.0;
+      for (int a = 0; a < 4; a++)
+        if (S.fvalid[a]) acc += weigf * S.unkf[a][q][k];
+      S.phy[q][k] = acc;
     }
     __syncwarp();
-    return;
-  }
-  if (lane == 0) {
-    int ifprj = 0;
-    for (int a = 0; a < 4; a++) ifprj += S.fvalid[a];
-    double unk_phy[4][6];
-    for (int q = 0; q < 4; q++) for (int k = 0; k < 6; k++) unk_phy[q][k] = 0.0;
-    const double weigf = 1.0 / ifprj;
-    for (int a = 0; a < 4; a++) {
-      if (!S.fvalid[a]) continue;
-      for (int q = 0; q < 4; q++)
-        for (int k = 1; k < 6; k++) unk_phy[q][k] = unk_phy[q][k] + weigf * S.unkf[a][q][k];
+    if (tid < 20) {
+      double acc = 0.0;
+#pragma unroll
+      for (int j = 0; j < 5; j++) acc += S.phy[q][j + 1] * S.bbq[0][j + 5 * (k - 1)];
+      S.rhsuk[q][k] = acc;
     }
-    // inverse L2 projection back to the target's Taylor basis, un-rotate
-    double rhsuk[5][4], out[4][6];
-    for (int i = 0; i < 5; i++) for (int q = 0; q < 4; q++) rhsuk[i][q] = 0.0;
-    for (int i = 1; i < 6; i++)
-      for (int j = 1; j < 6; j++)
-        for (int q = 0; q < 4; q++) rhsuk[i - 1][q] = rhsuk[i - 1][q] + unk_phy[q][j] * S.mtbbq[(j - 1) + 5 * (i - 1)];
-    for (int q = 0; q < 4; q++) for (int k = 1; k < 6; k++) out[q][k] = 0.0;
-    for (int i = 1; i < 6; i++)
-      for (int j = 1; j < 6; j++)
-        for (int q = 0; q < 4; q++) out[q][i] = out[q][i] + rhsuk[j - 1][q] * S.mtbbi[(j - 1) + 5 * (i - 1)];
-    for (int k = 1; k < 6; k++) vec_local_back(mp, out[1][k], out[2][k]);
-    for (int q = 0; q < 4; q++)
-      for (int k = 1; k < 6; k++) d.Uw[(q * 5 + (k - 1)) * d.nquad + iq] = out[q][k];
-    d.flag[ielem] = 2;  // reconstructed
+    __syncwarp();
+    if (tid < 20) {
+      double acc = 0.0;
+#pragma unroll
+      for (int j = 0; j < 5; j++) acc += S.rhsuk[q][j + 1] * S.bbi[j + 5 * (k - 1)];
+      S.out[q][k] = acc;
+    }
+    __syncwarp();
+    if (tid < 20) {
+      double v = S.out[q][k];
+      if (q == 1 || q == 2) {
+        double x = S.out[1][k], y = S.out[2][k];
+        vec_local_back(mp, x, y);
+        v = q == 1 ? x : y;
+      }
+      d.Uw[(q * 5 + (k - 1)) * nq + iq] = v;
+      if (tid == 0) d.flag[ielem] = 2;  // reconstructed
+    }
   }
-  __syncwarp();
+  __syncthreads();
+  return true;
 }
 
 // ---------------------------------------------------------------------------
 // The frozen reconstruction as a linear map, and its transpose (the WENO
 // part of the adjoint).  For troubled quad c (list slot t) with a complete
-// stencil, out_c = L_c v: the factors of L_c come from weno_warp_cell_t<true>
+// stencil, out_c = L_c v: the factors of L_c come from weno_block_cell<true>
 // at the state d.Us; v is a state-shaped vector.  The transpose kernel
 // writes L_c^T lam_c (lam_c: the adjoint of c's replaced moments 1..5) per
 // stencil cell into wbuf[(s*24 + q*6 + k) * cap + t]; the gather kernel adds
@@ -1034,8 +1174,7 @@ struct WenoAdjShared {
   double vphy[4][6];        // face-averaged moments / their adjoint
   double vd[8][4][9];       // transpose: adjoints of the Lagrangian differences and Hermite rows
 };
-__constant__ int cIelst1[4][7] = {{1, 2, 5, 6, 9, 8, 3}, {1, 3, 2, 7, 6, 9, 5}, {1, 4, 3, 8, 7, 6, 5}, {1, 5, 4, 9, 8, 7, 3}};
-__constant__ int cIelst2[4][4] = {{1, 2, 6, 9}, {1, 3, 6, 7}, {1, 4, 8, 7}, {1, 5, 8, 9}};
+
 
 // out moments 1..5 of troubled slot t = L_t v (v and out are state-shaped)
 __device__ void weno_tangent_cell(const Dev &d, int t, const WenoFactors &F, WenoAdjShared &A, const double *v,
@@ -1275,26 +1414,29 @@ struct WenoAdjBlock {
 };
 
 // mode 0: the tangent out = L v on troubled quads; mode 1: the transpose into wbuf
-__global__ void __launch_bounds__(32) k_weno_linear(Dev d, int mode, const double *v, double *out, double *wbuf,
+// (one block per troubled quad; its first warp applies the factors)
+__global__ void __launch_bounds__(kWenoThreads) k_weno_linear(Dev d, int mode, const double *v, double *out, double *wbuf,
                                                     int *wslot, int cap, int *overflow) {
   extern __shared__ __align__(16) unsigned char wsm[];
   WenoAdjBlock &B = *reinterpret_cast<WenoAdjBlock *>(wsm);
   const int n = *d.wcount;
-  const int lane = threadIdx.x & 31;
   for (int t = blockIdx.x; t < n; t += gridDim.x) {
     const int iq = d.wlist[t];
     if (d.stencil[iq] < 0 || d.flag[iq + d.ntria] != 2) continue;  // left unlimited by the forward pass
-    weno_warp_cell_t<true>(d, t, B.S, &B.F);
-    if (mode == 0) {
-      weno_tangent_cell(d, t, B.F, B.A, v, out);
-    } else {
-      if (t >= cap) {
-        if (lane == 0) atomicExch(overflow, 1);
-        continue;
-      }
-      if (lane == 0) wslot[iq] = t;
-      weno_transpose_cell(d, t, B.F, B.A, v, wbuf, cap);
+    if (mode == 1 && t >= cap) {
+      if (threadIdx.x == 0) atomicExch(overflow, 1);
+      continue;
     }
+    weno_block_cell<true>(d, t, B.S, &B.F);
+    if (threadIdx.x < 32) {
+      if (mode == 0) {
+        weno_tangent_cell(d, t, B.F, B.A, v, out);
+      } else {
+        if (threadIdx.x == 0) wslot[iq] = t;
+        weno_transpose_cell(d, t, B.F, B.A, v, wbuf, cap);
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -1346,11 +1488,12 @@ __global__ void k_weno_gather(Dev d, double *lamU, double *lamUn, int fold, cons
   for (int v = 0; v < 24; v++) lamU[v * nc + e] = l[v];
 }
 
-__global__ void __launch_bounds__(32) k_weno_warp(Dev d) {
-  __shared__ WenoShared S;
+__global__ void __launch_bounds__(kWenoThreads) k_weno_block(Dev d) {
+  extern __shared__ __align__(16) unsigned char wsm[];
+  WenoShared &S = *reinterpret_cast<WenoShared *>(wsm);
   if (stopped(d)) return;
   const int n = *d.wcount;
-  for (int t = blockIdx.x; t < n; t += gridDim.x) weno_warp_cell_t<false>(d, t, S, nullptr);
+  for (int t = blockIdx.x; t < n; t += gridDim.x) weno_block_cell<false>(d, t, S, nullptr);
 }
 
 
@@ -3458,22 +3601,32 @@ void launch_error(const Dev &d, cudaStream_t st, const double *X, const double *
   k_error_partial<<<nblk(d.nquad, 256), 256, 0, st>>>(d, X, Y, part);
 }
 void launch_weno(const Dev &d, cudaStream_t st) { k_weno<<<nblk(d.nquad, 64), 64, 0, st>>>(d); }
-// one warp per troubled quad, a grid of at most 8 blocks per SM looping over the list
-void launch_weno_warp(const Dev &d, cudaStream_t st) {
-  k_weno_warp<<<d.nquad < 1184 ? (d.nquad > 0 ? d.nquad : 1) : 1184, 32, 0, st>>>(d);
+// one block per troubled quad, a grid of at most 3 blocks per SM looping over the list
+static int weno_grid(const Dev &d) { return d.nquad < 444 ? (d.nquad > 0 ? d.nquad : 1) : 444; }
+void launch_weno_block(const Dev &d, cudaStream_t st) {
+  k_weno_block<<<weno_grid(d), kWenoThreads, sizeof(WenoShared), st>>>(d);
 }
-size_t weno_linear_smem() { return sizeof(WenoAdjBlock); }
 void launch_weno_linear(const Dev &d, cudaStream_t st, int mode, const double *v, double *out, double *wbuf,
                         int *wslot, int cap, int *overflow) {
-  const int g = d.nquad < 1184 ? (d.nquad > 0 ? d.nquad : 1) : 1184;
-  k_weno_linear<<<g, 32, sizeof(WenoAdjBlock), st>>>(d, mode, v, out, wbuf, wslot, cap, overflow);
+  k_weno_linear<<<weno_grid(d), kWenoThreads, sizeof(WenoAdjBlock), st>>>(d, mode, v, out, wbuf, wslot, cap, overflow);
+}
+// shared-memory limits of the kernels above 48 KB, on the current device
+cudaError_t set_kernel_limits() {
+  cudaError_t e = cudaFuncSetAttribute(k_weno_block, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(WenoShared));
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(k_weno_linear, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(WenoAdjBlock));
 }
 void launch_weno_gather(const Dev &d, cudaStream_t st, double *lamU, double *lamUn, int fold, const double *wbuf,
                         const int *wslot, int cap, const int *inv_ptr, const int *inv_ent) {
   k_weno_gather<<<nblk(d.ncell, 128), 128, 0, st>>>(d, lamU, lamUn, fold, wbuf, wslot, cap, inv_ptr, inv_ent);
 }
-void launch_weno_swap(const Dev &d, cudaStream_t st) { k_weno_swap<<<nblk(d.nquad, 256), 256, 0, st>>>(d); }
-void launch_weno_commit(const Dev &d, cudaStream_t st) { k_weno_commit<<<nblk(d.nquad, 256), 256, 0, st>>>(d); }
+// 20 moments per listed quad, at most one block of 256 per SM
+static int weno_list_grid(const Dev &d) {
+  const int g = nblk(20 * (d.nquad < 4096 ? d.nquad : 4096), 256);
+  return g < 148 ? g : 148;
+}
+void launch_weno_swap(const Dev &d, cudaStream_t st) { k_weno_swap<<<weno_list_grid(d), 256, 0, st>>>(d); }
+void launch_weno_commit(const Dev &d, cudaStream_t st) { k_weno_commit<<<weno_list_grid(d), 256, 0, st>>>(d); }
 void launch_corner(const Dev &d, cudaStream_t st) { k_corner<<<nblk(d.nquad, 128), 128, 0, st>>>(d); }
 void launch_node(const Dev &d, cudaStream_t st) { k_node<<<nblk(d.npoin, 256), 256, 0, st>>>(d); }
 void launch_rhs(const Dev &d, cudaStream_t st) { k_rhs<<<nblk(d.nquad, 128), 128, 0, st>>>(d); }
