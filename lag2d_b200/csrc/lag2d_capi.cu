@@ -23,8 +23,9 @@ void launch_reset_count(const Dev &d, cudaStream_t st);
 void launch_persson(const Dev &d, cudaStream_t st);
 void launch_flags_from_host(const Dev &d, cudaStream_t st, const int *flags);
 void launch_weno(const Dev &d, cudaStream_t st);
-void launch_weno_block(const Dev &d, cudaStream_t st);
+void launch_weno_block(const Dev &d, cudaStream_t st, int fixcorr);
 cudaError_t set_kernel_limits();
+cudaError_t set_fast_limits();
 void launch_weno_commit(const Dev &d, cudaStream_t st);
 void launch_corner(const Dev &d, cudaStream_t st);
 void launch_node(const Dev &d, cudaStream_t st);
@@ -43,10 +44,11 @@ void launch_unkno_out(const Dev &d, cudaStream_t st, double *aos);
 void launch_xy_in(int n, cudaStream_t st, const double *xy, double *x, double *y, double *x2, double *y2);
 void launch_xy_out(int n, cudaStream_t st, double *xy, const double *x, const double *y);
 void launch_fast_persson(const Dev &d, cudaStream_t st);
-void launch_fast_corner(const Dev &d, cudaStream_t st);
-void launch_fast_node(const Dev &d, cudaStream_t st);
+void launch_fast_corr(const Dev &d, cudaStream_t st);
+void launch_fast_faces(const Dev &d, cudaStream_t st);
+void launch_fast_node(const Dev &d, cudaStream_t st, int move, double alfa);
 void launch_fast_rhs(const Dev &d, cudaStream_t st, int fuse, double alfa);
-void launch_fast_dt(const Dev &d, cudaStream_t st, int ndt);
+void launch_fast_dt(const Dev &d, cudaStream_t st, int ndt, int itime);
 void launch_mixed_corner(const Dev &d, cudaStream_t st);
 void launch_fast_src(const Dev &d, cudaStream_t st);
 void launch_mixed_src(const Dev &d, cudaStream_t st);
@@ -108,6 +110,13 @@ struct lag2d_handle {
   double *stage_u = nullptr;   // staging for unkno(ndegr,nq,ncell) in the caller's layout
   double *stage_x = nullptr;   // staging for coord(2,npoin)
   double *stage_v = nullptr;   // staging for ustar(2,npoin) (its own, so no copy waits for another)
+  // the optimised step leaves its result in U^n, x^n only: Us, xs are then behind
+  bool stale = false;
+  // side streams of the captured step (independent passes of a stage run beside
+  // the main chain) and the event that orders them
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t fork = nullptr;
+  bool forking = false;
   cudaGraphExec_t graph = nullptr;
   long long graph_launches = 0;
   long long launches = 0;
@@ -307,40 +316,17 @@ static void enqueue_step_reference_order(lag2d_handle *h, int itime) {
   run(h, "copy", [&] { launch_copyback(d, h->st); launch_step_end(d, h->st, 1); }, 2);
 }
 
-// Corner and RHS passes of the optimised step: FP64, or the FP32-mixed form
-// (config precision = 1) with the same node pass, update and geometry.
-// Triangles run their FP64 kernels in both forms.
-// launches of corner_pass: the triangles' kernel, then two quad kernels
-// (sub-cell corrections, corner faces)
-static int corner_launches(const lag2d_handle *h, const Dev &d) {
-  (void)h;
-  return (d.ntria > 0) + 2;
+// Passes of the optimised step: FP64, or the FP32-mixed form (config precision
+// = 1) with the same node pass, update and geometry.  Triangles run their FP64
+// kernels in both forms.
+static bool has_src(const Dev &d) { return d.ncase == 1 && d.nquad > 0; }
+static void launch_src(lag2d_handle *h, const Dev &d, cudaStream_t st) {
+  if (h->cfg.precision == 1) launch_mixed_src(d, st);
+  else launch_fast_src(d, st);
 }
-
-// Taylor-Green energy source of the stage (quads; ncase 1 only), read by the
-// RHS pass
-static int src_launches(const Dev &d) { return d.ncase == 1 && d.nquad > 0; }
-static void src_pass(lag2d_handle *h, const Dev &d) {
-  if (!src_launches(d)) return;
-  if (h->cfg.precision == 1) launch_mixed_src(d, h->st);
-  else launch_fast_src(d, h->st);
-}
-
-static void corner_pass(lag2d_handle *h, const Dev &d) {
-  launch_tri_corner(d, h->st);
-  if (h->cfg.precision == 1) launch_mixed_corner(d, h->st);
-  else launch_fast_corner(d, h->st);
-}
-// launches of rhs_pass: the triangles' kernel, then one quad kernel
-static int rhs_launches(const lag2d_handle *h, const Dev &d) {
-  (void)h;
-  return (d.ntria > 0) + 1;
-}
-
-static void rhs_pass(lag2d_handle *h, const Dev &d, int fuse, double alfa) {
-  launch_tri_rhs(d, h->st, d.us_new, d.vs_new, fuse, alfa);
-  if (h->cfg.precision == 1) launch_mixed_rhs(d, h->st, fuse, alfa);
-  else launch_fast_rhs(d, h->st, fuse, alfa);
+static void launch_rhs_quads(lag2d_handle *h, const Dev &d, cudaStream_t st, int fuse, double alfa) {
+  if (h->cfg.precision == 1) launch_mixed_rhs(d, st, fuse, alfa);
+  else launch_fast_rhs(d, st, fuse, alfa);
 }
 
 // Stage recorder of the adjoint's recompute pass.  Before each stage the
@@ -379,43 +365,127 @@ struct StageRec {
     return d;
   }
 };
-// The same step with the optimised kernels: node partial sums, recomputed
-// corner data, closed-form volumes and the stage update fused into the RHS
-// pass in stages 2 and 3.
+// The same step with the optimised kernels.
+//
+// Buffers: stage 1 reads U^n, x^n themselves, the last stage writes them, the
+// stages between use Us and xs / xt, so nothing is copied at the end of the
+// step (1024 x 1024: 93 us a step).  WENO therefore leaves the stage state as
+// it is: the FP64 face and RHS passes take the moments of a limited quad from
+// its output (the mixed ones run on the swapped-in moments, which stage 1 swaps
+// back out).
+//
+// Order: the time step needs only the cell-average mass flux, which the node
+// velocities give, so dt follows the node pass and every RHS pass carries its
+// update.  Independent passes run beside the main chain when the step is
+// captured (h->forking): the sub-cell corrections beside the Persson pass, the
+// triangles' corners and the source beside both, the geometry of the new
+// nodes and the next stage's source beside the RHS pass.  On a small mesh a
+// stage is then a chain of 6 launches instead of 11 (64 x 64: 160 -> 113 us a
+// step); on a large one (1024 x 1024: 3.48 -> 3.37 ms) the
+// source, bound by FP64 arithmetic, overlaps passes that wait on memory.
 static void enqueue_step_fast(lag2d_handle *h, int itime, const StageRec *rec = nullptr) {
-  Dev d = h->d;
-  const int nstag = h->cfg.nstag;
-  const int T = d.ntria > 0;
-  run(h, "begin", [&] { launch_step_begin(d, h->st, itime); });
+  const Dev &d0 = h->d;
+  const int nstag = h->cfg.nstag, mixed = h->cfg.precision == 1;
+  const int T = d0.ntria > 0;
+  const bool par = h->forking && !h->timing && !rec;
+  cudaStream_t s0 = h->st, s1 = par ? h->side[0] : s0, s2 = par ? h->side[1] : s0;
+  // work queued on `waits` from here on follows what `on` holds so far; a side
+  // stream that has not joined the capture yet holds nothing
+  bool joined[2] = {false, false};
+  auto after = [&](cudaStream_t waits, cudaStream_t on) {
+    if (waits == on) return;
+    if (waits != s0) joined[waits == s2] = true;
+    else if (!joined[on == s2]) return;
+    cudaEventRecord(h->fork, on);
+    cudaStreamWaitEvent(waits, h->fork, 0);
+  };
+  auto view = [&](int istag) {
+    Dev d = d0;
+    const bool last = istag == nstag;
+    if (istag == 1) { d.Us = d0.Un; d.xs = d0.xn; d.ys = d0.yn; }
+    if (istag == 3) { d.xs = d0.xt; d.ys = d0.yt; }
+    d.Uo = last ? d0.Un : d0.Us;
+    d.xo = last ? d0.xn : istag == 1 ? d0.xs : d0.xt;
+    d.yo = last ? d0.yn : istag == 1 ? d0.ys : d0.yt;
+    d.us_new = d0.us;
+    d.vs_new = d0.vs;
+    d.wcount = d0.wcount + (istag - 1);
+    d.src = d0.src + ((istag - 1) & 1) * 6 * (size_t)d0.nquad;  // the next stage's source is written beside this RHS
+    return d;
+  };
   for (int istag = 1; istag <= nstag; istag++) {
     const double alfa = kRK[nstag - 2][istag - 1];
+    Dev d = view(istag);
     if (rec) {
       const size_t slot = (size_t)rec->step * rec->nstag + (istag - 1);
-      d = rec->outputs(h->d, slot);
-      cudaMemcpyAsync(rec->U + slot * rec->nu, d.Us, rec->nu * sizeof(double), cudaMemcpyDeviceToDevice, h->st);
-      cudaMemcpyAsync(rec->x + slot * rec->np, d.xs, rec->np * sizeof(double), cudaMemcpyDeviceToDevice, h->st);
-      cudaMemcpyAsync(rec->y + slot * rec->np, d.ys, rec->np * sizeof(double), cudaMemcpyDeviceToDevice, h->st);
-      cudaMemcpyAsync(rec->us + slot * rec->np, d.us, rec->np * sizeof(double), cudaMemcpyDeviceToDevice, h->st);
-      cudaMemcpyAsync(rec->vs + slot * rec->np, d.vs, rec->np * sizeof(double), cudaMemcpyDeviceToDevice, h->st);
+      d = rec->outputs(d, slot);
+      cudaMemcpyAsync(rec->U + slot * rec->nu, d.Us, rec->nu * sizeof(double), cudaMemcpyDeviceToDevice, s0);
+      cudaMemcpyAsync(rec->x + slot * rec->np, d.xs, rec->np * sizeof(double), cudaMemcpyDeviceToDevice, s0);
+      cudaMemcpyAsync(rec->y + slot * rec->np, d.ys, rec->np * sizeof(double), cudaMemcpyDeviceToDevice, s0);
+      cudaMemcpyAsync(rec->us + slot * rec->np, d.us, rec->np * sizeof(double), cudaMemcpyDeviceToDevice, s0);
+      cudaMemcpyAsync(rec->vs + slot * rec->np, d.vs, rec->np * sizeof(double), cudaMemcpyDeviceToDevice, s0);
     }
-    run(h, "persson", [&] { launch_reset_count(d, h->st); launch_fast_persson(d, h->st); }, 2);
-    run(h, "weno", [&] { launch_weno_block(d, h->st); launch_weno_commit(d, h->st); }, 2);
-    if (src_launches(d)) run(h, "src", [&] { src_pass(h, d); });
-    run(h, "corner", [&] { corner_pass(h, d); }, corner_launches(h, d));
-    run(h, "node", [&] { launch_fast_node(d, h->st); });
+    if (has_src(d) && istag == 1) {
+      after(s2, s0);
+      run(h, "src", [&] { launch_src(h, d, s2); });
+    }
+    if (T) {
+      after(s2, s0);
+      run(h, "corner", [&] { launch_tri_corner(d, s2); });
+    }
+    if (!mixed) {
+      after(s1, s0);
+      run(h, "corner", [&] { launch_fast_corr(d, s1); });
+    }
+    run(h, "persson", [&] { launch_fast_persson(d, s0); });
+    after(s0, s1);
+    run(h, "weno", [&] { launch_weno_block(d, s0, !mixed); });
+    if (mixed) {
+      run(h, "weno", [&] { launch_weno_swap(d, s0); });
+      run(h, "corner", [&] { launch_mixed_corner(d, s0); }, 2);
+    } else {
+      run(h, "corner", [&] { launch_fast_faces(d, s0); });
+    }
+    after(s0, s2);  // the triangles' corners; and the source, for the RHS pass
+    run(h, "node", [&] { launch_fast_node(d, s0, istag > 1, alfa); });
     if (istag == 1) {
-      // getdelt_lag needs only the cell-average mass flux of this stage's
-      // RHS, which the node velocities give: dt first, then every stage's
-      // RHS pass carries its own update
-      run(h, "dt", [&] { launch_fast_dt(d, h->st, h->cfg.ndt); }, 2);
+      run(h, "dt", [&] { launch_fast_dt(d, s0, h->cfg.ndt, itime); });
       if (rec)
-        cudaMemcpyAsync(rec->dt + rec->step, &d.sc_dev->dtfix, sizeof(double), cudaMemcpyDeviceToDevice, h->st);
+        cudaMemcpyAsync(rec->dt + rec->step, &d.sc_dev->dtfix, sizeof(double), cudaMemcpyDeviceToDevice, s0);
+      run(h, "nodes", [&] { launch_fast_nodes(d, s0, alfa); });
     }
-    run(h, "rhs", [&] { rhs_pass(h, d, 1, alfa); }, rhs_launches(h, d));
-    run(h, "nodes", [&] { launch_fast_nodes(d, h->st, alfa); });
-    run(h, "geom", [&] { launch_tri_geom(d, h->st, d.xs, d.ys); launch_fast_geom(d, h->st, 1); }, 1 + T);
+    // volumes and centre nodes at the new coordinates, then the next stage's source
+    Dev dx = d;
+    dx.xs = d.xo;
+    dx.ys = d.yo;
+    after(s2, s0);
+    run(h, "geom", [&] { launch_tri_geom(dx, s2, dx.xs, dx.ys); launch_fast_geom(dx, s2, 1); }, 1 + T);
+    if (T) {
+      after(s1, s0);
+      run(h, "rhs", [&] { launch_tri_rhs(d, s1, d.us_new, d.vs_new, 1, alfa); });
+    }
+    run(h, "rhs", [&] { launch_rhs_quads(h, d, s0, 1, alfa); });
+    if (mixed && istag == 1) run(h, "weno", [&] { launch_weno_swap(d, s0); });
+    if (T) after(s0, s1);
+    after(s0, s2);
+    if (has_src(d) && istag < nstag) {
+      const Dev dn = view(istag + 1);
+      run(h, "src", [&] { launch_src(h, dn, s2); });
+    }
   }
-  run(h, "copy", [&] { launch_copyback(d, h->st); launch_step_end(d, h->st, 1); }, 2);
+  run(h, "copy", [&] { launch_step_end(d0, s0, 1); });
+  h->stale = true;
+}
+
+// brings the stage buffers to the state (entry points that work on them)
+static void sync_stage(lag2d_handle *h) {
+  if (!h->stale) return;
+  const Dev &d = h->d;
+  const size_t np = d.npoin * sizeof(double);
+  cudaMemcpyAsync(d.Us, d.Un, NU * (size_t)d.ncell * sizeof(double), cudaMemcpyDeviceToDevice, h->st);
+  cudaMemcpyAsync(d.xs, d.xn, np, cudaMemcpyDeviceToDevice, h->st);
+  cudaMemcpyAsync(d.ys, d.yn, np, cudaMemcpyDeviceToDevice, h->st);
+  h->stale = false;
 }
 
 static void enqueue_step(lag2d_handle *h, int itime) {
@@ -423,16 +493,19 @@ static void enqueue_step(lag2d_handle *h, int itime) {
   else enqueue_step_fast(h, itime);
 }
 
-static int read_status(lag2d_handle *h) {
-  Scalars s;
-  CK(cudaMemcpyAsync(&s, h->d.sc_dev, sizeof(Scalars), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaStreamSynchronize(h->st));
+static int status_of(const Scalars &s) {
   CK(cudaGetLastError());
   // a broken state outranks the stencil notice (which leaves the step complete)
   if (s.status & ST_NONPHYS) return fail(LAG2D_ENONPHYS, "non-positive cell volume");
   if (s.status & ST_STENCIL)
     return fail(LAG2D_ESTENCIL, "WENO: a troubled quad has a vertex valence the reference rejects");
   return LAG2D_OK;
+}
+static int read_status(lag2d_handle *h) {
+  Scalars s;
+  CK(cudaMemcpyAsync(&s, h->d.sc_dev, sizeof(Scalars), cudaMemcpyDeviceToHost, h->st));
+  CK(cudaStreamSynchronize(h->st));
+  return status_of(s);
 }
 
 // npoly = 1: the linear branch on straight 4-node quads (ipqua(4, nquad)),
@@ -537,9 +610,20 @@ int lag2d_create(const lag2d_mesh *m, const lag2d_config *c, lag2d_handle **out)
     delete h;
     return fail(LAG2D_ECUDA, "cudaStreamCreate failed");
   }
-  if (cudaError_t e = set_kernel_limits()) {
+  cudaError_t attr_err = set_kernel_limits();
+  if (attr_err == cudaSuccess) attr_err = set_fast_limits();
+  if (attr_err != cudaSuccess) {
     lag2d_destroy(h);
-    return fail(LAG2D_ECUDA, std::string("kernel attributes: ") + cudaGetErrorString(e));
+    return fail(LAG2D_ECUDA, std::string("kernel attributes: ") + cudaGetErrorString(attr_err));
+  }
+  for (cudaStream_t &q : h->side)
+    if (cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) != cudaSuccess) {
+      lag2d_destroy(h);
+      return fail(LAG2D_ECUDA, "cudaStreamCreate failed");
+    }
+  if (cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming) != cudaSuccess) {
+    lag2d_destroy(h);
+    return fail(LAG2D_ECUDA, "cudaEventCreate failed");
   }
   const int nq = m->nquad, np = m->npoin;
   // ---- connectivity
@@ -622,17 +706,18 @@ int lag2d_create(const lag2d_mesh *m, const lag2d_config *c, lag2d_handle **out)
   A(&d.xn, np); A(&d.yn, np); A(&d.xs, np); A(&d.ys, np); A(&d.us, np); A(&d.vs, np);
   A(&d.amatr, 16 * (size_t)ncell); A(&d.rhs, NU * (size_t)ncell); A(&d.cf, 5 * 32 * (size_t)nq);
   A(&d.flag, ncell); A(&d.geoph, 2 * (size_t)ncell); A(&d.mapmt, 4 * (size_t)ncell);
-  A(&d.Uw, 20 * (size_t)nq); A(&d.wlist, nq); A(&d.wcount, 1);
+  A(&d.Uw, 20 * (size_t)nq); A(&d.wlist, nq); A(&d.wcount, 4); A(&d.xt, np); A(&d.yt, np);
   A(&d.dtpart, 2 * (size_t)dt_blocks(d) + 2); A(&d.sc_dev, 1); A(&h->flags_dev, ncell);
   A(&h->stage_u, NU * (size_t)ncell); A(&h->stage_x, 2 * (size_t)np); A(&h->stage_v, 2 * (size_t)np);
   int *ptr2_d, *slot_d;
   A(&ptr2_d, cnt2.size()); A(&slot_d, slots.size());
-  A(&d.npart, 45 * (size_t)nq); A(&d.corr, 4 * (size_t)nq); A(&d.src, 6 * (size_t)nq); A(&d.us_new, np); A(&d.vs_new, np);
+  A(&d.npart, 45 * (size_t)nq); A(&d.corr, 4 * (size_t)nq); A(&d.src, 12 * (size_t)nq); A(&d.us_new, np); A(&d.vs_new, np);
   A(&d.wmom, 9 * (size_t)nq);
   int *ipt_d;
   A(&ipt_d, ipt.size()); A(&d.tmsub, 4 * (size_t)nt); A(&d.tcf, 5 * 24 * (size_t)nt); A(&d.tpart, 5 * 6 * (size_t)nt);
   if (rc != LAG2D_OK) { lag2d_destroy(h); return rc; }
   d.ipt = ipt_d;
+  d.Uo = d.Us; d.xo = d.xs; d.yo = d.ys; d.dtcount = d.wcount + 3;
   d.ipq = ipq_d; d.esq = esq_d; d.stencil = sten_d; d.node_ptr = ptr_d; d.node_cf = ncf_d;
   d.bcmask = mask_d; d.x0 = x0; d.y0 = y0;
   d.node_ptr2 = ptr2_d; d.node_slot = slot_d;
@@ -749,6 +834,7 @@ int lag2d_init_fields(lag2d_handle *h, double *geoel, double *amatr, double *unk
   CK(cudaMemcpyAsync(d.ys, d.y0, np * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
   CK(cudaMemsetAsync(d.us, 0, np * sizeof(double), h->st));
   CK(cudaMemsetAsync(d.vs, 0, np * sizeof(double), h->st));
+  h->stale = false;
   run(h, "geom", [&] { geom_all(h, d.xn, d.yn); }, 1 + (d.ntria > 0));
   int st = read_status(h);
   if (st != LAG2D_OK) return st;
@@ -801,16 +887,16 @@ int lag2d_set_state(lag2d_handle *h, const double *unkno, const double *coord, c
   }
   Scalars s0{};
   CK(cudaMemcpyAsync(d.sc_dev, &s0, sizeof(Scalars), cudaMemcpyHostToDevice, h->st));
+  h->stale = false;
   run(h, "geom", [&] { geom_all(h, d.xs, d.ys); }, 1 + (d.ntria > 0));
   return read_status(h);
 }
 
 static int put_scalars(lag2d_handle *h, int itime, double dtfix, double tacru) {
   Scalars s{};
-  CK(cudaMemcpyAsync(&s, h->d.sc_dev, sizeof(Scalars), cudaMemcpyDeviceToHost, h->st));
-  CK(cudaStreamSynchronize(h->st));
-  s.dtfix = dtfix; s.tacru = tacru; s.itime = itime; s.done = 0; s.status = 0;
+  s.dtfix = dtfix; s.tacru = tacru; s.itime = itime;
   CK(cudaMemcpyAsync(h->d.sc_dev, &s, sizeof(Scalars), cudaMemcpyHostToDevice, h->st));
+  CK(cudaMemsetAsync(h->d.wcount, 0, 4 * sizeof(int), h->st));
   return LAG2D_OK;
 }
 
@@ -820,19 +906,46 @@ static int get_scalars(lag2d_handle *h, Scalars *s) {
   return LAG2D_OK;
 }
 
+// one step with itime incremented on the device, captured once per handle
+static int step_graph(lag2d_handle *h) {
+  if (h->graph) return LAG2D_OK;
+  cudaGraph_t g;
+  CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
+  const long long before = h->launches;
+  h->forking = true;
+  enqueue_step(h, -1);
+  h->forking = false;
+  h->graph_launches = h->launches - before;
+  h->launches = before;  // counted per replay
+  CK(cudaStreamEndCapture(h->st, &g));
+  const cudaError_t e = cudaGraphInstantiate(&h->graph, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) h->graph = nullptr;
+  CK(e);
+  return LAG2D_OK;
+}
+
 int lag2d_step(lag2d_handle *h, int itime, double *dtfix, double *tacru) {
   if (!h || !dtfix || !tacru) return fail(LAG2D_EINVAL, "null argument");
   if (h->p1) P1_CALL(p1::step(h->p1, itime, dtfix, tacru, err_));
-  int r = put_scalars(h, itime, *dtfix, *tacru);
+  // a replay of the captured step; with timing on, launch by launch
+  int r = put_scalars(h, itime - 1, *dtfix, *tacru);
   if (r) return r;
-  enqueue_step(h, itime);
+  if (h->timing) {
+    enqueue_step(h, itime);
+  } else {
+    if ((r = step_graph(h))) return r;
+    CK(cudaGraphLaunch(h->graph, h->st));
+    h->launches += h->graph_launches;
+  }
+  if (!h->cfg.order_exact) h->stale = true;
   Scalars s;
   r = get_scalars(h, &s);
   if (r) return r;
   if (h->timing) flush_timing(h);
   *dtfix = s.dtfix;
   *tacru = s.tacru;
-  return read_status(h);
+  return status_of(s);
 }
 
 int lag2d_run(lag2d_handle *h, int itime0, int nsteps, double *dtfix, double *tacru, int *done) {
@@ -846,18 +959,7 @@ int lag2d_run(lag2d_handle *h, int itime0, int nsteps, double *dtfix, double *ta
     for (int i = 0; i < nsteps; i++) { enqueue_step(h, itime0 + i); steps++; }
     flush_timing(h);
   } else {
-    if (!h->graph) {
-      // one step with itime incremented on the device, captured once
-      cudaGraph_t g;
-      CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
-      long long before = h->launches;
-      enqueue_step(h, -1);
-      CK(cudaStreamEndCapture(h->st, &g));
-      CK(cudaGraphInstantiate(&h->graph, g, 0));
-      cudaGraphDestroy(g);
-      h->graph_launches = h->launches - before;
-      h->launches = before;  // counted per replay below
-    }
+    if ((r = step_graph(h))) return r;
     const long long per_step = h->graph_launches;
     for (int i = 0; i < nsteps; i++) {
       CK(cudaGraphLaunch(h->graph, h->st));
@@ -865,13 +967,14 @@ int lag2d_run(lag2d_handle *h, int itime0, int nsteps, double *dtfix, double *ta
       steps++;
     }
   }
+  if (steps && !h->cfg.order_exact) h->stale = true;
   Scalars s;
   r = get_scalars(h, &s);
   if (r) return r;
   *dtfix = s.dtfix;
   *tacru = s.tacru;
   if (done) *done = s.done ? std::min(steps, std::max(0, s.itime - itime0 + 1)) : steps;
-  return read_status(h);
+  return status_of(s);
 }
 
 int lag2d_get_state(lag2d_handle *h, double *unkno, double *coord, double *ustar, double *geoel) {
@@ -904,6 +1007,7 @@ int lag2d_rhs(lag2d_handle *h, int itime, double *rhsel, int *flags) {
     P1_CALL(p1::rhs(h->p1, rhsel, err_));
   }
   Dev &d = h->d;
+  sync_stage(h);
   int r = put_scalars(h, itime, 0.0, 0.0);
   if (r) return r;
   const bool ex = h->cfg.order_exact != 0;
@@ -915,7 +1019,7 @@ int lag2d_rhs(lag2d_handle *h, int itime, double *rhsel, int *flags) {
     CK(cudaMemcpyAsync(h->flags_dev, d.flag, d.ncell * sizeof(int), cudaMemcpyDeviceToDevice, h->st));
   }
   run(h, "weno", [&] {
-    if (ex) launch_weno(d, h->st); else launch_weno_block(d, h->st);
+    if (ex) launch_weno(d, h->st); else launch_weno_block(d, h->st, 0);
     launch_weno_commit(d, h->st);
   }, 2);
   if (ex) {
@@ -923,13 +1027,18 @@ int lag2d_rhs(lag2d_handle *h, int itime, double *rhsel, int *flags) {
     run(h, "node", [&] { launch_node(d, h->st); });
     run(h, "rhs", [&] { launch_tri_rhs(d, h->st, d.us, d.vs, 0, 0.0); launch_rhs(d, h->st); }, 1 + (d.ntria > 0));
   } else {
-    if (src_launches(d)) run(h, "src", [&] { src_pass(h, d); });
-    run(h, "corner", [&] { corner_pass(h, d); }, corner_launches(h, d));
-    run(h, "node", [&] { launch_fast_node(d, h->st); });
-    run(h, "rhs", [&] { rhs_pass(h, d, 0, 0.0); }, rhs_launches(h, d));
-    // the RHS keeps ustar of the previous stage for the impedances; expose the new one
-    CK(cudaMemcpyAsync(d.us, d.us_new, d.npoin * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
-    CK(cudaMemcpyAsync(d.vs, d.vs_new, d.npoin * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
+    if (has_src(d)) run(h, "src", [&] { launch_src(h, d, h->st); });
+    const int T = d.ntria > 0;
+    run(h, "corner", [&] {
+      launch_tri_corner(d, h->st);
+      if (h->cfg.precision == 1) launch_mixed_corner(d, h->st);
+      else { launch_fast_corr(d, h->st); launch_fast_faces(d, h->st); }
+    }, 2 + T);
+    run(h, "node", [&] { launch_fast_node(d, h->st, 0, 0.0); });
+    run(h, "rhs", [&] {
+      launch_tri_rhs(d, h->st, d.us_new, d.vs_new, 0, 0.0);
+      launch_rhs_quads(h, d, h->st, 0, 0.0);
+    }, 1 + T);
   }
   r = read_status(h);
   if (h->timing) flush_timing(h);
@@ -957,6 +1066,7 @@ int lag2d_weno(lag2d_handle *h, const int *flags) {
   if (!h || !flags) return fail(LAG2D_EINVAL, "null argument");
   if (h->p1) return fail(LAG2D_EUNSUP, "WENO is not on the P1 branch");
   Dev &d = h->d;
+  sync_stage(h);
   int r = put_scalars(h, 1, 0.0, 0.0);
   if (r) return r;
   CK(cudaMemcpyAsync(h->flags_dev, flags, d.ncell * sizeof(int), cudaMemcpyHostToDevice, h->st));
@@ -974,12 +1084,13 @@ int lag2d_weno_linear(lag2d_handle *h, int transpose, const double *in, double *
   if (h->p1) return fail(LAG2D_EUNSUP, "WENO is not on the P1 branch");
   if (h->cfg.order_exact) return fail(LAG2D_EUNSUP, "the linearised WENO follows the optimised step (order_exact 0)");
   Dev &d = h->d;
+  sync_stage(h);
   const size_t nu = (size_t)NU * d.ncell;
   int r = put_scalars(h, 1, 0.0, 0.0);
   if (r) return r;
   // Persson marks and the reconstruction at the handle's state (not committed)
   run(h, "persson", [&] { launch_reset_count(d, h->st); launch_fast_persson(d, h->st); }, 2);
-  run(h, "weno", [&] { launch_weno_block(d, h->st); });
+  run(h, "weno", [&] { launch_weno_block(d, h->st, 0); });
   const int cap = std::max(1, std::min(d.nquad, 16384));
   double *vbuf = nullptr, *obuf = nullptr, *wbuf = nullptr;
   int *wslot = nullptr, *overflow = nullptr;
@@ -1023,6 +1134,7 @@ int lag2d_weno_linear(lag2d_handle *h, int transpose, const double *in, double *
 int lag2d_cellvol(lag2d_handle *h, double *geoel) {
   if (!h) return fail(LAG2D_EINVAL, "null handle");
   if (h->p1) P1_CALL(p1::cellvol(h->p1, geoel, err_));
+  sync_stage(h);
   run(h, "geom", [&] { geom_all(h, h->d.xs, h->d.ys); }, 1 + (h->d.ntria > 0));
   int r = read_status(h);
   if (r) return r;
@@ -1034,6 +1146,7 @@ int lag2d_error_norms(lag2d_handle *h, double *errl2) {
   if (!h || !errl2) return fail(LAG2D_EINVAL, "null argument");
   if (h->p1) return fail(LAG2D_EUNSUP, "the error norms are built for the P2 path");
   Dev &d = h->d;
+  sync_stage(h);
   if (d.ntria > 0) return fail(LAG2D_EUNSUP, "the error norms are built for all-quad meshes");
   if (d.ncase != 1 && d.ncase != 2)
     return fail(LAG2D_EUNSUP, "geterror_lag_curvhybrid has an exact solution for the cases 1 and 2 only");
@@ -1061,6 +1174,7 @@ int lag2d_cell_output(lag2d_handle *h, double *cellout, double *badcell) {
     P1_CALL(p1::cell_output(h->p1, cellout, err_));
   }
   Dev &d = h->d;
+  sync_stage(h);
   if (!h->cellout) {
     int r = dalloc(h, &h->cellout, 9 * (size_t)d.ncell);
     if (r) return r;
@@ -1219,7 +1333,7 @@ struct AdjWork {
         launch_fast_geom(ds, h->st, 0);
         launch_reset_count(ds, h->st);
         launch_fast_persson(ds, h->st);
-        launch_weno_block(ds, h->st);
+        launch_weno_block(ds, h->st, 0);
         launch_weno_swap(ds, h->st);
         // stage 1 reads x^n directly: its reverse folds the coordinate adjoints
         // in; the U^n fold waits for the WENO transpose (in the gather)
@@ -1265,6 +1379,8 @@ struct Snapshot {
     cudaMemcpyAsync(d.us, us + c * np, np * sizeof(double), cudaMemcpyDeviceToDevice, h->st);
     cudaMemcpyAsync(d.vs, vs + c * np, np * sizeof(double), cudaMemcpyDeviceToDevice, h->st);
     cudaMemcpyAsync(d.sc_dev, sc + c, sizeof(Scalars), cudaMemcpyDeviceToDevice, h->st);
+    cudaMemsetAsync(d.wcount, 0, 4 * sizeof(int), h->st);
+    h->stale = false;
     // cell volumes (and triangle centres) of the restored nodes: the next
     // stage 1 reads them in WENO and the time step
     launch_tri_geom(d, h->st, d.xs, d.ys);
@@ -1475,6 +1591,9 @@ void lag2d_destroy(lag2d_handle *h) {
   if (h->st) cudaStreamSynchronize(h->st);
   for (auto &p : h->pending) { cudaEventDestroy(p.second.first); cudaEventDestroy(p.second.second); }
   if (h->graph) cudaGraphExecDestroy(h->graph);
+  if (h->fork) cudaEventDestroy(h->fork);
+  for (cudaStream_t q : h->side)
+    if (q) cudaStreamDestroy(q);
   for (void *p : h->allocs) cudaFree(p);
   if (h->st) cudaStreamDestroy(h->st);
   delete h;

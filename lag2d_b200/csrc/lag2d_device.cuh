@@ -48,6 +48,10 @@ struct Dev {
   // state
   double *Un, *Us;         // U^n and the stage state
   double *xn, *yn, *xs, *ys;   // x^n and stage coordinates
+  // where a stage of the optimised step puts its result: U^(s+1) and x^(s+1).
+  // Stage 1 reads U^n, x^n themselves (Us = Un, xs = xn in its view) and the
+  // last stage writes them, so a step copies nothing back
+  double *Uo, *xo, *yo, *xt, *yt;
   double *us, *vs;         // nodal velocity ustar
   double *amatr;           // [16][ncell]
   // work
@@ -58,7 +62,8 @@ struct Dev {
   double *mapmt;           // [4][ncell] velocity-aligned frame
   double *Uw;              // [20][nquad] WENO output (high-order moments)
   int *wlist;              // compacted troubled-quad list
-  int *wcount;
+  int *wcount;             // list length; a step uses one counter per stage
+  int *dtcount;            // blocks done in the dt reduction (back to 0 after it)
   double *dtpart;          // [2][nblocks] partial minima for getdelt_lag
   Scalars *sc_dev;
   // optimised path

@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include "lag2d_device.cuh"
+#include "lag2d_dt.cuh"
 #include "lag2d_shape9.cuh"
 
 namespace lag2d {
@@ -672,6 +673,7 @@ struct WenoShared {
   double unksl[9][4][6];
   double qinvm[4][16], qmat[4][16], os[4][9], wsum[4][4][6], fch[4][4][6], unkf[4][4][6];
   double phy[4][6], rhsuk[4][6], out[4][6];
+  double xt[9][2], csum[4][3];              // target's nodes as they are; sub-cell sums of the corrections
   int cell[9], fvalid[4];
 };
 
@@ -761,9 +763,11 @@ __device__ __forceinline__ double weno_hrhs(const WenoShared &S, int is, int km,
 
 // Reconstructs troubled-list entry t with the whole block; every thread of the
 // block calls it (the early return is block-uniform).  With FACT the factors
-// go to F and nothing is written to the state.
+// go to F and nothing is written to the state.  fixcorr: d.corr holds the
+// sub-cell density corrections of the state before WENO; those of the target are
+// moved to its new tau moments.
 template <bool FACT>
-__device__ bool weno_block_cell(const Dev &d, int t, WenoShared &S, WenoFactors *F) {
+__device__ bool weno_block_cell(const Dev &d, int t, WenoShared &S, WenoFactors *F, int fixcorr = 0) {
   const int tid = threadIdx.x;
   const int iq = d.wlist[t];
   const int ielem = iq + d.ntria;
@@ -802,6 +806,7 @@ __device__ bool weno_block_cell(const Dev &d, int t, WenoShared &S, WenoFactors 
     S.xpqi[s][k][0] = d.x0[p];
     S.xpqi[s][k][1] = d.y0[p];
     double x = d.xs[p], y = d.ys[p];
+    if (s == 0) { S.xt[k][0] = x; S.xt[k][1] = y; }
     vec_local(mp, x, y);
     S.xpql[s][k][0] = x;
     S.xpql[s][k][1] = y;
@@ -1153,6 +1158,41 @@ __device__ bool weno_block_cell(const Dev &d, int t, WenoShared &S, WenoFactors 
     }
   }
   __syncthreads();
+  if (fixcorr) {
+    // corr = cdrho (rho0 V0 / V - (sum w det / tau) / V) per sub-cell: only the
+    // harmonic sum depends on the moments (getrhosubg_daverg)
+    if (tid < 100) {
+      const int isg = tid / 25, ig = tid - 25 * isg;
+      const double r = 0.5 * (cQ.g25[ig][0] + (isg == 0 || isg == 3 ? -1.0 : 1.0));
+      const double s = 0.5 * (cQ.g25[ig][1] + (isg < 2 ? -1.0 : 1.0));
+      double dr[9], ds[9];
+      shp9d(r, s, dr, ds);
+      const Jac j = jac9(S.xt, dr, ds);
+      const double det = cQ.w25[ig] * (j.xr * j.ys - j.yr * j.xs);
+      const double b1 = r - S.geo[0][0], b2 = s - S.geo[0][1];
+      const double b[6] = {1.0, b1, b2, 0.5 * b1 * b1 - S.geo[0][2], 0.5 * b2 * b2 - S.geo[0][3], b1 * b2 - S.geo[0][4]};
+      double told = S.unkrl[0][0][0], tnew = told;
+#pragma unroll
+      for (int k = 1; k < 6; k++) {
+        told += S.unkrl[0][0][k] * b[k];
+        tnew += S.out[0][k] * b[k];
+      }
+      S.rhodj[tid] = det;
+      S.xl[tid] = det / told;
+      S.yl[tid] = det / tnew;
+    }
+    __syncthreads();
+    if (tid < 12) {
+      const int isg = tid / 3, m = tid - 3 * isg;
+      const double *v = (m == 0 ? S.rhodj : m == 1 ? S.xl : S.yl) + 25 * isg;
+      double acc = 0.0;
+      for (int i = 0; i < 25; i++) acc += v[i];
+      S.csum[isg][m] = acc;
+    }
+    __syncthreads();
+    if (tid < 4) d.corr[tid * nq + iq] += d.cdrho * (S.csum[tid][1] - S.csum[tid][2]) / S.csum[tid][0];
+    __syncthreads();
+  }
   return true;
 }
 
@@ -1488,12 +1528,12 @@ __global__ void k_weno_gather(Dev d, double *lamU, double *lamUn, int fold, cons
   for (int v = 0; v < 24; v++) lamU[v * nc + e] = l[v];
 }
 
-__global__ void __launch_bounds__(kWenoThreads) k_weno_block(Dev d) {
+__global__ void __launch_bounds__(kWenoThreads) k_weno_block(Dev d, int fixcorr) {
   extern __shared__ __align__(16) unsigned char wsm[];
   WenoShared &S = *reinterpret_cast<WenoShared *>(wsm);
   if (stopped(d)) return;
   const int n = *d.wcount;
-  for (int t = blockIdx.x; t < n; t += gridDim.x) weno_block_cell<false>(d, t, S, nullptr);
+  for (int t = blockIdx.x; t < n; t += gridDim.x) weno_block_cell<false>(d, t, S, nullptr, fixcorr);
 }
 
 
@@ -1955,20 +1995,6 @@ __host__ __device__ void b_dt_values(const Dev &d, int iq, double &dtcfl, double
   dtvol = d.vol[e] / fabs(d.rhs[(0 * NDEG + 0) * d.ncell + e]);
 }
 
-// dtfix from the global minima (getdelt_lag :20705-20709, getsolvdg_lag :1766-1773)
-__host__ __device__ void b_dt_apply(const Dev &d, double mcfl, double mvol, int ndt) {
-  Scalars *S = d.sc_dev;
-  double dt = S->dtfix;
-  if (ndt == 1) {
-    double dtcfl = fmin(1e10, mcfl), dtvol = fmin(1e10, mvol);
-    if (S->itime == 1) dt = fmin(d.cfl * dtcfl, 0.1 * dtvol);
-    else dt = fmin(fmin(d.cfl * dtcfl, 0.1 * dtvol), 1.01 * dt);
-    if ((S->tacru + dt) > d.tend) dt = d.tend - S->tacru;
-  }
-  S->dtfix = dt;
-  S->tacru = S->tacru + dt;
-}
-
 // per-block minima; min is exact, so the reduction is order independent
 __global__ void k_dt_partial(Dev d) {
   __shared__ double sm_cfl[256], sm_vol[256];
@@ -2008,7 +2034,7 @@ __global__ void k_dt_final(Dev d, int nblk, int ndt) {
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) b_dt_apply(d, sm_cfl[0], sm_vol[0], ndt);
+  if (threadIdx.x == 0) dt_apply(d, sm_cfl[0], sm_vol[0], ndt);
 }
 
 // ---------------------------------------------------------------------------
@@ -2090,8 +2116,10 @@ __host__ __device__ void b_step_begin(const Dev &d, int itime) {
 }
 __global__ void k_step_begin(Dev d, int itime) { b_step_begin(d, itime); }
 
+// exit test; the WENO lists start the next step empty
 __host__ __device__ void b_step_end(const Dev &d, int check_done) {
   Scalars *S = d.sc_dev;
+  for (int i = 0; i < 3; i++) d.wcount[i] = 0;
   if (S->done) return;
   if (check_done && fabs(S->tacru - d.tend) / d.tend <= 1e-11) S->done = 1;
 }
@@ -2971,7 +2999,7 @@ __host__ __device__ void b_tri_rhs(const Dev &d, int it, const double *usn, cons
       for (int q = 0; q < 4; q++) unint[q] = unint[q] + mm[id][iu] * (dt * R[q][iu]);
     for (int q = 0; q < 4; q++) {
       const int idx = (q * NDEG + id) * d.ncell + e;
-      d.Us[idx] = alfa * d.Un[idx] + oma * (d.Us[idx] + unint[q]);
+      d.Uo[idx] = alfa * d.Un[idx] + oma * (d.Us[idx] + unint[q]);
     }
   }
 }
@@ -3603,8 +3631,8 @@ void launch_error(const Dev &d, cudaStream_t st, const double *X, const double *
 void launch_weno(const Dev &d, cudaStream_t st) { k_weno<<<nblk(d.nquad, 64), 64, 0, st>>>(d); }
 // one block per troubled quad, a grid of at most 3 blocks per SM looping over the list
 static int weno_grid(const Dev &d) { return d.nquad < 444 ? (d.nquad > 0 ? d.nquad : 1) : 444; }
-void launch_weno_block(const Dev &d, cudaStream_t st) {
-  k_weno_block<<<weno_grid(d), kWenoThreads, sizeof(WenoShared), st>>>(d);
+void launch_weno_block(const Dev &d, cudaStream_t st, int fixcorr) {
+  k_weno_block<<<weno_grid(d), kWenoThreads, sizeof(WenoShared), st>>>(d, fixcorr);
 }
 void launch_weno_linear(const Dev &d, cudaStream_t st, int mode, const double *v, double *out, double *wbuf,
                         int *wslot, int cap, int *overflow) {
@@ -3636,7 +3664,6 @@ void launch_dt(const Dev &d, cudaStream_t st, int ndt) {
   k_dt_partial<<<nb, 256, 0, st>>>(d);
   k_dt_final<<<1, 256, 0, st>>>(d, nb, ndt);
 }
-void launch_dt_final(const Dev &d, cudaStream_t st, int nb, int ndt) { k_dt_final<<<1, 256, 0, st>>>(d, nb, ndt); }
 void launch_update(const Dev &d, cudaStream_t st, double alfa) {
   k_update<<<nblk(d.ncell, 128), 128, 0, st>>>(d, alfa);
 }

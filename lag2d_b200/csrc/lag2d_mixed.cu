@@ -749,14 +749,14 @@ __device__ void m_rhs(const Dev &d, int iq, int fuse_update, double alfa, double
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     const size_t base = (size_t)(q * 6) * d.ncell + e;
-    d.Us[base] = alfa * MX_UN(q * 6) + oma * (MX_U(q, 0) + MX_AM(15) * (dt * R[q][0]));
+    d.Uo[base] = alfa * MX_UN(q * 6) + oma * (MX_U(q, 0) + MX_AM(15) * (dt * R[q][0]));
 #pragma unroll
     for (int i = 0; i < 5; i++) {
       double acc = 0.0;
 #pragma unroll
       for (int j = 0; j < 5; j++) acc += MX_AM(IDX[i][j]) * (dt * R[q][j + 1]);
       const size_t idx = base + (size_t)(i + 1) * d.ncell;
-      d.Us[idx] = alfa * MX_UN(q * 6 + i + 1) + oma * (MX_U(q, i + 1) + acc);
+      d.Uo[idx] = alfa * MX_UN(q * 6 + i + 1) + oma * (MX_U(q, i + 1) + acc);
     }
   }
 #undef MX_U
