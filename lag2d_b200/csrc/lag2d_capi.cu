@@ -59,6 +59,8 @@ void launch_init_wmom(const Dev &d, cudaStream_t st);
 void launch_tri_init(const Dev &d, cudaStream_t st);
 void launch_tri_geom(const Dev &d, cudaStream_t st, const double *X, const double *Y);
 void launch_tri_corner(const Dev &d, cudaStream_t st);
+void launch_fast_tri_corner(const Dev &d, cudaStream_t st);
+void launch_fast_tri_rhs(const Dev &d, cudaStream_t st, const double *usn, const double *vsn, int fuse, double alfa);
 void launch_tri_rhs(const Dev &d, cudaStream_t st, const double *usn, const double *vsn, int fuse, double alfa);
 void launch_adjoint_stage(const Dev &d, const void *adj, cudaStream_t st, double alfa, const double *dtp, int fold,
                           int fold_u, int mixed);
@@ -407,6 +409,7 @@ static void enqueue_step_fast(lag2d_handle *h, int itime, const StageRec *rec = 
     d.Uo = last ? d0.Un : d0.Us;
     d.xo = last ? d0.xn : istag == 1 ? d0.xs : d0.xt;
     d.yo = last ? d0.yn : istag == 1 ? d0.ys : d0.yt;
+    d.tcf = nullptr;  // the triangles' corner coefficients are kept only for the adjoint
     d.us_new = d0.us;
     d.vs_new = d0.vs;
     d.wcount = d0.wcount + (istag - 1);
@@ -431,7 +434,7 @@ static void enqueue_step_fast(lag2d_handle *h, int itime, const StageRec *rec = 
     }
     if (T) {
       after(s2, s0);
-      run(h, "corner", [&] { launch_tri_corner(d, s2); });
+      run(h, "corner", [&] { launch_fast_tri_corner(d, s2); });
     }
     if (!mixed) {
       after(s1, s0);
@@ -462,7 +465,7 @@ static void enqueue_step_fast(lag2d_handle *h, int itime, const StageRec *rec = 
     run(h, "geom", [&] { launch_tri_geom(dx, s2, dx.xs, dx.ys); launch_fast_geom(dx, s2, 1); }, 1 + T);
     if (T) {
       after(s1, s0);
-      run(h, "rhs", [&] { launch_tri_rhs(d, s1, d.us_new, d.vs_new, 1, alfa); });
+      run(h, "rhs", [&] { launch_fast_tri_rhs(d, s1, d.us_new, d.vs_new, 1, alfa); });
     }
     run(h, "rhs", [&] { launch_rhs_quads(h, d, s0, 1, alfa); });
     if (mixed && istag == 1) run(h, "weno", [&] { launch_weno_swap(d, s0); });
@@ -1030,13 +1033,13 @@ int lag2d_rhs(lag2d_handle *h, int itime, double *rhsel, int *flags) {
     if (has_src(d)) run(h, "src", [&] { launch_src(h, d, h->st); });
     const int T = d.ntria > 0;
     run(h, "corner", [&] {
-      launch_tri_corner(d, h->st);
+      launch_fast_tri_corner(d, h->st);
       if (h->cfg.precision == 1) launch_mixed_corner(d, h->st);
       else { launch_fast_corr(d, h->st); launch_fast_faces(d, h->st); }
     }, 2 + T);
     run(h, "node", [&] { launch_fast_node(d, h->st, 0, 0.0); });
     run(h, "rhs", [&] {
-      launch_tri_rhs(d, h->st, d.us_new, d.vs_new, 0, 0.0);
+      launch_fast_tri_rhs(d, h->st, d.us_new, d.vs_new, 0, 0.0);
       launch_rhs_quads(h, d, h->st, 0, 0.0);
     }, 1 + T);
   }
