@@ -218,7 +218,8 @@ int lag2d_adjoint_step(lag2d_handle *h, int itime, double *dtfix, double *tacru,
  * unkno, coord and ustar.  Checkpoints are taken every checkpoint_every steps;
  * each segment is recomputed once on the reverse sweep, so device memory is
  * (nsteps / checkpoint_every + 1) states plus checkpoint_every steps of RK
- * stage inputs.  dtfix and tacru are in/out as in lag2d_step; the handle ends
+ * stage inputs; the handle keeps up to 1 GiB of it for the next adjoint call.
+ * dtfix and tacru are in/out as in lag2d_step; the handle ends
  * at the final state.  ms[3] (may be NULL) receives the device time of the
  * forward pass, of the segment recomputes and of the reverse sweep. */
 int lag2d_adjoint(lag2d_handle *h, int itime0, int nsteps, int checkpoint_every, double *dtfix,

@@ -70,6 +70,7 @@ void launch_weno_gather(const Dev &d, cudaStream_t st, double *lamU, double *lam
                         const int *wslot, int cap, const int *inv_ptr, const int *inv_ent);
 void launch_weno_swap(const Dev &d, cudaStream_t st);
 int adjoint_stage_launches(const Dev &d);
+int launch_energy_seed(const Dev &d, cudaStream_t st, double *lU, double *part);
 int error_blocks(const Dev &d);
 void launch_error(const Dev &d, cudaStream_t st, const double *X, const double *Y, double *part);
 void launch_cell_output(const Dev &d, cudaStream_t st, const double *U, const double *X, const double *Y,
@@ -132,6 +133,10 @@ struct lag2d_handle {
   // quads c whose stencil position s is j, c ascending (the WENO transpose's
   // fixed summation order)
   int *sinv_ptr = nullptr, *sinv_ent = nullptr;
+  // device memory of the adjoint calls, kept from one call to the next up to
+  // kArenaKeep bytes (a larger window's is freed when the call returns)
+  char *arena = nullptr;
+  size_t arena_bytes = 0;
 };
 
 template <typename T>
@@ -1246,9 +1251,10 @@ double lag2d_kernel_ms(const lag2d_handle *h, const char *family, long long *lau
 // The stage inputs are recorded by recomputing each checkpoint segment, so the
 // device memory of a window is (segments + 1) checkpoints plus K steps of
 // stage records.
+constexpr size_t kArenaKeep = (size_t)1 << 30;
 struct AdjWork {
   lag2d_handle *h;
-  std::vector<void *> mem;
+  std::vector<std::pair<void **, size_t>> want;
   Adj a{};
   StageRec rec{};
   int rc = LAG2D_OK;
@@ -1260,21 +1266,40 @@ struct AdjWork {
   explicit AdjWork(lag2d_handle *hh) : h(hh) {}
   ~AdjWork() {
     cudaStreamSynchronize(h->st);
-    for (void *q : mem) cudaFree(q);
+    if (h->arena_bytes > kArenaKeep) {
+      cudaFree(h->arena);
+      h->arena = nullptr;
+      h->arena_bytes = 0;
+    }
   }
   template <typename T> void alloc(T **p, size_t n) {
-    if (rc != LAG2D_OK) return;
-    void *q = nullptr;
-    const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
-    cudaError_t e = cudaMalloc(&q, bytes);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      rc = fail(LAG2D_ECUDA, std::string("cudaMalloc (adjoint): ") + cudaGetErrorString(e));
-      return;
+    want.push_back({(void **)p, (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256});
+  }
+  // One block for all requests, zeroed: the window's forty buffers were
+  // allocated, cleared and freed on every call, 20 ms of a 256 x 256 window
+  // whose device work takes 9.
+  int commit() {
+    size_t total = 0;
+    for (auto &w : want) total += w.second;
+    if (h->arena_bytes < total) {
+      cudaFree(h->arena);
+      h->arena = nullptr;
+      h->arena_bytes = 0;
+      const cudaError_t e = cudaMalloc((void **)&h->arena, total);
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        h->arena = nullptr;
+        return rc = fail(LAG2D_ECUDA, std::string("cudaMalloc (adjoint): ") + cudaGetErrorString(e));
+      }
+      h->arena_bytes = total;
     }
-    cudaMemsetAsync(q, 0, bytes, h->st);
-    mem.push_back(q);
-    *p = static_cast<T *>(q);
+    CK(cudaMemsetAsync(h->arena, 0, total, h->st));
+    char *q = h->arena;
+    for (auto &w : want) {
+      *w.first = q;
+      q += w.second;
+    }
+    return LAG2D_OK;
   }
   // adjoint buffers plus the stage records of K steps
   void setup(int K) {
@@ -1400,53 +1425,45 @@ static int adjoint_supported(lag2d_handle *h) {
 }
 
 // caller layouts <-> device SoA for the adjoint fields
+// the layout conversions read and write the view's U^n slab
 static int put_adjoint(lag2d_handle *h, const Adj &a, const double *unkno, const double *coord,
                        const double *ustar) {
   const Dev &d = h->d;
-  const size_t nc = d.ncell, np = d.npoin, nu = (size_t)NU * nc;
-  std::vector<double> g(nu, 0.0);
-  if (unkno)
-    for (size_t e = 0; e < nc; e++)
-      for (int t = 0; t < NU; t++) g[(size_t)t * nc + e] = unkno[e * NU + t];
-  CK(cudaMemcpyAsync(a.lU, g.data(), nu * sizeof(double), cudaMemcpyHostToDevice, h->st));
-  CK(cudaStreamSynchronize(h->st));
-  const double *src[2] = {coord, ustar};
-  double *dst[2][2] = {{a.lx, a.ly}, {a.lus, a.lvs}};
-  std::vector<double> gx(np), gy(np);
-  for (int f = 0; f < 2; f++) {
-    for (size_t p = 0; p < np; p++) {
-      gx[p] = src[f] ? src[f][2 * p] : 0.0;
-      gy[p] = src[f] ? src[f][2 * p + 1] : 0.0;
-    }
-    CK(cudaMemcpyAsync(dst[f][0], gx.data(), np * sizeof(double), cudaMemcpyHostToDevice, h->st));
-    CK(cudaMemcpyAsync(dst[f][1], gy.data(), np * sizeof(double), cudaMemcpyHostToDevice, h->st));
-    CK(cudaStreamSynchronize(h->st));
+  const size_t np = d.npoin, nu = (size_t)NU * d.ncell;
+  if (unkno) {
+    Dev v = d;
+    v.Un = a.lU;
+    CK(cudaMemcpyAsync(h->stage_u, unkno, nu * sizeof(double), cudaMemcpyHostToDevice, h->st));
+    launch_unkno_in(v, h->st, h->stage_u, 0);
+  } else {
+    CK(cudaMemsetAsync(a.lU, 0, nu * sizeof(double), h->st));
   }
+  const double *src[2] = {coord, ustar};
+  double *dst[2][2] = {{a.lx, a.ly}, {a.lus, a.lvs}}, *stage[2] = {h->stage_x, h->stage_v};
+  for (int f = 0; f < 2; f++) {
+    if (src[f]) {
+      CK(cudaMemcpyAsync(stage[f], src[f], 2 * np * sizeof(double), cudaMemcpyHostToDevice, h->st));
+      launch_xy_in((int)np, h->st, stage[f], dst[f][0], dst[f][1], nullptr, nullptr);
+    } else {
+      for (double *q : dst[f]) CK(cudaMemsetAsync(q, 0, np * sizeof(double), h->st));
+    }
+  }
+  h->launches += (unkno != nullptr) + (coord != nullptr) + (ustar != nullptr);
   return LAG2D_OK;
 }
 static int get_adjoint(lag2d_handle *h, const Adj &a, double *unkno, double *coord, double *ustar) {
   const Dev &d = h->d;
-  const size_t nc = d.ncell, np = d.npoin, nu = (size_t)NU * nc;
-  if (unkno) {
-    std::vector<double> g(nu);
-    CK(cudaMemcpyAsync(g.data(), a.lU, nu * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-    CK(cudaStreamSynchronize(h->st));
-    for (size_t e = 0; e < nc; e++)
-      for (int t = 0; t < NU; t++) unkno[e * NU + t] = g[(size_t)t * nc + e];
-  }
-  const double *src[2][2] = {{a.lx, a.ly}, {a.lus, a.lvs}};
-  double *dst[2] = {coord, ustar};
-  std::vector<double> gx(np), gy(np);
-  for (int f = 0; f < 2; f++) {
-    if (!dst[f]) continue;
-    CK(cudaMemcpyAsync(gx.data(), src[f][0], np * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-    CK(cudaMemcpyAsync(gy.data(), src[f][1], np * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-    CK(cudaStreamSynchronize(h->st));
-    for (size_t p = 0; p < np; p++) {
-      dst[f][2 * p] = gx[p];
-      dst[f][2 * p + 1] = gy[p];
-    }
-  }
+  const size_t np = d.npoin, nu = (size_t)NU * d.ncell;
+  Dev v = d;
+  v.Un = a.lU;
+  if (unkno) launch_unkno_out(v, h->st, h->stage_u);
+  if (coord) launch_xy_out((int)np, h->st, h->stage_x, a.lx, a.ly);
+  if (ustar) launch_xy_out((int)np, h->st, h->stage_v, a.lus, a.lvs);
+  h->launches += (unkno != nullptr) + (coord != nullptr) + (ustar != nullptr);
+  if (unkno) CK(cudaMemcpyAsync(unkno, h->stage_u, nu * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  if (coord) CK(cudaMemcpyAsync(coord, h->stage_x, 2 * np * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  if (ustar) CK(cudaMemcpyAsync(ustar, h->stage_v, 2 * np * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  CK(cudaStreamSynchronize(h->st));
   return LAG2D_OK;
 }
 
@@ -1460,7 +1477,9 @@ int lag2d_adjoint_step(lag2d_handle *h, int itime, double *dtfix, double *tacru,
   if (r) return r;
   AdjWork w(h);
   w.setup(1);
-  if (w.rc) return w.rc;
+  Snapshot out;
+  out.alloc(w, 1);
+  if ((r = w.commit())) return r;
   r = put_scalars(h, itime, *dtfix, *tacru);
   if (r) return r;
   w.record(itime, 1);
@@ -1473,9 +1492,6 @@ int lag2d_adjoint_step(lag2d_handle *h, int itime, double *dtfix, double *tacru,
   r = put_adjoint(h, w.a, seed_unkno, seed_coord, seed_ustar);
   if (r) return r;
   // keep the step's outputs: the reverse pass overwrites the stage buffers
-  Snapshot out;
-  out.alloc(w, 1);
-  if (w.rc) return w.rc;
   out.save(h, 0);
   w.reverse(1);
   out.restore(h, 0);
@@ -1500,12 +1516,13 @@ int lag2d_adjoint(lag2d_handle *h, int itime0, int nsteps, int checkpoint_every,
   Dev &d = h->d;
   const int K = std::min(checkpoint_every, nsteps);
   const int nseg = (nsteps + K - 1) / K;
-  const size_t nc = d.ncell, nu = (size_t)NU * nc;
   AdjWork w(h);
   w.setup(K);
   Snapshot ck;
   ck.alloc(w, nseg + 1);
-  if (w.rc) return w.rc;
+  double *part = nullptr;
+  w.alloc(&part, 1024);
+  if ((r = w.commit())) return r;
   cudaEvent_t ev[2];
   CK(cudaEventCreate(&ev[0]));
   CK(cudaEventCreate(&ev[1]));
@@ -1521,13 +1538,16 @@ int lag2d_adjoint(lag2d_handle *h, int itime0, int nsteps, int checkpoint_every,
   };
   double t_fwd = 0, t_rec = 0, t_rev = 0;
   // forward with a checkpoint at every segment start and at the end
-  r = put_scalars(h, itime0, *dtfix, *tacru);
+  r = put_scalars(h, itime0 - 1, *dtfix, *tacru);
   if (r) return r;
+  if ((r = step_graph(h))) return r;
   cudaEventRecord(ev[0], h->st);
   for (int n = 0; n < nsteps; n++) {
     if (n % K == 0) ck.save(h, n / K);
-    enqueue_step_fast(h, itime0 + n);
+    CK(cudaGraphLaunch(h->graph, h->st));
+    h->launches += h->graph_launches;
   }
+  h->stale = true;
   ck.save(h, nseg);
   cudaEventRecord(ev[1], h->st);
   t_fwd = elapsed();
@@ -1539,21 +1559,13 @@ int lag2d_adjoint(lag2d_handle *h, int itime0, int nsteps, int checkpoint_every,
     return fail(LAG2D_EINVAL, "the window runs past tend (the steps after it are skipped)");
   // J and its seed dJ/dU = m (0, u, v, 0) in the cell-average modes
   {
-    std::vector<double> u(nc), v(nc), m(nc);
-    CK(cudaMemcpyAsync(u.data(), d.Un + 6 * nc, nc * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-    CK(cudaMemcpyAsync(v.data(), d.Un + 12 * nc, nc * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-    CK(cudaMemcpyAsync(m.data(), d.mass, nc * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+    std::vector<double> pj(launch_energy_seed(d, h->st, w.a.lU, part));
+    h->launches += 1;
+    CK(cudaMemcpyAsync(pj.data(), part, pj.size() * sizeof(double), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     double s = 0.0;
-    std::vector<double> seed(nu, 0.0);
-    for (size_t e = 0; e < nc; e++) {
-      s += 0.5 * m[e] * (u[e] * u[e] + v[e] * v[e]);
-      seed[6 * nc + e] = m[e] * u[e];
-      seed[12 * nc + e] = m[e] * v[e];
-    }
+    for (double v : pj) s += v;
     *J = s;
-    CK(cudaMemcpyAsync(w.a.lU, seed.data(), nu * sizeof(double), cudaMemcpyHostToDevice, h->st));
-    CK(cudaStreamSynchronize(h->st));
   }
   // reverse sweep, one segment at a time: recompute it from its checkpoint
   // with the stage inputs recorded, then run its steps backwards
@@ -1598,6 +1610,7 @@ void lag2d_destroy(lag2d_handle *h) {
   for (cudaStream_t q : h->side)
     if (q) cudaStreamDestroy(q);
   for (void *p : h->allocs) cudaFree(p);
+  cudaFree(h->arena);
   if (h->st) cudaStreamDestroy(h->st);
   delete h;
 }

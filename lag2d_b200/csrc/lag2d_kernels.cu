@@ -2096,6 +2096,26 @@ __host__ __device__ void b_nodes(const Dev &d, int p, double alfa) {
 }
 __global__ void k_nodes(Dev d, double alfa) { b_nodes(d, blockIdx.x * blockDim.x + threadIdx.x, alfa); }
 
+// Kinetic energy of the cell averages, J = sum m (u^2 + v^2) / 2, as partial sums
+// of a fixed number of blocks in a fixed order, and its derivative in lU
+__global__ void __launch_bounds__(256) k_energy_seed(Dev d, double *lU, double *part) {
+  __shared__ double sm[256];
+  const size_t nc = d.ncell;
+  double j = 0.0;
+  for (size_t e = blockIdx.x * (size_t)256 + threadIdx.x; e < nc; e += (size_t)gridDim.x * 256) {
+    const double m = d.mass[e], u = d.Un[6 * nc + e], v = d.Un[12 * nc + e];
+    j += 0.5 * m * (u * u + v * v);
+    for (int k = 0; k < NU; k++) lU[k * nc + e] = k == 6 ? m * u : k == 12 ? m * v : 0.0;
+  }
+  sm[threadIdx.x] = j;
+  __syncthreads();
+  for (int s = 128; s > 0; s >>= 1) {
+    if (threadIdx.x < s) sm[threadIdx.x] += sm[threadIdx.x + s];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
+}
+
 // Driver copy-back (dgflo2d.f90:407-423) and exit test (dgflo2d.f90:459)
 __host__ __device__ void b_copyback(const Dev &d, int i, int stride) {
   if (stopped(d)) return;
@@ -3669,6 +3689,12 @@ void launch_update(const Dev &d, cudaStream_t st, double alfa) {
 }
 void launch_nodes(const Dev &d, cudaStream_t st, double alfa) {
   k_nodes<<<nblk(d.npoin, 256), 256, 0, st>>>(d, alfa);
+}
+// returns the number of partial sums (at most 1024)
+int launch_energy_seed(const Dev &d, cudaStream_t st, double *lU, double *part) {
+  const int g = d.ncell < 256 * 592 ? nblk(d.ncell, 256) : 592;
+  k_energy_seed<<<g, 256, 0, st>>>(d, lU, part);
+  return g;
 }
 void launch_copyback(const Dev &d, cudaStream_t st) { k_copyback<<<1184, 256, 0, st>>>(d); }
 void launch_step_begin(const Dev &d, cudaStream_t st, int itime) { k_step_begin<<<1, 1, 0, st>>>(d, itime); }
