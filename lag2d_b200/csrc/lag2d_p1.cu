@@ -31,18 +31,14 @@
 // barthlimit_sympre_quadlb writes only geoel(10), which this branch never
 // reads.  With order_exact the kernels keep the reference's expression and
 // summation order, so the build with --fmad=false reproduces the CPU
-// restatement bit for bit; the optimised form (order_exact 0) sums the two
-// faces of each corner before the node gather and the face integral, takes
-// the volume of the straight quad in closed form and evaluates the limiter
-// function with one division.
+// restatement bit for bit; the optimised form (order_exact 0) has its own
+// kernels, described in lag2d_p1_fast.cuh.
 //
 // Layout in HBM (0-based, structure of arrays):
 //   U[(q*3 + k)*ncell + e]        P1 DOF k of field q (tau, u, v, e)
 //   ipq[k*nquad + iq]             vertex k (0..3, counter-clockwise) of quad iq
 //   cf[(v*8 + f + 2*iv)*nquad+iq] corner-face coefficient v (m, m u, m v,
 //                                 sigma.n A x, y) of corner iv, face f
-//                                 (optimised kernels: cf[(v*4 + iv)*nquad+iq],
-//                                 the two faces of corner iv summed)
 //   lim[k*ncell + e]              aflim(1), aflim(4), aflim(5), afvec(1,1),
 //                                 afvec(1,2), afvec(2,1), afvec(2,2)
 #include <cuda_runtime.h>
@@ -91,6 +87,11 @@ struct Dev1 {
   double *rc, *sc, *vol, *vcx, *vcy, *mass, *amatr;  // amatr [4][ncell]
   double *Un, *Us;                    // [12][ncell]
   double *xn, *yn, *xs, *ys, *us, *vs;
+  // where a stage of the optimised step puts its result (stage 1 reads U^n, x^n
+  // themselves, the last stage writes them); xt, yt: coordinates of stage 3
+  double *Uo, *xo, *yo, *xt, *yt;
+  double *pbar;                       // [ncell] cell-average pressures (optimised step)
+  int *count;                         // blocks done: dt reduction, last RHS pass
   double *bmax, *bmin;                // [5][npoin]
   double *lim;                        // [7][ncell]
   double *cf;                         // [5][8][nquad]
@@ -383,28 +384,6 @@ __global__ void k1_geom(Dev1 d, const double *X, const double *Y) {
     d.vcy[iq] = scvrz / areel;
     d.rbar[iq] = volel / areel;
   }
-  if (!(volel > 0.0)) atomicOr(&d.sc_dev->status, ST_NONPHYS);
-}
-
-// The same volume and volume centre in closed form: the 9-node image of a
-// straight quad is its bilinear map, whose Jacobian is J0 + J1 r + J2 s, so
-// V = 4 J0 and the centre in reference coordinates is (J1, J2) / (3 J0).
-__global__ void k1_geom_fast(Dev1 d, const double *X, const double *Y) {
-  const int iq = blockIdx.x * blockDim.x + threadIdx.x;
-  if (iq >= d.nquad || stopped(d)) return;
-  double x[4][2];
-  load4(d, X, Y, iq, x);
-  const double e1 = 0.25 * (-x[0][0] + x[1][0] + x[2][0] - x[3][0]);
-  const double e2 = 0.25 * (-x[0][0] - x[1][0] + x[2][0] + x[3][0]);
-  const double e3 = 0.25 * (x[0][0] - x[1][0] + x[2][0] - x[3][0]);
-  const double f1 = 0.25 * (-x[0][1] + x[1][1] + x[2][1] - x[3][1]);
-  const double f2 = 0.25 * (-x[0][1] - x[1][1] + x[2][1] + x[3][1]);
-  const double f3 = 0.25 * (x[0][1] - x[1][1] + x[2][1] - x[3][1]);
-  const double j0 = e1 * f2 - f1 * e2, j1 = e1 * f3 - f1 * e3, j2 = e3 * f2 - f3 * e2;
-  const double volel = 4.0 * j0;
-  d.vol[iq] = volel;
-  d.vcx[iq] = j1 / (3.0 * j0);
-  d.vcy[iq] = j2 / (3.0 * j0);
   if (!(volel > 0.0)) atomicOr(&d.sc_dev->status, ST_NONPHYS);
 }
 
@@ -1065,8 +1044,14 @@ __device__ void aw_node(const Dev1 &d, int p) {
   d.vs[p] = vs;
 }
 
+// motion of the optimised step (stages after the first)
+__device__ __forceinline__ void move_node(const Dev1 &d, int p, double alfa) {
+  const double dt = d.sc_dev->dtfix, oma = 1.0 - alfa;
+  d.xo[p] = alfa * d.xn[p] + oma * (d.xs[p] + dt * d.us[p]);
+  d.yo[p] = alfa * d.yn[p] + oma * (d.ys[p] + dt * d.vs[p]);
+}
 template <bool FAST, int GEO>
-__global__ void k1_node(Dev1 d) {
+__global__ void k1_node(Dev1 d, int move = 0, double alfa = 0.0) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= d.npoin || stopped(d)) return;
   if (GEO == 1) {
@@ -1117,6 +1102,7 @@ __global__ void k1_node(Dev1 d) {
   if (bc & (BC_U0 | BC_UV0)) us = 0.0;
   d.us[p] = us;
   d.vs[p] = vs;
+  if (FAST && move) move_node(d, p, alfa);
 }
 
 // ---------------------------------------------------------------------------
@@ -1163,7 +1149,7 @@ __device__ void update_cell(const Dev1 &d, int e, double alfa, const double (*R)
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const size_t idx = (q * ND + id) * nc + e;
-      d.Us[idx] = alfa * d.Un[idx] + oma * (s[q][id] + unint[q]);
+      d.Uo[idx] = alfa * d.Un[idx] + oma * (s[q][id] + unint[q]);
     }
   }
 }
@@ -1289,8 +1275,12 @@ __device__ void aw_faces(const Dev1 &d, int iq, const double (*x4)[2], double rc
   }
 }
 
+// one thread per cell over the 25 points, latency-bound on its FP64 chain: FAST
+// keeps 4 blocks of 128 resident (128 registers, no spills) and writes the update:
+// 148 us a launch at 1024 x 512 against 145 at 168 registers plus 54 for an update
+// kernel of its own
 template <int MD, bool FAST, int GEO>
-__global__ void __launch_bounds__(128) k1_rhs(Dev1 d, int fuse, double alfa) {
+__global__ void __launch_bounds__(128, FAST ? 4 : 1) k1_rhs(Dev1 d, int fuse, double alfa) {
   const int iq = blockIdx.x * blockDim.x + threadIdx.x;
   if (iq >= d.nquad || stopped(d)) return;
   const int e = iq;
@@ -1522,6 +1512,19 @@ __global__ void __launch_bounds__(128) k1_rhs(Dev1 d, int fuse, double alfa) {
 // ---------------------------------------------------------------------------
 // getdelt_lag (Getrhslag.f90:20600-20716, straight edges :20649-20654)
 // ---------------------------------------------------------------------------
+// the step size from the mesh minima (:20705-20709; getsolvdg_lag :1766-1773)
+__device__ __forceinline__ void dt_apply1(const Dev1 &d, double mcfl, double mvol, int ndt) {
+  Scalars *S = d.sc_dev;
+  double dt = S->dtfix;
+  if (ndt == 1) {
+    const double dtcfl = fmin(1e10, mcfl), dtvol = fmin(1e10, mvol);
+    if (S->itime == 1) dt = fmin(d.cfl * dtcfl, 0.1 * dtvol);
+    else dt = fmin(fmin(d.cfl * dtcfl, 0.1 * dtvol), 1.01 * dt);
+    if ((S->tacru + dt) > d.tend) dt = d.tend - S->tacru;
+  }
+  S->dtfix = dt;
+  S->tacru = S->tacru + dt;
+}
 __global__ void k1_dt_partial(Dev1 d) {
   __shared__ double sm_cfl[256], sm_vol[256];
   const int iq = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1580,16 +1583,7 @@ __global__ void k1_dt_final(Dev1 d, int nblk, int ndt) {
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    Scalars *S = d.sc_dev;
-    double dt = S->dtfix;
-    if (ndt == 1) {
-      const double dtcfl = fmin(1e10, sm_cfl[0]), dtvol = fmin(1e10, sm_vol[0]);
-      if (S->itime == 1) dt = fmin(d.cfl * dtcfl, 0.1 * dtvol);
-      else dt = fmin(fmin(d.cfl * dtcfl, 0.1 * dtvol), 1.01 * dt);
-      if ((S->tacru + dt) > d.tend) dt = d.tend - S->tacru;
-    }
-    S->dtfix = dt;
-    S->tacru = S->tacru + dt;
+    dt_apply1(d, sm_cfl[0], sm_vol[0], ndt);
   }
 }
 
@@ -1642,6 +1636,8 @@ __global__ void k1_unkno_out(Dev1 d, const double *src, double *aos) {
   }
 }
 
+#include "lag2d_p1_fast.cuh"
+
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
@@ -1683,7 +1679,13 @@ struct Solver {
   lag2d_config cfg{};
   cudaStream_t st = nullptr;
   std::vector<void *> allocs;
+  char *block = nullptr;  // what is left of the newest block of dalloc
+  size_t block_left = 0;
   double *stage_u = nullptr, *stage_x = nullptr, *cellout = nullptr;
+  bool stale = false;  // the optimised step leaves its result in U^n, x^n only
+  cudaStream_t side = nullptr;  // of the captured step: passes beside the main chain
+  cudaEvent_t fork = nullptr;
+  bool forking = false;
   cudaGraphExec_t graph = nullptr;
   long long graph_launches = 0, launches = 0;
   bool timing = false;
@@ -1693,13 +1695,27 @@ struct Solver {
 
 static int nb(int n, int t) { return std::max(1, (n + t - 1) / t); }
 
+// zeroed device memory; the many small arrays of a small mesh come out of shared
+// blocks, since each cudaMalloc costs some 10 us of the handle's set-up
 template <typename T>
 static bool dalloc(Solver *s, T **p, size_t n) {
-  void *q = nullptr;
-  if (cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) return false;
-  cudaMemsetAsync(q, 0, std::max<size_t>(n, 1) * sizeof(T), s->st);
-  s->allocs.push_back(q);
-  *p = static_cast<T *>(q);
+  const size_t kBlock = 2 << 20, bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
+  if (bytes > s->block_left) {
+    void *q = nullptr;
+    const size_t get = std::max(bytes, kBlock);
+    if (cudaMalloc(&q, get) != cudaSuccess) return false;
+    cudaMemsetAsync(q, 0, get, s->st);
+    s->allocs.push_back(q);
+    if (bytes >= kBlock) {
+      *p = static_cast<T *>(q);
+      return true;
+    }
+    s->block = static_cast<char *>(q);
+    s->block_left = get;
+  }
+  *p = reinterpret_cast<T *>(s->block);
+  s->block += bytes;
+  s->block_left -= bytes;
   return true;
 }
 
@@ -1744,40 +1760,29 @@ static void flush_timing(Solver *s) {
 
 static const double kRK[2][3] = {{0.0, 0.5, 0.0}, {0.0, 0.75, 0.3333333333333333}};
 
-static void geom(Solver *s, const double *X, const double *Y) {
+static void launch_geom(Solver *s, cudaStream_t st, const double *X, const double *Y) {
   const Dev1 &d = s->d;
-  launch(s, "geom", [&] {
-    // the closed form is the plane area; RZ volumes carry the radius weight
-    if (s->cfg.order_exact || d.nrz) k1_geom<<<nb(d.nquad, 128), 128, 0, s->st>>>(d, X, Y);
-    else k1_geom_fast<<<nb(d.nquad, 128), 128, 0, s->st>>>(d, X, Y);
-  });
+  const int g = nb(d.nquad, 128);
+  if (s->cfg.order_exact) k1_geom<<<g, 128, 0, st>>>(d, X, Y);
+  else if (d.nrz == 0) k1f_geom<0><<<g, 128, 0, st>>>(d, X, Y);
+  else if (d.nrz == 1) k1f_geom<1><<<g, 128, 0, st>>>(d, X, Y);
+  else k1f_geom<2><<<g, 128, 0, st>>>(d, X, Y);
+}
+static void geom(Solver *s, const double *X, const double *Y) {
+  launch(s, "geom", [&] { launch_geom(s, s->st, X, Y); });
 }
 
-// RZ runs its own instantiations (in the reference's order: the RZ branch
-// has no optimised variant), so the plane kernels keep their registers
 template <int GEO, bool FAST>
-static void launch_cell_g(const Dev1 &d, dim3 g, dim3 b, cudaStream_t st, int stage) {
+static void launch_cell(const Dev1 &d, dim3 g, dim3 b, cudaStream_t st, int stage) {
   if (d.mdegr == 3) k1_cell<3, FAST, GEO><<<g, b, 0, st>>>(d, stage);
   else if (d.mdegr == 2) k1_cell<2, FAST, GEO><<<g, b, 0, st>>>(d, stage);
   else k1_cell<1, FAST, GEO><<<g, b, 0, st>>>(d, stage);
 }
-template <bool FAST>
-static void launch_cell(const Dev1 &d, dim3 g, dim3 b, cudaStream_t st, int stage) {
-  if (d.nrz == 1) launch_cell_g<1, false>(d, g, b, st, stage);
-  else if (d.nrz == 2) launch_cell_g<2, false>(d, g, b, st, stage);
-  else launch_cell_g<0, FAST>(d, g, b, st, stage);
-}
 template <int GEO, bool FAST>
-static void launch_rhs_g(const Dev1 &d, dim3 g, dim3 b, cudaStream_t st, int fuse, double alfa) {
+static void launch_rhs(const Dev1 &d, dim3 g, dim3 b, cudaStream_t st, int fuse, double alfa) {
   if (d.mdegr == 3) k1_rhs<3, FAST, GEO><<<g, b, 0, st>>>(d, fuse, alfa);
   else if (d.mdegr == 2) k1_rhs<2, FAST, GEO><<<g, b, 0, st>>>(d, fuse, alfa);
   else k1_rhs<1, FAST, GEO><<<g, b, 0, st>>>(d, fuse, alfa);
-}
-template <bool FAST>
-static void launch_rhs(const Dev1 &d, dim3 g, dim3 b, cudaStream_t st, int fuse, double alfa) {
-  if (d.nrz == 1) launch_rhs_g<1, false>(d, g, b, st, fuse, alfa);
-  else if (d.nrz == 2) launch_rhs_g<2, false>(d, g, b, st, fuse, alfa);
-  else launch_rhs_g<0, FAST>(d, g, b, st, fuse, alfa);
 }
 
 // the stage sequence of getrhsdg_lag_mcnew's linear branch
@@ -1785,19 +1790,129 @@ static void enqueue_rhs(Solver *s, int fuse, double alfa, int stage) {
   const Dev1 &d = s->d;
   launch(s, "bounds", [&] { k1_bounds<<<nb(d.npoin, 256), 256, 0, s->st>>>(d); });
   const dim3 gq(nb(d.nquad, 128)), bq(128), gp(nb(d.npoin, 256)), bp(256);
-  const bool ex = s->cfg.order_exact != 0;
   launch(s, "cell", [&] {
-    ex ? launch_cell<false>(d, gq, bq, s->st, stage) : launch_cell<true>(d, gq, bq, s->st, stage);
+    if (d.nrz == 1) launch_cell<1, false>(d, gq, bq, s->st, stage);
+    else if (d.nrz == 2) launch_cell<2, false>(d, gq, bq, s->st, stage);
+    else launch_cell<0, false>(d, gq, bq, s->st, stage);
   });
   launch(s, "node", [&] {
     if (d.nrz == 1) k1_node<false, 1><<<gp, bp, 0, s->st>>>(d);
     else if (d.nrz == 2) k1_node<false, 2><<<gp, bp, 0, s->st>>>(d);
-    else if (ex) k1_node<false, 0><<<gp, bp, 0, s->st>>>(d);
-    else k1_node<true, 0><<<gp, bp, 0, s->st>>>(d);
+    else k1_node<false, 0><<<gp, bp, 0, s->st>>>(d);
   });
   launch(s, "rhs", [&] {
-    ex ? launch_rhs<false>(d, gq, bq, s->st, fuse, alfa) : launch_rhs<true>(d, gq, bq, s->st, fuse, alfa);
+    if (d.nrz == 1) launch_rhs<1, false>(d, gq, bq, s->st, fuse, alfa);
+    else if (d.nrz == 2) launch_rhs<2, false>(d, gq, bq, s->st, fuse, alfa);
+    else launch_rhs<0, false>(d, gq, bq, s->st, fuse, alfa);
   });
+}
+
+// the same passes of the optimised stage
+template <int GEO>
+static void fast_cell(Solver *s, const Dev1 &d, int stage, int itime) {
+  launch(s, "cell", [&] {
+    k1f_cell<GEO><<<nb(4 * d.nquad, kCellThreads), kCellThreads, 0, s->st>>>(d, stage, itime);
+  });
+}
+template <int GEO>
+static void fast_node(Solver *s, const Dev1 &d, bool move, double alfa) {
+  launch(s, "node", [&] {
+    if (move) k1f_node<GEO, true><<<nb(d.npoin, 64), 64, 0, s->st>>>(d, alfa);
+    else k1f_node<GEO, false><<<nb(d.npoin, 64), 64, 0, s->st>>>(d, alfa);
+  });
+}
+template <int GEO>
+static void fast_rhs(Solver *s, const Dev1 &d, int fuse, double alfa, int last) {
+  launch(s, "rhs", [&] { k1f_rhs<GEO><<<nb(d.nquad, kRhsThreads), kRhsThreads, 0, s->st>>>(d, fuse, alfa, last); });
+}
+// Plane meshes of this many cells and more keep the order of operations of the
+// kernels above (their FAST form) instead of the closed-form moments.  The
+// limiter's absolute thresholds (1e-8 on slopes and on the strain rate) sit in the
+// foot of a wave, where some cells always are within rounding of them: on the
+// 1024 x 512 Sod mesh any change of rounding, an input's last bit included, comes
+// back as 1e-9 of the state within 10 steps (512 x 256: 4e-11), so runs of that
+// size stay comparable to the bit.  Below, the shorter chain of the fused kernels
+// decides (200 x 10: 98 -> 40 us a step with its launches; 1024 x 512: 853 us
+// before, 786 in this form, 670 with them).
+constexpr int kWideCells = 65536;
+static bool wide(const Solver *s) { return s->d.nrz == 0 && s->d.nquad >= kWideCells; }
+
+static void wide_cell(Solver *s, const Dev1 &d, int stage) {
+  launch(s, "bounds", [&] { k1_bounds<<<nb(d.npoin, 256), 256, 0, s->st>>>(d); });
+  launch(s, "cell", [&] { launch_cell<0, true>(d, dim3(nb(d.nquad, 128)), dim3(128), s->st, stage); });
+}
+static void wide_node(Solver *s, const Dev1 &d, bool move, double alfa) {
+  launch(s, "node", [&] { k1_node<true, 0><<<nb(d.npoin, 256), 256, 0, s->st>>>(d, move, alfa); });
+}
+static void wide_rhs(Solver *s, const Dev1 &d, int fuse, double alfa) {
+  launch(s, "rhs", [&] { launch_rhs<0, true>(d, dim3(nb(d.nquad, 128)), dim3(128), s->st, fuse, alfa); });
+}
+// the inner seam: RHS written, limiter coefficients in lim, no update
+template <int GEO>
+static void enqueue_rhs_fast(Solver *s) {
+  if (GEO == 0 && wide(s)) {
+    wide_cell(s, s->d, 1);
+    wide_node(s, s->d, false, 0.0);
+    wide_rhs(s, s->d, 0, 0.0);
+    return;
+  }
+  launch(s, "cell", [&] { k1f_pbar<<<nb(s->d.ncell, 128), 128, 0, s->st>>>(s->d, s->d.Us); });
+  fast_cell<GEO>(s, s->d, 1, 1);
+  fast_node<GEO>(s, s->d, false, 0.0);
+  fast_rhs<GEO>(s, s->d, 0, 0.0, 0);
+}
+template <int GEO>
+static void enqueue_step_fast(Solver *s, int itime) {
+  const Dev1 &d0 = s->d;
+  const int ns = s->cfg.nstag;
+  const bool par = s->forking && !s->timing;
+  cudaStream_t s1 = par ? s->side : s->st;
+  auto after = [&](cudaStream_t waits, cudaStream_t on) {
+    if (waits == on) return;
+    cudaEventRecord(s->fork, on);
+    cudaStreamWaitEvent(waits, s->fork, 0);
+  };
+  for (int istag = 1; istag <= ns; istag++) {
+    const double alfa = kRK[ns - 2][istag - 1];
+    const bool last = istag == ns;
+    Dev1 d = d0;
+    if (istag == 1) { d.Us = d0.Un; d.xs = d0.xn; d.ys = d0.yn; }
+    if (istag == 3) { d.xs = d0.xt; d.ys = d0.yt; }
+    d.Uo = last ? d0.Un : d0.Us;
+    d.xo = last ? d0.xn : istag == 1 ? d0.xs : d0.xt;
+    d.yo = last ? d0.yn : istag == 1 ? d0.ys : d0.yt;
+    const bool w = GEO == 0 && wide(s);
+    if (w) {
+      wide_cell(s, d, istag);
+      wide_node(s, d, istag > 1, alfa);
+    } else {
+      fast_cell<GEO>(s, d, istag, itime);
+      fast_node<GEO>(s, d, istag > 1, alfa);
+    }
+    if (istag == 1) {
+      launch(s, "dt", [&] { k1f_dt<GEO><<<nb(d.nquad, 256), 256, 0, s->st>>>(d, s->cfg.ndt, itime); });
+      after(s1, s->st);
+      launch(s, "nodes", [&] { k1f_move<<<nb(d.npoin, 64), 64, 0, s1>>>(d, alfa); });
+    }
+    if (last) {
+      after(s1, s->st);
+      launch(s, "geom", [&] { launch_geom(s, s1, d.xo, d.yo); });
+    }
+    if (w) wide_rhs(s, d, 1, alfa);
+    else fast_rhs<GEO>(s, d, 1, alfa, last);
+    if (istag == 1 || last) after(s->st, s1);
+    if (w && last) launch(s, "copy", [&] { k1_step_end<<<1, 1, 0, s->st>>>(d); });
+  }
+  s->stale = true;
+}
+// brings the stage buffers to the state (entry points that work on them)
+static void sync_stage(Solver *s) {
+  if (!s->stale) return;
+  const Dev1 &d = s->d;
+  cudaMemcpyAsync(d.Us, d.Un, NU1 * (size_t)d.ncell * sizeof(double), cudaMemcpyDeviceToDevice, s->st);
+  cudaMemcpyAsync(d.xs, d.xn, d.npoin * sizeof(double), cudaMemcpyDeviceToDevice, s->st);
+  cudaMemcpyAsync(d.ys, d.yn, d.npoin * sizeof(double), cudaMemcpyDeviceToDevice, s->st);
+  s->stale = false;
 }
 
 // getsolvdg_lag (Getrhslag.f90:1553-2035) and the driver copy-back.  On
@@ -1811,6 +1926,12 @@ static void enqueue_rhs(Solver *s, int fuse, double alfa, int stage) {
 static void enqueue_step(Solver *s, int itime) {
   const Dev1 &d = s->d;
   const int ns = s->cfg.nstag;
+  if (!s->cfg.order_exact) {
+    if (d.nrz == 0) enqueue_step_fast<0>(s, itime);
+    else if (d.nrz == 1) enqueue_step_fast<1>(s, itime);
+    else enqueue_step_fast<2>(s, itime);
+    return;
+  }
   launch(s, "copy", [&] { k1_step_begin<<<1, 1, 0, s->st>>>(d, itime); });
   for (int istag = 1; istag <= ns; istag++) {
     const double alfa = kRK[ns - 2][istag - 1];
@@ -1847,7 +1968,6 @@ static int put_scalars(Solver *s, int itime, double dtfix, double tacru, std::st
   Scalars sc{};
   sc.dtfix = dtfix; sc.tacru = tacru; sc.itime = itime;
   CK1(cudaMemcpyAsync(s->d.sc_dev, &sc, sizeof(Scalars), cudaMemcpyHostToDevice, s->st));
-  CK1(cudaStreamSynchronize(s->st));
   return LAG2D_OK;
 }
 
@@ -1952,13 +2072,21 @@ int create(const lag2d_mesh *m, const lag2d_config *c, cudaStream_t st, Solver *
        dalloc(s, &d.xs, np) && dalloc(s, &d.ys, np) && dalloc(s, &d.us, np) && dalloc(s, &d.vs, np) &&
        dalloc(s, &d.bmax, 5 * (size_t)np) && dalloc(s, &d.bmin, 5 * (size_t)np) && dalloc(s, &d.lim, 7 * ncl) &&
        dalloc(s, &d.cf, (c->nrz == 1 ? 80 : 40) * ncl) && dalloc(s, &d.rhs, NU1 * ncl) && dalloc(s, &d.rbar, ncl) &&
-       dalloc(s, &d.dtpart, 2 * (size_t)nb(nq, 256)) && dalloc(s, &d.sc_dev, 1) &&
+       dalloc(s, &d.dtpart, 2 * (size_t)nb(nq, 256)) && dalloc(s, &d.pbar, ncl) && dalloc(s, &d.count, 2) &&
+       dalloc(s, &d.xt, np) && dalloc(s, &d.yt, np) && dalloc(s, &d.sc_dev, 1) &&
        dalloc(s, &s->stage_u, NU1 * ncl) && dalloc(s, &s->stage_x, 2 * (size_t)np);
   if (!ok) {
     destroy(s);
     err = "cudaMalloc failed";
     return LAG2D_ECUDA;
   }
+  if (cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) != cudaSuccess) {
+    destroy(s);
+    err = "cudaStreamCreate failed";
+    return LAG2D_ECUDA;
+  }
+  d.Uo = d.Us; d.xo = d.xs; d.yo = d.ys;
   d.ipq = ipq_d; d.esuv_ptr = eptr_d; d.esuv = esv_d; d.ncor_ptr = cptr_d; d.ncor = cor_d; d.bc = bc_d;
   d.wall = wall_d; d.x0 = x0; d.y0 = y0;
   d.bf_ptr = bptr_d; d.bf_list = blist_d; d.bfn = bfn_d; d.bfcode = bfcode_d;
@@ -2036,6 +2164,8 @@ int init_fields(Solver *s, double *geoel, double *amatr, double *unkno, std::str
   CK1(cudaMemsetAsync(d.vs, 0, np * sizeof(double), s->st));
   Scalars s0{};
   CK1(cudaMemcpyAsync(d.sc_dev, &s0, sizeof(Scalars), cudaMemcpyHostToDevice, s->st));
+  s->stale = false;
+  launch(s, "init", [&] { k1f_pbar<<<nb(ncell, 128), 128, 0, s->st>>>(d, d.Un); });
   geom(s, d.xn, d.yn);
   int r = read_status(s, err);
   if (r) return r;
@@ -2084,55 +2214,65 @@ int set_state(Solver *s, const double *unkno, const double *coord, const double 
   }
   Scalars s0{};
   CK1(cudaMemcpyAsync(d.sc_dev, &s0, sizeof(Scalars), cudaMemcpyHostToDevice, s->st));
+  s->stale = false;
+  launch(s, "copy", [&] { k1f_pbar<<<nb(ncell, 128), 128, 0, s->st>>>(d, d.Un); });
   geom(s, d.xs, d.ys);
   return read_status(s, err);
 }
 
-int step(Solver *s, int itime, double *dtfix, double *tacru, std::string &err) {
-  int r = put_scalars(s, itime, *dtfix, *tacru, err);
-  if (r) return r;
-  enqueue_step(s, itime);
-  Scalars sc;
-  CK1(cudaMemcpyAsync(&sc, s->d.sc_dev, sizeof(Scalars), cudaMemcpyDeviceToHost, s->st));
-  CK1(cudaStreamSynchronize(s->st));
-  if (s->timing) flush_timing(s);
-  *dtfix = sc.dtfix;
-  *tacru = sc.tacru;
-  return read_status(s, err);
+// one step with itime incremented on the device, captured once per handle
+static int step_graph(Solver *s, std::string &err) {
+  if (s->graph) return LAG2D_OK;
+  cudaGraph_t g;
+  CK1(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
+  const long long before = s->launches;
+  s->forking = true;
+  enqueue_step(s, -1);
+  s->forking = false;
+  s->graph_launches = s->launches - before;
+  s->launches = before;  // counted per replay
+  CK1(cudaStreamEndCapture(s->st, &g));
+  const cudaError_t e = cudaGraphInstantiate(&s->graph, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) s->graph = nullptr;
+  CK1(e);
+  return LAG2D_OK;
 }
 
-int run(Solver *s, int itime0, int nsteps, double *dtfix, double *tacru, int *done, std::string &err) {
+// nsteps replays of the captured step (with timing on, launch by launch)
+static int advance(Solver *s, int itime0, int nsteps, double *dtfix, double *tacru, Scalars &sc, std::string &err) {
   int r = put_scalars(s, itime0 - 1, *dtfix, *tacru, err);
   if (r) return r;
-  int steps = 0;
   if (s->timing) {
-    for (int i = 0; i < nsteps; i++) { enqueue_step(s, itime0 + i); steps++; }
+    for (int i = 0; i < nsteps; i++) enqueue_step(s, itime0 + i);
     flush_timing(s);
   } else {
-    if (!s->graph) {
-      cudaGraph_t g;
-      CK1(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
-      const long long before = s->launches;
-      enqueue_step(s, -1);
-      CK1(cudaStreamEndCapture(s->st, &g));
-      CK1(cudaGraphInstantiate(&s->graph, g, 0));
-      cudaGraphDestroy(g);
-      s->graph_launches = s->launches - before;
-      s->launches = before;
-    }
+    if ((r = step_graph(s, err))) return r;
     for (int i = 0; i < nsteps; i++) {
       CK1(cudaGraphLaunch(s->graph, s->st));
       s->launches += s->graph_launches;
-      steps++;
     }
   }
-  Scalars sc;
+  if (nsteps && !s->cfg.order_exact) s->stale = true;
   CK1(cudaMemcpyAsync(&sc, s->d.sc_dev, sizeof(Scalars), cudaMemcpyDeviceToHost, s->st));
   CK1(cudaStreamSynchronize(s->st));
+  CK1(cudaGetLastError());
   *dtfix = sc.dtfix;
   *tacru = sc.tacru;
-  if (done) *done = sc.done ? std::min(steps, std::max(0, sc.itime - itime0 + 1)) : steps;
-  return read_status(s, err);
+  if (sc.status & ST_NONPHYS) { err = "non-positive cell volume"; return LAG2D_ENONPHYS; }
+  return LAG2D_OK;
+}
+
+int step(Solver *s, int itime, double *dtfix, double *tacru, std::string &err) {
+  Scalars sc;
+  return advance(s, itime, 1, dtfix, tacru, sc, err);
+}
+
+int run(Solver *s, int itime0, int nsteps, double *dtfix, double *tacru, int *done, std::string &err) {
+  Scalars sc{};
+  const int r = advance(s, itime0, nsteps, dtfix, tacru, sc, err);
+  if (done) *done = sc.done ? std::min(nsteps, std::max(0, sc.itime - itime0 + 1)) : nsteps;
+  return r;
 }
 
 int get_state(Solver *s, double *unkno, double *coord, double *ustar, double *geoel, std::string &err) {
@@ -2151,9 +2291,13 @@ int get_state(Solver *s, double *unkno, double *coord, double *ustar, double *ge
 // updates ustar, returns rhsel(3, 4, ncell)
 int rhs(Solver *s, double *rhsel, std::string &err) {
   const Dev1 &d = s->d;
+  sync_stage(s);
   int r = put_scalars(s, 1, 0.0, 0.0, err);
   if (r) return r;
-  enqueue_rhs(s, 0, 0.0, 1);
+  if (s->cfg.order_exact) enqueue_rhs(s, 0, 0.0, 1);
+  else if (d.nrz == 0) enqueue_rhs_fast<0>(s);
+  else if (d.nrz == 1) enqueue_rhs_fast<1>(s);
+  else enqueue_rhs_fast<2>(s);
   // the slope application of :7283-7298 alone: the update with alfa = 0 and dt = 0
   launch(s, "update", [&] { k1_update<<<nb(d.ncell, 128), 128, 0, s->st>>>(d, 0.0); });
   if ((r = read_status(s, err))) return r;
@@ -2164,6 +2308,7 @@ int rhs(Solver *s, double *rhsel, std::string &err) {
 }
 
 int cellvol(Solver *s, double *geoel, std::string &err) {
+  sync_stage(s);
   geom(s, s->d.xs, s->d.ys);
   int r = read_status(s, err);
   if (r) return r;
@@ -2206,6 +2351,8 @@ void destroy(Solver *s) {
   if (s->st) cudaStreamSynchronize(s->st);
   for (auto &p : s->pending) { cudaEventDestroy(p.second.first); cudaEventDestroy(p.second.second); }
   if (s->graph) cudaGraphExecDestroy(s->graph);
+  if (s->fork) cudaEventDestroy(s->fork);
+  if (s->side) cudaStreamDestroy(s->side);
   for (void *p : s->allocs) cudaFree(p);
   delete s;
 }
