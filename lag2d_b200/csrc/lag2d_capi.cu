@@ -351,13 +351,13 @@ struct StageRec {
   // the handle's device view with the corner/node outputs of a slot
   Dev outputs(const Dev &d0, size_t slot) const {
     Dev d = d0;
-    d.npart = npart + slot * 45 * nq;
+    d.npart = npart + slot * 9 * d0.nrow * nq;
     d.corr = corr + slot * 4 * nq;
     d.us_new = usn + slot * np;
     d.vs_new = vsn + slot * np;
     if (nt > 0) {
       d.tcf = tcf + slot * 120 * nt;
-      d.tpart = tpart + slot * 30 * nt;
+      d.tpart = tpart + slot * 6 * d0.nrow * nt;
     }
     return d;
   }
@@ -611,6 +611,7 @@ int lag2d_create(const lag2d_mesh *m, const lag2d_config *c, lag2d_handle **out)
   Dev &d = h->d;
   d.ntria = m->ntria; d.nquad = m->nquad; d.npoin = m->npoin; d.nbfac = m->nbfac; d.ncell = ncell;
   d.ndegr = c->ndegr; d.mdegr = c->mdegr; d.ncase = c->ncase; d.nlimi = c->nlimi;
+  d.nrow = c->precision == 1 || c->order_exact ? 5 : 3;
   d.gamlg = c->gamlg; d.cfl = c->cfl; d.cdrho = c->cdrho; d.cimpd = c->cimpd; d.tend = c->tend;
   d.sedov_energy = c->sedov_energy; d.nsedov = c->nsedov;
   for (int i = 0; i < 4; i++) d.sedov_cell[i] = c->sedov_cell[i];
@@ -719,10 +720,10 @@ int lag2d_create(const lag2d_mesh *m, const lag2d_config *c, lag2d_handle **out)
   A(&h->stage_u, NU * (size_t)ncell); A(&h->stage_x, 2 * (size_t)np); A(&h->stage_v, 2 * (size_t)np);
   int *ptr2_d, *slot_d;
   A(&ptr2_d, cnt2.size()); A(&slot_d, slots.size());
-  A(&d.npart, 45 * (size_t)nq); A(&d.corr, 4 * (size_t)nq); A(&d.src, 12 * (size_t)nq); A(&d.us_new, np); A(&d.vs_new, np);
+  A(&d.npart, 9 * d.nrow * (size_t)nq); A(&d.corr, 4 * (size_t)nq); A(&d.src, 12 * (size_t)nq); A(&d.us_new, np); A(&d.vs_new, np);
   A(&d.wmom, 9 * (size_t)nq);
   int *ipt_d;
-  A(&ipt_d, ipt.size()); A(&d.tmsub, 4 * (size_t)nt); A(&d.tcf, 5 * 24 * (size_t)nt); A(&d.tpart, 5 * 6 * (size_t)nt);
+  A(&ipt_d, ipt.size()); A(&d.tmsub, 4 * (size_t)nt); A(&d.tcf, 5 * 24 * (size_t)nt); A(&d.tpart, 6 * d.nrow * (size_t)nt);
   if (rc != LAG2D_OK) { lag2d_destroy(h); return rc; }
   d.ipt = ipt_d;
   d.Uo = d.Us; d.xo = d.xs; d.yo = d.ys; d.dtcount = d.wcount + 3;
@@ -1309,15 +1310,15 @@ struct AdjWork {
     alloc(&a.lU, nu); alloc(&a.lUn, nu); alloc(&a.lR, nu);
     alloc(&a.lx, np); alloc(&a.ly, np); alloc(&a.lxn, np); alloc(&a.lyn, np); alloc(&a.lus, np); alloc(&a.lvs, np);
     alloc(&a.luw, np); alloc(&a.lvw, np); alloc(&a.tx, np); alloc(&a.ty, np);
-    alloc(&a.lS, 5 * np); alloc(&a.lP, 45 * (size_t)d.nquad); alloc(&a.pbuf, 54 * (size_t)d.nquad);
+    alloc(&a.lS, 3 * np); alloc(&a.lP, 27 * (size_t)d.nquad); alloc(&a.pbuf, 54 * (size_t)d.nquad);
     alloc(&a.lcorr, 4 * (size_t)d.nquad);
     alloc(&a.tbuf, 36 * (size_t)d.ntria); alloc(&a.ltcf, 120 * (size_t)d.ntria);
     const size_t ns = (size_t)K * nstag;
     alloc(&rec.U, ns * nu); alloc(&rec.x, ns * np); alloc(&rec.y, ns * np);
     alloc(&rec.us, ns * np); alloc(&rec.vs, ns * np); alloc(&rec.dt, K);
-    alloc(&rec.npart, ns * 45 * (size_t)d.nquad); alloc(&rec.corr, ns * 4 * (size_t)d.nquad);
+    alloc(&rec.npart, ns * 9 * d.nrow * (size_t)d.nquad); alloc(&rec.corr, ns * 4 * (size_t)d.nquad);
     alloc(&rec.usn, ns * np); alloc(&rec.vsn, ns * np);
-    alloc(&rec.tcf, ns * 120 * (size_t)d.ntria); alloc(&rec.tpart, ns * 30 * (size_t)d.ntria);
+    alloc(&rec.tcf, ns * 120 * (size_t)d.ntria); alloc(&rec.tpart, ns * 6 * d.nrow * (size_t)d.ntria);
     rec.nstag = nstag; rec.nu = nu; rec.np = np; rec.nq = d.nquad; rec.nt = d.ntria;
     cap = std::max(1, std::min(d.nquad, 16384));
     alloc(&wbuf, 216 * (size_t)cap); alloc(&wslot, (size_t)d.nquad); alloc(&overflow, 1);

@@ -69,7 +69,8 @@ struct Dev {
   // optimised path
   const int *node_ptr2;    // [npoin+1]
   const int *node_slot;    // iq*9 + k: quad iq touches the node as its node k, cells ascending
-  double *npart;           // [5][9][nquad] per-cell node partial sums (m, m*u, m*v, s_x, s_y)
+  int nrow;                // rows of npart and tpart: 3, or 5 in the FP32-mixed and reference-order paths
+  double *npart;           // [nrow][9][nquad] per-cell node partial sums: (m, m u - s_x, m v - s_y), or (m, m u, m v, s_x, s_y)
   double *corr;            // [4][nquad] sub-cell density corrections
   double *src;             // [6][nquad] Taylor-Green source moments of the stage (corner pass -> RHS pass)
   double *us_new, *vs_new; // ustar of the current stage (us, vs hold the previous one)
@@ -78,7 +79,7 @@ struct Dev {
   const int *ipt;          // [6][ntria] node k of triangle it
   double *tmsub;           // [4][ntria] initial sub-cell masses
   double *tcf;             // [5][24][ntria] corner coefficients (m, m u, m v, sigma.n A) per corner face
-  double *tpart;           // [5][6][ntria] their per-node sums
+  double *tpart;           // [nrow][6][ntria] their per-node sums
 };
 
 // Quadrature tables (filled from the host with the reference's literals).
@@ -98,8 +99,8 @@ struct Adj {
   double *lus, *lvs;       // adjoint of the stage's previous ustar
   double *luw, *lvw;       // adjoint of the stage's new ustar
   double *lR;              // [24][ncell] adjoint of the stage RHS
-  double *lS;              // [5][npoin] adjoint of the node sums (m, m u, m v, sigma.n A)
-  double *lP;              // [5][9][nquad] RHS pass's adjoint of each quad's node partial sums
+  double *lS;              // [3][npoin] adjoint of the node sums (m, m u, m v); that of sigma.n A is minus the last two
+  double *lP;              // [3][9][nquad] RHS pass's adjoint of each quad's node partial sums, alike
   double *lcorr;           // [4][nquad] adjoint of the sub-cell density corrections (corner faces -> corrections)
   double *pbuf;            // [6][9][nquad] per (quad, node) adjoint contributions
   double *tx, *ty;         // scratch of the centre-node transpose

@@ -584,17 +584,22 @@ __host__ __device__ void f_corner_corr(const Dev &d, int iq) {
 // move: the node motion of the stage in the same pass (the stages after the
 // first, whose dt is known).  u* is updated in place; us_new receives it too
 // where it is a buffer of its own.
-__device__ __forceinline__ void node_add(const Dev &d, int id, double s[5]) {
+// NR = 3 rows of partial sums (m, m u - sigma.n A), or 5 in the FP32-mixed step,
+// whose sums keep their bits.  Three carry the same solve and corner forces with
+// 40% less traffic: at 1024 x 1024 the node pass with the motion went from 129 to
+// 101 us a launch, the RHS pass from 366 to 341, the face pass from 242 to 224.
+template <int NR>
+__device__ __forceinline__ void node_add(const Dev &d, int id, double s[NR]) {
   if (id < 0) {  // triangle: -1 - (it*6 + k), partials of its node k
     const int t = -1 - id, it = t / 6, k = t - 6 * it;
     const size_t nt = d.ntria;
 #pragma unroll
-    for (int v = 0; v < 5; v++) s[v] += d.tpart[(v * 6 + k) * nt + it];
+    for (int v = 0; v < NR; v++) s[v] += d.tpart[(v * 6 + k) * nt + it];
     return;
   }
   const int iq = id / 9, k = id - 9 * iq;
 #pragma unroll
-  for (int v = 0; v < 5; v++) s[v] += d.npart[(v * 9 + k) * (size_t)d.nquad + iq];
+  for (int v = 0; v < NR; v++) s[v] += d.npart[(v * 9 + k) * (size_t)d.nquad + iq];
 }
 __device__ __forceinline__ void move_node(const Dev &d, int p, double alfa, double dt, double un, double vn, double xn,
                                           double yn, double xs, double ys) {
@@ -602,7 +607,7 @@ __device__ __forceinline__ void move_node(const Dev &d, int p, double alfa, doub
   d.xo[p] = alfa * xn + oma * (xs + dt * un);
   d.yo[p] = alfa * yn + oma * (ys + dt * vn);
 }
-template <bool MOVE>
+template <bool MOVE, int NR>
 __device__ void f_node(const Dev &d, int p, double alfa) {
   if (p >= d.npoin) return;
   const int done = d.sc_dev->done;
@@ -621,14 +626,16 @@ __device__ void f_node(const Dev &d, int p, double alfa) {
 #pragma unroll
   for (int j = 0; j < 4; j++) id[j] = b + j < en ? d.node_slot[b + j] : 0;
   if (done) return;
-  double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  double s[NR];
+#pragma unroll
+  for (int v = 0; v < NR; v++) s[v] = 0.0;
 #pragma unroll
   for (int j = 0; j < 4; j++)
-    if (b + j < en) node_add(d, id[j], s);
-  for (int i = b + 4; i < en; i++) node_add(d, d.node_slot[i], s);
+    if (b + j < en) node_add<NR>(d, id[j], s);
+  for (int i = b + 4; i < en; i++) node_add<NR>(d, d.node_slot[i], s);
   if (!(mask & 4)) {
-    us = (s[1] - s[3]) / s[0];
-    vs = (s[2] - s[4]) / s[0];
+    us = (NR == 5 ? s[1] - s[NR - 2] : s[1]) / s[0];
+    vs = (NR == 5 ? s[2] - s[NR - 1] : s[2]) / s[0];
   }
   if (mask & 1) us = 0.0;
   if (mask & 2) vs = 0.0;
@@ -698,11 +705,10 @@ __host__ __device__ __forceinline__ void mass_flux_weights(const Loaded &L, int 
 // k the corner force of corner face f is F_f = sigma.n A w_f + m_f (u* - u_k),
 // with u* the node's new velocity and m_f, sigma.n A w_f, u_k what the corner
 // pass used (Getrhslaggauss.f90:10409-10867).  The momentum sum is therefore
-// affine in u*: sum_f F_f = (P3, P4) + u* P0 - (P1, P2), where P0..P4 are the
-// node partial sums the corner pass wrote (sum m, sum m u_k, sum m v_k, sum
-// sigma.n A w); the energy term is u* . sum_f F_f; the mass term is
+// affine in u*: sum_f F_f = u* P0 - (P1, P2), where P0..P2 are the node partial
+// sums the corner pass wrote (sum m, sum m u_k - sigma.n A w); the energy term is u* . sum_f F_f; the mass term is
 // u* . sum_f 2 w_mass,f an_f over the 16 outer corner faces.  So the corner
-// data are not recomputed here: 40 partials and the 8 boundary nodes'
+// data are not recomputed here: 24 partials and the 8 boundary nodes'
 // velocities replace the 32 corner faces' vertex states, impedances and
 // forces (same sums up to rounding and summation order).
 //
@@ -734,7 +740,7 @@ __device__ void f_rhs3(const Dev &d, int iq, int fuse_update, double alfa, doubl
     // the 1024x1024 Taylor-Green mesh)
     const size_t nq = d.nquad;
 #pragma unroll
-    for (int v = 0; v < 5; v++)
+    for (int v = 0; v < 3; v++)
 #pragma unroll
       for (int k = 0; k < 8; k++) asm volatile("prefetch.global.L2 [%0];" ::"l"(d.npart + (v * 9 + k) * nq + iq));
     if (d.ncase == 1) {
@@ -757,11 +763,9 @@ __device__ void f_rhs3(const Dev &d, int iq, int fuse_update, double alfa, doubl
     mass_flux_weights(L, k, tx, ty);
     const double tw = un * tx + vn * ty;
     const size_t nq = d.nquad;
-    const double P0 = d.npart[(0 * 9 + k) * nq + iq], P1 = d.npart[(1 * 9 + k) * nq + iq];
-    const double P2 = d.npart[(2 * 9 + k) * nq + iq], P3 = d.npart[(3 * 9 + k) * nq + iq];
-    const double P4 = d.npart[(4 * 9 + k) * nq + iq];
-    const double f0 = P3 + (un * P0 - P1);
-    const double f1 = P4 + (vn * P0 - P2);
+    const double P0 = d.npart[(0 * 9 + k) * nq + iq];
+    const double f0 = un * P0 - d.npart[(1 * 9 + k) * nq + iq];
+    const double f1 = vn * P0 - d.npart[(2 * 9 + k) * nq + iq];
     const double fe = un * f0 + vn * f1;
 #pragma unroll
     for (int kk = 0; kk < 6; kk++) {
@@ -1242,8 +1246,7 @@ __host__ __device__ void a_corner_faces(const Dev &d, const Adj &a, int iq) {
     const double lP0 = a.lS[0 * (size_t)d.npoin + pn] + a.lP[(0 * 9 + k) * nq + iq];
     const double lP1 = a.lS[1 * (size_t)d.npoin + pn] + a.lP[(1 * 9 + k) * nq + iq];
     const double lP2 = a.lS[2 * (size_t)d.npoin + pn] + a.lP[(2 * 9 + k) * nq + iq];
-    const double lP3 = a.lS[3 * (size_t)d.npoin + pn] + a.lP[(3 * 9 + k) * nq + iq];
-    const double lP4 = a.lS[4 * (size_t)d.npoin + pn] + a.lP[(4 * 9 + k) * nq + iq];
+    const double lP3 = -lP1, lP4 = -lP2;
     double lst1 = 0, lst2 = 0, lrhovt = 0, lke = 0, ldux = 0, lduy = 0;
     for (int i = nc_start(k); i < nc_start(k + 1); i++) {
       const int isg = nc_entry(i) >> 2, ivsg = nc_entry(i) & 3;
@@ -1658,14 +1661,14 @@ __host__ __device__ void a_rhs(const Dev &d, const Adj &a, int iq) {
   for (int q = 0; q < 4; q++) for (int k = 0; k < 6; k++) lu[q][k] = 0.0;
   double lX[3][3], lY[3][3];
   for (int i = 0; i < 3; i++) for (int j = 0; j < 3; j++) { lX[i][j] = 0.0; lY[i][j] = 0.0; }
-  // ---- face integral (f_rhs3): transpose of f = (P3, P4) + u* P0 - (P1, P2),
+  // ---- face integral (f_rhs3): transpose of f = u* P0 - (P1, P2),
   // fe = u* . f, tw = u* . t per boundary node; the adjoints of the node
-  // partial sums P0..P4 go to a.lP for the corner pass's transpose, those of
+  // partial sums go to a.lP for the corner pass's transpose, those of
   // u* to pbuf, those of the mass-flux weights t to the face vectors
   for (int k = 0; k < 9; k++) {
     if (k == 8) {
       for (int v = 2; v < 6; v++) a.pbuf[(v * 9 + k) * nq + iq] = 0.0;
-      for (int v = 0; v < 5; v++) a.lP[(v * 9 + k) * nq + iq] = 0.0;
+      for (int v = 0; v < 3; v++) a.lP[(v * 9 + k) * nq + iq] = 0.0;
       continue;
     }
     double b[6];
@@ -1675,9 +1678,15 @@ __host__ __device__ void a_rhs(const Dev &d, const Adj &a, int iq) {
     double tx, ty;
     mass_flux_weights(L, k, tx, ty);
     const double P0 = d.npart[(0 * 9 + k) * nq + iq], P1 = d.npart[(1 * 9 + k) * nq + iq];
-    const double P2 = d.npart[(2 * 9 + k) * nq + iq], P3 = d.npart[(3 * 9 + k) * nq + iq];
-    const double P4 = d.npart[(4 * 9 + k) * nq + iq];
-    const double f0 = P3 + (un * P0 - P1), f1 = P4 + (vn * P0 - P2);
+    const double P2 = d.npart[(2 * 9 + k) * nq + iq];
+    double f0, f1;
+    if (d.nrow == 3) {
+      f0 = un * P0 - P1;
+      f1 = vn * P0 - P2;
+    } else {
+      f0 = d.npart[(3 * 9 + k) * nq + iq] + (un * P0 - P1);
+      f1 = d.npart[(4 * 9 + k) * nq + iq] + (vn * P0 - P2);
+    }
     double ltw = 0, lf0 = 0, lf1 = 0, lfe = 0;
     for (int kk = 0; kk < 6; kk++) {
       ltw += lR[0][kk] * b[kk];
@@ -1692,8 +1701,6 @@ __host__ __device__ void a_rhs(const Dev &d, const Adj &a, int iq) {
     a.lP[(0 * 9 + k) * nq + iq] = lf0 * un + lf1 * vn;
     a.lP[(1 * 9 + k) * nq + iq] = -lf0;
     a.lP[(2 * 9 + k) * nq + iq] = -lf1;
-    a.lP[(3 * 9 + k) * nq + iq] = lf0;
-    a.lP[(4 * 9 + k) * nq + iq] = lf1;
     a.pbuf[(2 * 9 + k) * nq + iq] = 0.0;
     a.pbuf[(3 * 9 + k) * nq + iq] = 0.0;
     a.pbuf[(4 * 9 + k) * nq + iq] = lun;
@@ -1755,8 +1762,8 @@ __host__ __device__ void a_gather(const Dev &d, const Adj &a, int p, int nv) {
 }
 
 // Gather of the RHS pass's per-(cell, node) contributions (x, y, u*_prev,
-// u*_new) fused with the reverse of the node solve u* = (S1 - S3) / S0,
-// v* = (S2 - S4) / S0 (wall masks; kept nodes take u*_prev).  Only S0 is
+// u*_new) fused with the reverse of the node solve u* = S1 / S0,
+// v* = S2 / S0 (wall masks; kept nodes take u*_prev).  Only S0 is
 // gathered again: u* itself is the forward pass's d.us_new / d.vs_new.
 __host__ __device__ void a_gather_solve(const Dev &d, const Adj &a, int p) {
   if (p >= d.npoin) return;
@@ -1787,7 +1794,7 @@ __host__ __device__ void a_gather_solve(const Dev &d, const Adj &a, int p) {
     a.lus[p] = lus + lu;
     a.lvs[p] = lvs + lv;
 #pragma unroll
-    for (int v = 0; v < 5; v++) a.lS[v * np + p] = 0.0;
+    for (int v = 0; v < 3; v++) a.lS[v * np + p] = 0.0;
     return;
   }
   a.lus[p] = lus;
@@ -1795,9 +1802,7 @@ __host__ __device__ void a_gather_solve(const Dev &d, const Adj &a, int p) {
   const double iS0 = 1.0 / S0;
   a.lS[0 * np + p] = -(lu * d.us_new[p] + lv * d.vs_new[p]) * iS0;
   a.lS[1 * np + p] = lu * iS0;
-  a.lS[3 * np + p] = -lu * iS0;
   a.lS[2 * np + p] = lv * iS0;
-  a.lS[4 * np + p] = -lv * iS0;
 }
 
 // fold (stage 1, the last one reversed): U^(1) is U^n itself, so the adjoint
@@ -1890,9 +1895,9 @@ __global__ void __launch_bounds__(128, LAG2D_CCORR_MINB) k_corner2_corr(Dev d) {
   f_corner_corr(d, blockIdx.x * blockDim.x + threadIdx.x);
 }
 __global__ void __launch_bounds__(128) k_tgv_src2(Dev d) { f_tgv_src(d, blockIdx.x * blockDim.x + threadIdx.x); }
-template <bool MOVE>
+template <bool MOVE, int NR>
 __global__ void __launch_bounds__(256) k_node2(Dev d, double alfa) {
-  f_node<MOVE>(d, blockIdx.x * blockDim.x + threadIdx.x, alfa);
+  f_node<MOVE, NR>(d, blockIdx.x * blockDim.x + threadIdx.x, alfa);
 }
 __global__ void __launch_bounds__(kRhsBlock, LAG2D_RHS_MINB) k_rhs3(Dev d, int fuse, double alfa) {
   extern __shared__ double rhs_stage[];
@@ -2031,8 +2036,13 @@ void launch_fast_faces(const Dev &d, cudaStream_t st) {
 void launch_fast_src(const Dev &d, cudaStream_t st) { fast::k_tgv_src2<<<fast::nb(d.nquad, 128), 128, 0, st>>>(d); }
 void launch_fast_node(const Dev &d, cudaStream_t st, int move, double alfa) {
   const int g = fast::nb(d.npoin, 256);
-  if (move) fast::k_node2<true><<<g, 256, 0, st>>>(d, alfa);
-  else fast::k_node2<false><<<g, 256, 0, st>>>(d, alfa);
+  if (d.nrow == 3) {
+    if (move) fast::k_node2<true, 3><<<g, 256, 0, st>>>(d, alfa);
+    else fast::k_node2<false, 3><<<g, 256, 0, st>>>(d, alfa);
+  } else {
+    if (move) fast::k_node2<true, 5><<<g, 256, 0, st>>>(d, alfa);
+    else fast::k_node2<false, 5><<<g, 256, 0, st>>>(d, alfa);
+  }
 }
 void launch_fast_rhs(const Dev &d, cudaStream_t st, int fuse, double alfa) {
   constexpr int smem = fast::kRhsStage * fast::kRhsBlock * sizeof(double);

@@ -3430,7 +3430,8 @@ __host__ __device__ void a_tri_corner(const Dev &d, const Adj &a, int it) {
         const double n0 = sg * gt[slot][0], n1 = sg * gt[slot][1], ar = gt[slot][2] * w;
         const int cs = f + 2 * (ivsg + 3 * isg);
         double L[5];
-        for (int v = 0; v < 5; v++) L[v] = a.ltcf[(v * 24 + cs) * nt + it] + a.lS[v * np + pn];
+        for (int v = 0; v < 5; v++)
+          L[v] = a.ltcf[(v * 24 + cs) * nt + it] + (v < 3 ? a.lS[v * np + pn] : -a.lS[(v - 2) * np + pn]);
         const double m = rhoct * sdctr * ar;
         // (m, m u, m v, -p A n0, -p A n1)
         const double lm = L[0] + L[1] * uv + L[2] * vv;

@@ -37,7 +37,9 @@ __device__ __forceinline__ void basis_at(const CellGeo &g, double x, double y, d
 }
 
 // ---------------------------------------------------------------------------
-// Corner faces: the node partial sums P0..P4 (m, m u, m v, sigma.n A)
+// Corner faces: the node partial sums (m, m u - sigma.n A), three rows a node:
+// the node solve and the corner forces need m u and sigma.n A only as their
+// difference
 // ---------------------------------------------------------------------------
 // rows of a thread's column: x, y, u*_prev, v*_prev of the 9 nodes, 4 corrections
 constexpr int kFaceBlock = 128;
@@ -135,10 +137,8 @@ __device__ void f_faces(const Dev &d, int iq_in, double *col) {
       const double pw = (-1.0 / 3.0) * fmax(eps, gm * (s.rho + corr0) * s.ke);
       double *o = d.npart + v * nq + iq;
       o[0] = P0;
-      o[9 * nq] = P0 * s.u;
-      o[18 * nq] = P0 * s.v;
-      o[27 * nq] = pw * (ax + bx);
-      o[36 * nq] = pw * (ay + by);
+      o[9 * nq] = P0 * s.u - pw * (ax + bx);
+      o[18 * nq] = P0 * s.v - pw * (ay + by);
     }
     {
       // edge node e: A with weight 1/3 and -B, B with weight 2/3 in sub-cells
@@ -159,10 +159,8 @@ __device__ void f_faces(const Dev &d, int iq_in, double *col) {
       const double wa = (-2.0 / 3.0) * (p0 + p1), wb = (4.0 / 3.0) * (p0 - p1);
       double *o = d.npart + (4 + v) * nq + iq;
       o[0] = P0;
-      o[9 * nq] = P0 * s.u;
-      o[18 * nq] = P0 * s.v;
-      o[27 * nq] = wa * ax + wb * bx;
-      o[36 * nq] = wa * ay + wb * by;
+      o[9 * nq] = P0 * s.u - (wa * ax + wb * bx);
+      o[18 * nq] = P0 * s.v - (wa * ay + wb * by);
       M0 += impedance(rhoc, kap, nb, fabs(mdx * bx + mdy * by), mreg, mrj);
       const double pn1 = fmax(eps, (m.rho + corr1) * mpe);
       M3 += (pm - pn1) * bx;
@@ -172,10 +170,8 @@ __device__ void f_faces(const Dev &d, int iq_in, double *col) {
   }
   double *o = d.npart + 8 * nq + iq;
   o[0] = M0;
-  o[9 * nq] = M0 * m.u;
-  o[18 * nq] = M0 * m.v;
-  o[27 * nq] = 0.5 * M3;
-  o[36 * nq] = 0.5 * M4;
+  o[9 * nq] = M0 * m.u - 0.5 * M3;
+  o[18 * nq] = M0 * m.v - 0.5 * M4;
 #undef FX
 #undef FY
 #undef FU

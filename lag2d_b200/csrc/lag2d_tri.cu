@@ -207,6 +207,7 @@ __device__ __forceinline__ double sub_density(const Dev &d, const Tri &T, const 
   return (msub - rt * num / den) / vol;
 }
 
+template <int NR>
 __global__ void __launch_bounds__(64) k_corner(Dev d) {
   const int it = blockIdx.x * blockDim.x + threadIdx.x;
   if (it >= d.ntria) return;
@@ -271,7 +272,8 @@ __global__ void __launch_bounds__(64) k_corner(Dev d) {
 #pragma unroll
   for (int k = 0; k < 6; k++)
 #pragma unroll
-    for (int v = 0; v < 5; v++) d.tpart[(v * 6 + k) * nt + it] = P[k][v];
+    for (int v = 0; v < NR; v++)
+      d.tpart[(v * 6 + k) * nt + it] = NR == 3 && v > 0 ? P[k][v] - P[k][v + 2] : P[k][v];
 }
 
 // sum of the weights with which slot N (1..15) enters the mass flux of node V
@@ -294,13 +296,17 @@ __device__ __forceinline__ void mass_vec(const Tri &T, double &tx, double &ty) {
   if constexpr (N < 15) mass_vec<V, N + 1>(T, tx, ty);
 }
 // face integral at node V: the corner forces are affine in the node's velocity,
-// sum_f F_f = (P3, P4) + u* P0 - (P1, P2)
-template <int V>
-__device__ __forceinline__ void face_node(const Tri &T, double us, double vs, const double P[5], double R[4][6]) {
+// sum_f F_f = u* P0 - (P1, P2), plus (P3, P4) where sigma.n A has its own rows
+template <int V, int NR>
+__device__ __forceinline__ void face_node(const Tri &T, double us, double vs, const double P[NR], double R[4][6]) {
   double tx = 0.0, ty = 0.0, b[6];
   mass_vec<V, 1>(T, tx, ty);
   basis(T, xv(V), yv(V), b);
-  const double f0 = P[3] + (us * P[0] - P[1]), f1 = P[4] + (vs * P[0] - P[2]);
+  double f0 = us * P[0] - P[1], f1 = vs * P[0] - P[2];
+  if (NR == 5) {
+    f0 = P[NR - 2] + f0;
+    f1 = P[NR - 1] + f1;
+  }
   const double tw = us * tx + vs * ty, fe = us * f0 + vs * f1;
 #pragma unroll
   for (int k = 0; k < 6; k++) {
@@ -311,6 +317,7 @@ __device__ __forceinline__ void face_node(const Tri &T, double us, double vs, co
   }
 }
 
+template <int NR>
 __global__ void __launch_bounds__(64) k_rhs(Dev d, const double *usn, const double *vsn, int fuse, double alfa) {
   const int it = blockIdx.x * blockDim.x + threadIdx.x;
   if (it >= d.ntria) return;
@@ -319,7 +326,7 @@ __global__ void __launch_bounds__(64) k_rhs(Dev d, const double *usn, const doub
   const double g = d.gamlg;
   Tri T;
   int pn[6];
-  double u[4][6], P[6][5], us[6], vs[6];
+  double u[4][6], P[6][NR], us[6], vs[6];
 #pragma unroll
   for (int q = 0; q < 4; q++)
 #pragma unroll
@@ -327,7 +334,7 @@ __global__ void __launch_bounds__(64) k_rhs(Dev d, const double *usn, const doub
 #pragma unroll
   for (int k = 0; k < 6; k++)
 #pragma unroll
-    for (int v = 0; v < 5; v++) P[k][v] = d.tpart[(v * 6 + k) * nt + it];
+    for (int v = 0; v < NR; v++) P[k][v] = d.tpart[(v * 6 + k) * nt + it];
   load(d, it, pn, T);
 #pragma unroll
   for (int k = 0; k < 6; k++) {
@@ -340,12 +347,12 @@ __global__ void __launch_bounds__(64) k_rhs(Dev d, const double *usn, const doub
   for (int q = 0; q < 4; q++)
 #pragma unroll
     for (int k = 0; k < 6; k++) R[q][k] = 0.0;
-  face_node<0>(T, us[0], vs[0], P[0], R);
-  face_node<1>(T, us[1], vs[1], P[1], R);
-  face_node<2>(T, us[2], vs[2], P[2], R);
-  face_node<3>(T, us[3], vs[3], P[3], R);
-  face_node<4>(T, us[4], vs[4], P[4], R);
-  face_node<5>(T, us[5], vs[5], P[5], R);
+  face_node<0, NR>(T, us[0], vs[0], P[0], R);
+  face_node<1, NR>(T, us[1], vs[1], P[1], R);
+  face_node<2, NR>(T, us[2], vs[2], P[2], R);
+  face_node<3, NR>(T, us[3], vs[3], P[3], R);
+  face_node<4, NR>(T, us[4], vs[4], P[4], R);
+  face_node<5, NR>(T, us[5], vs[5], P[5], R);
   // volume integral (cofactor form, 7-point rule) and, on Taylor-Green, the
   // energy source on the same points
   const double csrc = d.ncase == 1 ? 0.25 * 3.14159265358979311599796346854 / (g - 1.0) : 0.0;
@@ -421,10 +428,14 @@ __global__ void __launch_bounds__(64) k_rhs(Dev d, const double *usn, const doub
 }  // namespace tri
 
 void launch_fast_tri_corner(const Dev &d, cudaStream_t st) {
-  if (d.ntria) tri::k_corner<<<(d.ntria + 63) / 64, 64, 0, st>>>(d);
+  if (!d.ntria) return;
+  if (d.nrow == 3) tri::k_corner<3><<<(d.ntria + 63) / 64, 64, 0, st>>>(d);
+  else tri::k_corner<5><<<(d.ntria + 63) / 64, 64, 0, st>>>(d);
 }
 void launch_fast_tri_rhs(const Dev &d, cudaStream_t st, const double *usn, const double *vsn, int fuse, double alfa) {
-  if (d.ntria) tri::k_rhs<<<(d.ntria + 63) / 64, 64, 0, st>>>(d, usn, vsn, fuse, alfa);
+  if (!d.ntria) return;
+  if (d.nrow == 3) tri::k_rhs<3><<<(d.ntria + 63) / 64, 64, 0, st>>>(d, usn, vsn, fuse, alfa);
+  else tri::k_rhs<5><<<(d.ntria + 63) / 64, 64, 0, st>>>(d, usn, vsn, fuse, alfa);
 }
 
 }  // namespace lag2d
