@@ -6,8 +6,8 @@
 //    (cell: getcellvol_lag 6x6; sub-cells: getrhosubg_averg 5x5) is exact for
 //    those polynomial integrands, so it is evaluated in closed form from the
 //    36 node cross products x_i y_j - x_j y_i (lag2d_tables.inc);
-//  * det J at fixed points (Persson, sub-cell densities, source) comes from its
-//    16 bicubic coefficients, a fixed linear map of the same cross products;
+//  * det J at fixed points (sub-cell densities, source) comes from its bicubic
+//    coefficients, built from those of the quad's map (lag2d_cell.cuh);
 //  * Jacobians on the 5x5 Gauss-Lobatto grid are sum-factorised on the 3x3
 //    tensor of quad nodes;
 //  * the corner pass reduces its 32 corner faces to per-node partial sums
@@ -321,258 +321,7 @@ __host__ __device__ __forceinline__ void load_u(const Dev &d, const double *U, i
     for (int k = 0; k < 6; k++) u[q][k] = U[(q * 6 + k) * (size_t)d.ncell + e];
 }
 
-// ---------------------------------------------------------------------------
-// Persson indicator (all quads).  The physical mass centre and the frame that
-// WENO needs are computed by WENO for its stencils, not here for every quad
-// (1024 x 1024: 110 -> 64 us a launch without their 13 loads and 6 stores).
-// ---------------------------------------------------------------------------
-__host__ __device__ void f_persson(const Dev &d, int iq) {
-  if (iq >= d.nquad || d.sc_dev->done) return;
-  const int e = iq + d.ntria;
-  Loaded L;
-  load_cell(d, d.xs, d.ys, iq, L);
-  double c[36], D[16];
-  {
-    double xp[9][2];
-    node_xy_rel(L, xp);
-    cross36_rel(xp, c);
-  }
-  detpoly(c, D);
-  const CellGeo g{d.rc[e], d.sc[e], d.g19[e], d.g20[e], d.g21[e]};
-  double t[6];
-#pragma unroll
-  for (int k = 0; k < 6; k++) t[k] = d.Us[k * (size_t)d.ncell + e];
-  double unvar2 = 0.0, unvar1 = 0.0;
-#pragma unroll
-  for (int i = 0; i < 5; i++) {
-    const double r = g5p(i);
-    const double dr = r - g.rc;
-    // along the row r: det J cubic, P1 part linear and P2 part quadratic in s
-    double e[4];
-#pragma unroll
-    for (int n = 0; n < 4; n++) e[n] = D[n] + r * (D[4 + n] + r * (D[8 + n] + r * D[12 + n]));
-    const double a0 = t[0] + t[1] * dr;
-    const double h0 = t[3] * (0.5 * dr * dr - g.g19) - t[4] * g.g20 - t[5] * g.g21;
-    const double h1 = t[5] * dr, h2 = 0.5 * t[4];
-    const double wi = g5w(i);
-#pragma unroll
-    for (int j = 0; j < 5; j++) {
-      const double s = g5p(j);
-      const double ds = s - g.sc;
-      const double djaco = wi * g5w(j) * (e[0] + s * (e[1] + s * (e[2] + s * e[3])));
-      const double p1 = a0 + t[2] * ds;
-      const double hi = h0 + ds * (h1 + h2 * ds);
-      const double un = p1 + hi;
-      unvar2 += hi * hi * djaco;
-      unvar1 += un * un * djaco;
-    }
-  }
-  const double thr = -3.0 * log10(4.0) - 4.0;
-  const int fl = (log10(unvar2 / unvar1) <= thr) ? 0 : 1;
-  d.flag[e] = fl;
-  if (fl) {
-#ifdef __CUDA_ARCH__
-    const int slot = atomicAdd(d.wcount, 1);
-#else
-    const int slot = (*d.wcount)++;
-#endif
-    d.wlist[slot] = iq;
-  }
-}
-
-// Taylor-Green source moments el[k] += sum_g src(x_g) b_k(g) detJ_g w_g over
-// the 5x5 Gauss points.  cos(pi x) at the points by angle addition from the
-// centre node x_c: cos(pi x) = cos(pi x_c) cos(pi d) - sin(pi x_c) sin(pi d),
-// d = x - x_c, with the NSER-term series of cossin_pi_series when every node
-// of the cell lies within delta of the centre node in x and y (the quadratic
-// map then keeps |d| <= 1.5625 delta at the Gauss points): delta <= 0.09 for
-// 7 terms, 0.004 for 4, 0.0006 for 3; otherwise (NSER = 0) cospi at each
-// point.  The point loop has no branch.  The basis sums are taken per row:
-// b_k along a row is a polynomial in ds of degree <= 2.
-template <int NSER>
-__host__ __device__ __forceinline__ void tgv_source_rows(const Loaded &L, const CellGeo &G, const double D[16],
-                                                         double g, double el[6]) {
-  const double coef = 0.25 * 3.14159265358979311599796346854 / (g - 1.0);
-  const double xc = L.X[1][1], yc = L.Y[1][1];
-  const double cxc = cospi(xc), sxc = sinpi(xc), cyc = cospi(yc), syc = sinpi(yc);
-#pragma unroll 1
-  for (int i = 0; i < 5; i++) {
-    const double r = g5p(i), dr = r - G.rc;
-    double lr[3];
-    lag3(r, lr);
-    double Px[3], Py[3];
-#pragma unroll
-    for (int bb = 0; bb < 3; bb++) {
-      Px[bb] = lr[0] * (L.X[0][bb] - xc) + lr[1] * (L.X[1][bb] - xc) + lr[2] * (L.X[2][bb] - xc);
-      Py[bb] = lr[0] * (L.Y[0][bb] - yc) + lr[1] * (L.Y[1][bb] - yc) + lr[2] * (L.Y[2][bb] - yc);
-    }
-    double e[4];
-#pragma unroll
-    for (int n = 0; n < 4; n++) e[n] = D[n] + r * (D[4 + n] + r * (D[8 + n] + r * D[12 + n]));
-    const double wi = coef * g5w(i);
-    double m0 = 0.0, m1 = 0.0, m2 = 0.0;
-#pragma unroll
-    for (int j = 0; j < 5; j++) {
-      const double s = g5p(j), ds = s - G.sc;
-      double ls[3];
-      lag3(s, ls);
-      const double dx = Px[0] * ls[0] + Px[1] * ls[1] + Px[2] * ls[2];
-      const double dy = Py[0] * ls[0] + Py[1] * ls[1] + Py[2] * ls[2];
-      const double djaco = wi * g5w(j) * (e[0] + s * (e[1] + s * (e[2] + s * e[3])));
-      double cx, cy;
-      if (NSER > 0) {
-        double cdx, sdx, cdy, sdy;
-        cossin_pi_series<NSER>(dx, cdx, sdx);
-        cossin_pi_series<NSER>(dy, cdy, sdy);
-        cx = cxc * cdx - sxc * sdx;
-        cy = cyc * cdy - syc * sdy;
-      } else {
-        cx = cospi(xc + dx);
-        cy = cospi(yc + dy);
-      }
-      const double c3x = cx * (4.0 * cx * cx - 3.0), c3y = cy * (4.0 * cy * cy - 3.0);
-      const double src = (c3x * cy - c3y * cx) * djaco;
-      m0 += src;
-      m1 += src * ds;
-      m2 += src * ds * ds;
-    }
-    // b = (1, dr, ds, dr^2/2 - g19, ds^2/2 - g20, dr ds - g21) along the row
-    el[0] += m0;
-    el[1] += m0 * dr;
-    el[2] += m1;
-    el[3] += m0 * (0.5 * dr * dr - G.g19);
-    el[4] += 0.5 * m2 - G.g20 * m0;
-    el[5] += m1 * dr - G.g21 * m0;
-  }
-}
-__host__ __device__ __forceinline__ void tgv_source(const Loaded &L, const CellGeo &G, const double D[16], double g,
-                                                    double el[6]) {
-  double mx = 0.0, my = 0.0;
-#pragma unroll
-  for (int a = 0; a < 3; a++)
-#pragma unroll
-    for (int b = 0; b < 3; b++) {
-      mx = fmax(mx, fabs(L.X[a][b] - L.X[1][1]));
-      my = fmax(my, fabs(L.Y[a][b] - L.Y[1][1]));
-    }
-  const double delta = fmax(mx, my);
-  if (delta <= 0.0006) tgv_source_rows<3>(L, G, D, g, el);
-  else if (delta <= 0.004) tgv_source_rows<4>(L, G, D, g, el);
-  else if (delta <= 0.09) tgv_source_rows<7>(L, G, D, g, el);
-  else tgv_source_rows<0>(L, G, D, g, el);
-}
-
-// Taylor-Green energy source of the stage (rhsdomnsrcdg_lag_curvquad,
-// Getrhslag.f90:4070-4251), one thread per quad: it depends on the stage's
-// nodes and the reference geometry only; the RHS pass adds the 6 moments
-// (d.src, [6][nquad]).  A kernel of its own: inside the corner or RHS kernels
-// its registers and code cost those kernels more than its own launch.
-__host__ __device__ void f_tgv_src(const Dev &d, int iq) {
-  if (iq >= d.nquad || d.sc_dev->done) return;
-  const int e = iq + d.ntria;
-  Loaded L;
-  load_cell(d, d.xs, d.ys, iq, L);
-  double c[36], D[16];
-  {
-    double xp[9][2];
-    node_xy_rel(L, xp);
-    cross36_rel(xp, c);
-  }
-  detpoly(c, D);
-  const CellGeo G{d.rc[e], d.sc[e], d.g19[e], d.g20[e], d.g21[e]};
-  double el[6] = {0, 0, 0, 0, 0, 0};
-  tgv_source(L, G, D, d.gamlg, el);
-#pragma unroll
-  for (int k = 0; k < 6; k++) d.src[k * (size_t)d.nquad + iq] = el[k];
-}
-
-// ---------------------------------------------------------------------------
-// Corner pass: node partial sums of the Riemann coefficients + sub-cell
-// density corrections (getriem_quadsubg2 with getrhosubg_averg/_daverg)
-// ---------------------------------------------------------------------------
-// The corner pass runs as two kernels: f_corner_corr, the sub-cell density
-// corrections (written to d.corr), and f_faces (lag2d_tiles.cuh), the corner
-// faces with the corrections read back.  Each is compiled for 4 resident blocks
-// of 128 per SM (128 registers).  The corrections use the state before WENO,
-// beside which they run; WENO replaces those of the quads it limits.
-__host__ __device__ void f_corner_corr(const Dev &d, int iq) {
-  if (iq >= d.nquad || d.sc_dev->done) return;
-  const int e = iq + d.ntria;
-  Loaded L;
-  load_cell(d, d.xs, d.ys, iq, L);
-  double c[36], D[16];
-  {
-    double xp[9][2];
-    node_xy_rel(L, xp);
-    cross36_rel(xp, c);
-  }
-  detpoly(c, D);
-  const CellGeo G{d.rc[e], d.sc[e], d.g19[e], d.g20[e], d.g21[e]};
-  // the tau DOFs
-  double u[6];
-#pragma unroll
-  for (int k = 0; k < 6; k++) u[k] = d.Us[k * (size_t)d.ncell + e];
-  // sub-cell densities: initial mass / exact sub-cell area, and the DG-implied
-  // harmonic mean of tau over each sub-cell (5x5 Gauss per sub-cell)
-  double vsub4[4];
-  subareas(c, vsub4);
-  // The harmonic mean sum masel = sum_g w_g det_g / tau_g is kept as one
-  // fraction num / den (a/b + c/d = (a d + c b) / (b d)): three multiply-adds
-  // per point and one division per sub-cell instead of one division per point.
-  // tau is scaled by the cell-average tau first (rtc), so that the product of
-  // the 25 scaled values stays near 1; masel = rtc num / den.
-  // Sub-cells 0 and 3 (r in [-1, 0]) share their Gauss rows, and so do 1 and
-  // 2 (r in [0, 1]): each row's det J and tau coefficients serve both, whose
-  // two fraction chains (s in [-1, 0] and [0, 1]) run side by side.
-  const double rtc = 1.0 / u[0];
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const double ofr = h == 0 ? -1.0 : 1.0;
-    const int ilo = h == 0 ? 0 : 1, ihi = h == 0 ? 3 : 2;  // s in [-1, 0], [0, 1]
-    double nlo = 0.0, dlo = 1.0, nhi = 0.0, dhi = 1.0;
-#pragma unroll 1
-    for (int i = 0; i < 5; i++) {
-      const double r = (g5p(i) + ofr) / 2.0;
-      // along the row r, det J is a cubic and tau a quadratic in s
-      double e[4];
-#pragma unroll
-      for (int n = 0; n < 4; n++) e[n] = D[n] + r * (D[4 + n] + r * (D[8 + n] + r * D[12 + n]));
-      const double dr = r - G.rc;
-      const double t0 = rtc * (u[0] + u[1] * dr + u[3] * (0.5 * dr * dr - G.g19) - u[4] * G.g20 - u[5] * G.g21);
-      const double t1 = rtc * (u[2] + u[5] * dr), t2 = rtc * (0.5 * u[4]);
-      const double wi = 0.25 * g5w(i);
-#pragma unroll
-      for (int j = 0; j < 5; j++) {
-        const double w = wi * g5w(j);
-        {
-          const double s = (g5p(j) - 1.0) / 2.0;
-          const double ds = s - G.sc;
-          const double tau = t0 + ds * (t1 + t2 * ds);
-          const double det = e[0] + s * (e[1] + s * (e[2] + s * e[3]));
-          nlo = nlo * tau + (w * det) * dlo;
-          dlo = dlo * tau;
-        }
-        {
-          const double s = (g5p(j) + 1.0) / 2.0;
-          const double ds = s - G.sc;
-          const double tau = t0 + ds * (t1 + t2 * ds);
-          const double det = e[0] + s * (e[1] + s * (e[2] + s * e[3]));
-          nhi = nhi * tau + (w * det) * dhi;
-          dhi = dhi * tau;
-        }
-      }
-    }
-    // 1 / uqsgc = masel / volel with masel = rtc num / den
-#pragma unroll
-    for (int t = 0; t < 2; t++) {
-      const int isg = t == 0 ? ilo : ihi;
-      const double num = t == 0 ? nlo : nhi, den = t == 0 ? dlo : dhi;
-      const double unksgq = (1.0 / vsub4[isg]) * d.msub[isg * (size_t)d.nquad + iq];
-      const double volel = det_integral(D, (isg == 0 || isg == 3) ? -1.0 : 0.0, (isg == 0 || isg == 1) ? -1.0 : 0.0);
-      d.corr[isg * (size_t)d.nquad + iq] = d.cdrho * (unksgq - (rtc * num) / (den * volel));
-    }
-  }
-}
+#include "lag2d_cell.cuh"
 
 // ---------------------------------------------------------------------------
 // Node pass: gather the per-cell partial sums in cell order, 2x2 solve and
@@ -1890,11 +1639,11 @@ __host__ __device__ void a_centre(const Dev &d, const Adj &a, int p) {
 
 #include "lag2d_tiles.cuh"
 
-__global__ void __launch_bounds__(128) k_persson2(Dev d) { f_persson(d, blockIdx.x * blockDim.x + threadIdx.x); }
+__global__ void __launch_bounds__(128, 8) k_persson2(Dev d) { f_persson(d, blockIdx.x * blockDim.x + threadIdx.x); }
 __global__ void __launch_bounds__(128, LAG2D_CCORR_MINB) k_corner2_corr(Dev d) {
   f_corner_corr(d, blockIdx.x * blockDim.x + threadIdx.x);
 }
-__global__ void __launch_bounds__(128) k_tgv_src2(Dev d) { f_tgv_src(d, blockIdx.x * blockDim.x + threadIdx.x); }
+__global__ void __launch_bounds__(128, 4) k_tgv_src2(Dev d) { f_tgv_src(d, blockIdx.x * blockDim.x + threadIdx.x); }
 template <bool MOVE, int NR>
 __global__ void __launch_bounds__(256) k_node2(Dev d, double alfa) {
   f_node<MOVE, NR>(d, blockIdx.x * blockDim.x + threadIdx.x, alfa);
