@@ -23,12 +23,11 @@
 #ifndef LAG2D_ACF_MINB
 #define LAG2D_ACF_MINB 2
 #endif
-// the RHS kernel: 2 resident blocks of kRhsBlock per SM leave it up to 255
-// registers and no spills (on the 1024 x 1024 Taylor-Green step 1.11 ms per
-// step against 1.49 ms at 3 blocks and 168 registers with 584 bytes of
-// spill loads per thread)
+// the RHS kernel: 4 resident blocks of 64 per SM leave it up to 255 registers and
+// no spills (at 5 or 6 and 168 registers with 480 bytes of spill loads per thread
+// 350 us a launch on 1024 x 1024 against 270)
 #ifndef LAG2D_RHS_MINB
-#define LAG2D_RHS_MINB 2
+#define LAG2D_RHS_MINB 4
 #endif
 #ifndef LAG2D_FACES_MINB
 #define LAG2D_FACES_MINB 4
@@ -455,107 +454,151 @@ __host__ __device__ __forceinline__ void mass_flux_weights(const Loaded &L, int 
 // with u* the node's new velocity and m_f, sigma.n A w_f, u_k what the corner
 // pass used (Getrhslaggauss.f90:10409-10867).  The momentum sum is therefore
 // affine in u*: sum_f F_f = u* P0 - (P1, P2), where P0..P2 are the node partial
-// sums the corner pass wrote (sum m, sum m u_k - sigma.n A w); the energy term is u* . sum_f F_f; the mass term is
-// u* . sum_f 2 w_mass,f an_f over the 16 outer corner faces.  So the corner
-// data are not recomputed here: 24 partials and the 8 boundary nodes'
-// velocities replace the 32 corner faces' vertex states, impedances and
-// forces (same sums up to rounding and summation order).
+// sums the corner pass wrote (sum m, sum m u_k - sigma.n A w); the energy
+// term is u* . sum_f F_f; the mass term is u* . t with t the sum of 2 w_mass,f
+// an_f over the node's outer corner faces (node_flux).  So the corner data are
+// not recomputed here: 24 partials and the 8 boundary nodes' velocities replace
+// the 32 corner faces' vertex states, impedances and forces (same sums up to
+// rounding and summation order).  The nodes sit at -1, 0, 1 in r and s, so the
+// moments over 1, r, s, r^2, s^2, r s are sums and differences; the basis about
+// (rc, sc) is taken once at the end.
+//
+// Volume integral on the 5x5 Gauss-Lobatto grid (cofactor form).  Along the row
+// r_i the Jacobian entries are polynomials in s from the map's coefficients.
+// Every equation adds (alpha, beta) . grad b with
+//   mass -(u y_s - v x_s, v x_r - u y_r), x momentum p (y_s, -y_r),
+//   y momentum p (-x_s, x_r), energy p times minus the mass's,
+// and grad b = (1, 0), (0, 1), (dr, 0), (0, ds), (ds, dr), so a row needs the
+// sums of alpha and beta with weights 1 and s only: 16 sums instead of 20 x 5
+// terms.
 //
 // Staging: the cell's DOFs U^(s) (24 values) and, for the fused update, M^-1
 // (16) and U^n (24) are copied asynchronously (cp.async) into this thread's
 // column of shared memory (stride kRhsBlock) when the thread starts, so their
 // load latency overlaps the face integral and they are read from shared
 // memory where used instead of being held in registers.
-constexpr int kRhsBlock = 128;
+//
+// 1024 x 1024: 341 -> 270 us a launch (65% of the copy rate, FP64 pipe 40%, 8 warps
+// an SM by its 254 registers); 256 x 256 29 -> 24.5.  Rows unrolled, 152 bytes of
+// spills: 8% slower a step.  The map's coefficients in shared memory in place of
+// U^n, which is then copied after the rows: 289.
+constexpr int kRhsBlock = 64;
 constexpr int kRhsStage = 64;
+// the rule of the rolled row loop
+__constant__ double cL5[5] = {-1.0, -0.6546536707079771437983, 0.0, 0.6546536707079771437983, 1.0};
+__constant__ double cLw[5] = {0.1, 0.544444444444444444444, 0.7111111111111111111111, 0.544444444444444444444, 0.1};
+constexpr double kMassCorner = 1.0 / 3.0, kMassEdge = 2.0 / 3.0;
+// t of a corner node (previous corner p and edge node q, next corner n and edge
+// node e) and of the edge node between the corners c and n
+__device__ __forceinline__ void corner_flux(double px, double py, double qx, double qy, double ex, double ey, double nx,
+                                            double ny, double &tx, double &ty) {
+  tx = kMassCorner * (2.0 * (ey - qy) + 0.5 * (py - ny));
+  ty = kMassCorner * (2.0 * (qx - ex) + 0.5 * (nx - px));
+}
+__device__ __forceinline__ void edge_flux(double cx, double cy, double nx, double ny, double &tx, double &ty) {
+  tx = kMassEdge * (ny - cy);
+  ty = kMassEdge * (cx - nx);
+}
+// moments of 8 node values over the basis about (rc, sc); c = (rc^2/2 - g19, sc^2/2 - g20, rc sc - g21)
+__device__ __forceinline__ void node_moments(const double f[8], double rc, double sc, const double c[3], double R[6]) {
+  const double a = f[1] + f[2], b = f[0] + f[3], cs = a + b, ex = f[5] + f[7], ey = f[4] + f[6];
+  const double xx = cs + ex, m0 = xx + ey;
+  const double mx = (a - b) + (f[5] - f[7]), my = ((f[2] + f[3]) - (f[0] + f[1])) + (f[6] - f[4]);
+  R[0] = m0;
+  R[1] = mx - rc * m0;
+  R[2] = my - sc * m0;
+  R[3] = 0.5 * xx - rc * mx + c[0] * m0;
+  R[4] = 0.5 * (cs + ey) - sc * my + c[1] * m0;
+  R[5] = ((f[0] + f[2]) - (f[1] + f[3])) - rc * my - sc * mx + c[2] * m0;
+}
 __device__ void f_rhs3(const Dev &d, int iq, int fuse_update, double alfa, double *col) {
   if (iq >= d.nquad || d.sc_dev->done) return;
   const int e = iq + d.ntria;
-  const double eps = 1.0e-6, g = d.gamlg;
-  {
-    const size_t nc = d.ncell;
-    for (int v = 0; v < 24; v++) __pipeline_memcpy_async(col + v * kRhsBlock, d.Us + v * nc + e, sizeof(double));
-    if (fuse_update) {
-      for (int i = 0; i < 16; i++)
-        __pipeline_memcpy_async(col + (24 + i) * kRhsBlock, d.amatr + i * nc + e, sizeof(double));
-      if (alfa != 0.0)
-        for (int v = 0; v < 24; v++)
-          __pipeline_memcpy_async(col + (40 + v) * kRhsBlock, d.Un + v * nc + e, sizeof(double));
-    }
-    __pipeline_commit();
-    // the node partial sums of the 8 boundary nodes (and the source moments)
-    // towards L2 while the coordinates are gathered: their loads in the face
-    // loop then wait on L2, not HBM (RHS pass 1.635 -> 1.507 ms per step on
-    // the 1024x1024 Taylor-Green mesh)
-    const size_t nq = d.nquad;
+  const double eps = 1.0e-6, gm = d.gamlg - 1.0;
+  const size_t nq = d.nquad, nc = d.ncell;
+  for (int v = 0; v < 24; v++) __pipeline_memcpy_async(col + v * kRhsBlock, d.Us + v * nc + e, sizeof(double));
+  if (fuse_update) {
+    for (int i = 0; i < 16; i++)
+      __pipeline_memcpy_async(col + (24 + i) * kRhsBlock, d.amatr + i * nc + e, sizeof(double));
+    if (alfa != 0.0)
+      for (int v = 0; v < 24; v++)
+        __pipeline_memcpy_async(col + (40 + v) * kRhsBlock, d.Un + v * nc + e, sizeof(double));
+  }
+  __pipeline_commit();
+  // the node partial sums of the 8 boundary nodes (and the source moments)
+  // towards L2 while the coordinates are gathered
 #pragma unroll
-    for (int v = 0; v < 3; v++)
+  for (int v = 0; v < 3; v++)
 #pragma unroll
-      for (int k = 0; k < 8; k++) asm volatile("prefetch.global.L2 [%0];" ::"l"(d.npart + (v * 9 + k) * nq + iq));
-    if (d.ncase == 1) {
+    for (int k = 0; k < 8; k++) asm volatile("prefetch.global.L2 [%0];" ::"l"(d.npart + (v * 9 + k) * nq + iq));
+  if (d.ncase == 1) {
 #pragma unroll
-      for (int k = 0; k < 6; k++) asm volatile("prefetch.global.L2 [%0];" ::"l"(d.src + k * nq + iq));
-    }
+    for (int k = 0; k < 6; k++) asm volatile("prefetch.global.L2 [%0];" ::"l"(d.src + k * nq + iq));
   }
 #define RHS_U(q, k) col[((q) * 6 + (k)) * kRhsBlock]
-  Loaded L;
-  load_cell(d, d.xs, d.ys, iq, L);
   const CellGeo G{d.rc[e], d.sc[e], d.g19[e], d.g20[e], d.g21[e]};
-  double ul[6] = {0, 0, 0, 0, 0, 0}, p0[6] = {0, 0, 0, 0, 0, 0}, p1[6] = {0, 0, 0, 0, 0, 0}, el[6] = {0, 0, 0, 0, 0, 0};
+  double R[4][6];
+  QuadMap m;
+  {
+    Loaded L;
+    load_cell(d, d.xs, d.ys, iq, L);
+    const int A[8] = {0, 2, 2, 0, 1, 2, 1, 0}, B[8] = {0, 0, 2, 2, 0, 1, 2, 1};
+    double tw[8], f0[8], f1[8], fe[8];
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
-    double b[6];
-    node_basis2(G, k, b);
-    const int pn = d.ipq[k * d.nquad + iq];
-    const double un = d.us_new[pn], vn = d.vs_new[pn];
-    double tx, ty;
-    mass_flux_weights(L, k, tx, ty);
-    const double tw = un * tx + vn * ty;
-    const size_t nq = d.nquad;
-    const double P0 = d.npart[(0 * 9 + k) * nq + iq];
-    const double f0 = un * P0 - d.npart[(1 * 9 + k) * nq + iq];
-    const double f1 = vn * P0 - d.npart[(2 * 9 + k) * nq + iq];
-    const double fe = un * f0 + vn * f1;
-#pragma unroll
-    for (int kk = 0; kk < 6; kk++) {
-      ul[kk] += tw * b[kk];
-      p0[kk] += f0 * b[kk];
-      p1[kk] += f1 * b[kk];
-      el[kk] += fe * b[kk];
+    for (int k = 0; k < 8; k++) {
+      const int pn = d.ipq[k * nq + iq];
+      const double un = d.us_new[pn], vn = d.vs_new[pn];
+      const double P0 = d.npart[(0 * 9 + k) * nq + iq];
+      f0[k] = un * P0 - d.npart[(1 * 9 + k) * nq + iq];
+      f1[k] = vn * P0 - d.npart[(2 * 9 + k) * nq + iq];
+      fe[k] = un * f0[k] + vn * f1[k];
+      const int v = k & 3, n = (v + 1) & 3, p = (v + 3) & 3, q = 4 + p;
+      double tx, ty;
+      if (k < 4)
+        corner_flux(L.X[A[p]][B[p]], L.Y[A[p]][B[p]], L.X[A[q]][B[q]], L.Y[A[q]][B[q]], L.X[A[4 + v]][B[4 + v]],
+                    L.Y[A[4 + v]][B[4 + v]], L.X[A[n]][B[n]], L.Y[A[n]][B[n]], tx, ty);
+      else
+        edge_flux(L.X[A[v]][B[v]], L.Y[A[v]][B[v]], L.X[A[n]][B[n]], L.Y[A[n]][B[n]], tx, ty);
+      tw[k] = un * tx + vn * ty;
     }
+    const double c[3] = {0.5 * G.rc * G.rc - G.g19, 0.5 * G.sc * G.sc - G.g20, G.rc * G.sc - G.g21};
+    node_moments(tw, G.rc, G.sc, c, R[0]);
+    node_moments(f0, G.rc, G.sc, c, R[1]);
+    node_moments(f1, G.rc, G.sc, c, R[2]);
+    node_moments(fe, G.rc, G.sc, c, R[3]);
+    map_coeffs(L.X, m.a);
+    map_coeffs(L.Y, m.b);
   }
   __pipeline_wait_prior(0);
   if (d.flag[e] == 2) {
     // the moments WENO replaced (they are not committed to the stage state)
 #pragma unroll 1
-    for (int v = 0; v < 20; v++) col[(v / 5 * 6 + v % 5 + 1) * kRhsBlock] = d.Uw[v * (size_t)d.nquad + iq];
+    for (int v = 0; v < 20; v++) col[(v / 5 * 6 + v % 5 + 1) * kRhsBlock] = d.Uw[v * nq + iq];
   }
-  // volume integral on the 5x5 Gauss-Lobatto grid (cofactor form), sum
-  // factorised row by row: for fixed r_i, Q_b = sum_a L'_a(r_i) X[a][b] and
-  // P_b = sum_a L_a(r_i) X[a][b] give dx/dr and dx/ds along the row
 #pragma unroll 1
   for (int i = 0; i < 5; i++) {
-    const double r = l5p(i), dr = r - G.rc;
-    double lr[3], dlr[3];
-    lag3(r, lr);
-    dlag3(r, dlr);
-    double Qx[3], Qy[3], Px[3], Py[3];
+    const double r = cL5[i], dr = r - G.rc;
+    // x_r = xr[0] + s (xr[1] + s xr[2]), x_s = xs[0] + s xs[1]
+    double xr[3], yr[3], xs[2], ys[2];
 #pragma unroll
-    for (int bb = 0; bb < 3; bb++) {
-      Qx[bb] = dlr[0] * L.X[0][bb] + dlr[1] * L.X[1][bb] + dlr[2] * L.X[2][bb];
-      Qy[bb] = dlr[0] * L.Y[0][bb] + dlr[1] * L.Y[1][bb] + dlr[2] * L.Y[2][bb];
-      Px[bb] = lr[0] * L.X[0][bb] + lr[1] * L.X[1][bb] + lr[2] * L.X[2][bb];
-      Py[bb] = lr[0] * L.Y[0][bb] + lr[1] * L.Y[1][bb] + lr[2] * L.Y[2][bb];
+    for (int n = 0; n < 3; n++) {
+      xr[n] = m.a[1][n] + (2.0 * r) * m.a[2][n];
+      yr[n] = m.b[1][n] + (2.0 * r) * m.b[2][n];
+    }
+#pragma unroll
+    for (int n = 0; n < 2; n++) {
+      const double c = n + 1.0;
+      xs[n] = c * (m.a[0][n + 1] + r * (m.a[1][n + 1] + r * m.a[2][n + 1]));
+      ys[n] = c * (m.b[0][n + 1] + r * (m.b[1][n + 1] + r * m.b[2][n + 1]));
     }
     // the DOFs along the row: u_q(s) = a_q + ds (b_q + c_q ds), ds = s - sc
     double ra[4], rb[4];
+    const double b3 = 0.5 * dr * dr - G.g19;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      ra[q] = RHS_U(q, 0) + RHS_U(q, 1) * dr + RHS_U(q, 3) * (0.5 * dr * dr - G.g19) - RHS_U(q, 4) * G.g20 -
-              RHS_U(q, 5) * G.g21;
+      ra[q] = RHS_U(q, 0) + RHS_U(q, 1) * dr + RHS_U(q, 3) * b3 - RHS_U(q, 4) * G.g20 - RHS_U(q, 5) * G.g21;
       rb[q] = RHS_U(q, 2) + RHS_U(q, 5) * dr;
     }
-    const double wi = l5w(i);
     // 1/tau at the row's 5 points with one division (batched reciprocals:
     // prefix products, one reciprocal of the last, then back substitution)
     double rtau[5];
@@ -575,71 +618,69 @@ __device__ void f_rhs3(const Dev &d, int iq, int fuse_update, double alfa, doubl
       }
       rtau[0] = inv;
     }
+    // sums over the row of (alpha, beta) with weights w_j and w_j s_j
+    double A0[4] = {0, 0, 0, 0}, A1[4] = {0, 0, 0, 0}, B0[4] = {0, 0, 0, 0}, B1[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int j = 0; j < 5; j++) {
-      const double s = l5p(j), ds = s - G.sc;
-      double ls[3], dls[3];
-      lag3(s, ls);
-      dlag3(s, dls);
-      const double w = wi * l5w(j);
-      const double xr = Qx[0] * ls[0] + Qx[1] * ls[1] + Qx[2] * ls[2];
-      const double yr = Qy[0] * ls[0] + Qy[1] * ls[1] + Qy[2] * ls[2];
-      const double xs = Px[0] * dls[0] + Px[1] * dls[1] + Px[2] * dls[2];
-      const double ys = Py[0] * dls[0] + Py[1] * dls[1] + Py[2] * dls[2];
+      const double s = l5p(j), ds = s - G.sc, w = l5w(j);
+      const double jxr = xr[0] + s * (xr[1] + s * xr[2]), jyr = yr[0] + s * (yr[1] + s * yr[2]);
+      const double jxs = xs[0] + s * xs[1], jys = ys[0] + s * ys[1];
       double un[4];
 #pragma unroll
       for (int q = 1; q < 4; q++) un[q] = ra[q] + ds * (rb[q] + 0.5 * RHS_U(q, 4) * ds);
-      const double rhoad = rtau[j];
-      const double pres = fmax(eps, (g - 1.0) * rhoad * (un[3] - 0.5 * (un[1] * un[1] + un[2] * un[2])));
-      // G . grad_xi b for b = 2..6: dbdr = (1, 0, dr, 0, ds), dbds = (0, 1, 0, ds, dr)
-      // (the FP32-mixed kernel sums these per row instead; here the row sums'
-      // 16 extra accumulators cost more in spills than the 16 operations a
-      // point they save)
-      double gd0[5], gd1[5];
-      gd0[0] = ys;       gd1[0] = -xs;
-      gd0[1] = -yr;      gd1[1] = xr;
-      gd0[2] = ys * dr;  gd1[2] = -xs * dr;
-      gd0[3] = -yr * ds; gd1[3] = xr * ds;
-      gd0[4] = ys * ds - yr * dr;
-      gd1[4] = -xs * ds + xr * dr;
+      const double pres = fmax(eps, gm * rtau[j] * (un[3] - 0.5 * (un[1] * un[1] + un[2] * un[2])));
+      const double al = jys * un[1] - jxs * un[2], be = jxr * un[2] - jyr * un[1];
       const double wp = w * pres;
-#pragma unroll
-      for (int kk = 0; kk < 5; kk++) {
-        const double fv = gd0[kk] * un[1] + gd1[kk] * un[2];
-        ul[kk + 1] -= fv * w;
-        p0[kk + 1] += gd0[kk] * wp;
-        p1[kk + 1] += gd1[kk] * wp;
-        el[kk + 1] += fv * wp;
+      A0[0] += w * al;
+      B0[0] += w * be;
+      A0[1] += wp * jys;
+      B0[1] -= wp * jyr;
+      A0[2] -= wp * jxs;
+      B0[2] += wp * jxr;
+      A0[3] += wp * al;
+      B0[3] += wp * be;
+      if (j != 2) {
+        const double ws = w * s, wps = wp * s;
+        A1[0] += ws * al;
+        B1[0] += ws * be;
+        A1[1] += wps * jys;
+        B1[1] -= wps * jyr;
+        A1[2] -= wps * jxs;
+        B1[2] += wps * jxr;
+        A1[3] += wps * al;
+        B1[3] += wps * be;
       }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const double wi = q == 0 ? -cLw[i] : cLw[i], wr = wi * dr;
+      R[q][1] += wi * A0[q];
+      R[q][2] += wi * B0[q];
+      R[q][3] += wr * A0[q];
+      R[q][4] += wi * (B1[q] - G.sc * B0[q]);
+      R[q][5] += wi * (A1[q] - G.sc * A0[q]) + wr * B0[q];
     }
   }
   if (d.ncase == 1) {
-    // Taylor-Green energy source, computed by k_tgv_src2 before the corner pass
+    // Taylor-Green energy source, computed by k_tgv_src2
 #pragma unroll
-    for (int k = 0; k < 6; k++) el[k] += d.src[k * (size_t)d.nquad + iq];
+    for (int k = 0; k < 6; k++) R[3][k] += d.src[k * nq + iq];
   }
   if (!fuse_update) {
 #pragma unroll
-    for (int k = 0; k < 6; k++) {
-      d.rhs[(0 * 6 + k) * (size_t)d.ncell + e] = ul[k];
-      d.rhs[(1 * 6 + k) * (size_t)d.ncell + e] = p0[k];
-      d.rhs[(2 * 6 + k) * (size_t)d.ncell + e] = p1[k];
-      d.rhs[(3 * 6 + k) * (size_t)d.ncell + e] = el[k];
-    }
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+      for (int k = 0; k < 6; k++) d.rhs[(q * 6 + k) * nc + e] = R[q][k];
     return;
   }
   // fused stage update (Getrhslag.f90:1789-1904)
   const double dt = d.sc_dev->dtfix;
 #define RHS_AM(i) col[(24 + (i)) * kRhsBlock]
 #define RHS_UN(v) col[(40 + (v)) * kRhsBlock]
-  double R[4][6];
 #pragma unroll
-  for (int k = 0; k < 6; k++) {
-    R[0][k] = dt * ul[k];
-    R[1][k] = dt * p0[k];
-    R[2][k] = dt * p1[k];
-    R[3][k] = dt * el[k];
-  }
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int k = 0; k < 6; k++) R[q][k] = dt * R[q][k];
   const double oma = 1.0 - alfa;
   // symmetric 5x5 block rows from the packed upper triangle, M(1,1) = amatr(16)
   const int IDX[5][5] = {{0, 1, 2, 3, 4}, {1, 5, 6, 7, 8}, {2, 6, 9, 10, 11}, {3, 7, 10, 12, 13}, {4, 8, 11, 13, 14}};
