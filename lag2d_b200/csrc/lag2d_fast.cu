@@ -32,6 +32,12 @@
 #ifndef LAG2D_FACES_MINB
 #define LAG2D_FACES_MINB 4
 #endif
+#ifndef LAG2D_FACES4_MINB
+#define LAG2D_FACES4_MINB 4
+#endif
+#ifndef LAG2D_RHS4_MINB
+#define LAG2D_RHS4_MINB 4
+#endif
 #ifndef LAG2D_AREVF_MINB
 #define LAG2D_AREVF_MINB 3
 #endif
@@ -572,8 +578,11 @@ __device__ void f_rhs3(const Dev &d, int iq, int fuse_update, double alfa, doubl
   __pipeline_wait_prior(0);
   if (d.flag[e] == 2) {
     // the moments WENO replaced (they are not committed to the stage state)
-#pragma unroll 1
-    for (int v = 0; v < 20; v++) col[(v / 5 * 6 + v % 5 + 1) * kRhsBlock] = d.Uw[v * nq + iq];
+    double w[20];
+#pragma unroll
+    for (int v = 0; v < 20; v++) w[v] = d.Uw[v * nq + iq];
+#pragma unroll
+    for (int v = 0; v < 20; v++) col[(v / 5 * 6 + v % 5 + 1) * kRhsBlock] = w[v];
   }
 #pragma unroll 1
   for (int i = 0; i < 5; i++) {
@@ -1819,8 +1828,22 @@ void launch_fast_persson(const Dev &d, cudaStream_t st) { fast::k_persson2<<<fas
 void launch_fast_corr(const Dev &d, cudaStream_t st) {
   fast::k_corner2_corr<<<fast::nb(d.nquad, 128), 128, 0, st>>>(d);
 }
+// Four lanes per quad while the mesh is small, where a launch takes as long as a
+// thread's chain; one thread per quad from where the chip is full several times
+// over and the lanes' repeated loads and centre state count.
+// Faces, us a step with one thread and with four lanes: 16 x 16 88 / 73, 64 x 64
+// 98 / 82, 128 x 128 110 / 100, 256 x 256 206 / 204, 512 x 512 704 / 696,
+// 1024 x 1024 2531 / 2566.
+constexpr int kFaces4Max = 512 * 512;
+// RHS (255 registers either way): 16 x 16 73 / 69, 64 x 64 82 / 77, 128 x 128
+// 100 / 102, 256 x 256 204 / 236, so one wave of its blocks on 148 SMs.
+constexpr int kRhs4Max = 148 * 4 * (fast::kRhs4Block / 4);
 void launch_fast_faces(const Dev &d, cudaStream_t st) {
   constexpr int smem = fast::kFaceRows * fast::kFaceBlock * sizeof(double);
+  if (d.nquad <= kFaces4Max) {
+    fast::k_faces4<<<fast::nb(4 * d.nquad, fast::kFace4Block), fast::kFace4Block, 0, st>>>(d);
+    return;
+  }
   fast::k_faces<<<fast::nb(d.nquad, fast::kFaceBlock), fast::kFaceBlock, smem, st>>>(d);
 }
 void launch_fast_src(const Dev &d, cudaStream_t st) { fast::k_tgv_src2<<<fast::nb(d.nquad, 128), 128, 0, st>>>(d); }
@@ -1836,6 +1859,10 @@ void launch_fast_node(const Dev &d, cudaStream_t st, int move, double alfa) {
 }
 void launch_fast_rhs(const Dev &d, cudaStream_t st, int fuse, double alfa) {
   constexpr int smem = fast::kRhsStage * fast::kRhsBlock * sizeof(double);
+  if (d.nquad <= kRhs4Max) {
+    fast::k_rhs4<<<fast::nb(4 * d.nquad, fast::kRhs4Block), fast::kRhs4Block, 0, st>>>(d, fuse, alfa);
+    return;
+  }
   fast::k_rhs3<<<fast::nb(d.nquad, fast::kRhsBlock), fast::kRhsBlock, smem, st>>>(d, fuse, alfa);
 }
 // shared-memory limits of the kernels above 48 KB, on the current device
