@@ -385,8 +385,8 @@ struct StageRec {
 // velocities give, so dt follows the node pass and every RHS pass carries its
 // update.  Independent passes run beside the main chain when the step is
 // captured (h->forking): the sub-cell corrections beside the Persson pass, the
-// triangles' corners and the source beside both, the geometry of the new
-// nodes and the next stage's source beside the RHS pass.  On a small mesh a
+// triangles' corners and the source beside both, the motion of stage 1, the geometry
+// of the new nodes and the next stage's source beside the RHS pass.  On a small mesh a
 // stage is then a chain of 6 launches instead of 11 (64 x 64: 160 -> 113 us a
 // step); on a large one (1024 x 1024: 3.48 -> 3.37 ms) the
 // source, bound by FP64 arithmetic, overlaps passes that wait on memory.
@@ -460,7 +460,8 @@ static void enqueue_step_fast(lag2d_handle *h, int itime, const StageRec *rec = 
       run(h, "dt", [&] { launch_fast_dt(d, s0, h->cfg.ndt, itime); });
       if (rec)
         cudaMemcpyAsync(rec->dt + rec->step, &d.sc_dev->dtfix, sizeof(double), cudaMemcpyDeviceToDevice, s0);
-      run(h, "nodes", [&] { launch_fast_nodes(d, s0, alfa); });
+      after(s2, s0);  // the motion beside the RHS pass, which works on the old nodes
+      run(h, "nodes", [&] { launch_fast_nodes(d, s2, alfa); });
     }
     // volumes and centre nodes at the new coordinates, then the next stage's source
     Dev dx = d;

@@ -17,6 +17,7 @@
 //    the RHS pass.
 #include <cuda_pipeline.h>
 #include <cuda_runtime.h>
+#include "lag2d_launch.cuh"
 #ifndef LAG2D_ACC_MINB
 #define LAG2D_ACC_MINB 3
 #endif
@@ -379,6 +380,7 @@ __device__ void f_node(const Dev &d, int p, double alfa) {
   int id[4];
 #pragma unroll
   for (int j = 0; j < 4; j++) id[j] = b + j < en ? d.node_slot[b + j] : 0;
+  await_previous();  // the corner passes: partial sums
   if (done) return;
   double s[NR];
 #pragma unroll
@@ -517,7 +519,10 @@ __device__ __forceinline__ void node_moments(const double f[8], double rc, doubl
   R[4] = 0.5 * (cs + ey) - sc * my + c[1] * m0;
   R[5] = ((f[0] + f[2]) - (f[1] + f[3])) - rc * my - sc * mx + c[2] * m0;
 }
+// AHEAD: the state, geometry and partial sums are read ahead of the wait
+template <bool AHEAD>
 __device__ void f_rhs3(const Dev &d, int iq, int fuse_update, double alfa, double *col) {
+  if (!AHEAD) await_previous();
   if (iq >= d.nquad || d.sc_dev->done) return;
   const int e = iq + d.ntria;
   const double eps = 1.0e-6, gm = d.gamlg - 1.0;
@@ -550,6 +555,7 @@ __device__ void f_rhs3(const Dev &d, int iq, int fuse_update, double alfa, doubl
     load_cell(d, d.xs, d.ys, iq, L);
     const int A[8] = {0, 2, 2, 0, 1, 2, 1, 0}, B[8] = {0, 0, 2, 2, 0, 1, 2, 1};
     double tw[8], f0[8], f1[8], fe[8];
+    if (AHEAD) await_previous();  // the node pass, in stage 1 the time step
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const int pn = d.ipq[k * nq + iq];
@@ -721,21 +727,32 @@ __device__ void f_rhs3(const Dev &d, int iq, int fuse_update, double alfa, doubl
 // with the same per-node sums as f_rhs3.  With dt known before the RHS pass,
 // stage 1 fuses its M^-1 solve and update into the RHS kernel like the later
 // stages.  Edge lengths use the stage's nodes, which in stage 1 are x^n.
-__host__ __device__ void f_dt_quad(const Dev &d, int iq, double &dtcfl, double &dtvol) {
+__device__ void f_dt_quad(const Dev &d, int iq, double &dtcfl, double &dtvol) {
   dtcfl = 1e10;
   dtvol = 1e10;
-  if (iq >= d.nquad || d.sc_dev->done) return;
+  const bool mine = iq < d.nquad && !d.sc_dev->done;
+  if (!mine) {
+    await_previous();
+    return;
+  }
   const int e = iq + d.ntria;
   const double eps = 1.0e-6, g = d.gamlg;
+  const size_t nc = d.ncell;
+  int pn[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) pn[k] = d.ipq[k * d.nquad + iq];
   Loaded L;
   load_cell(d, d.xs, d.ys, iq, L);
+  const double rhomc = d.Us[0 * nc + e];
+  const double uctr = d.Us[6 * nc + e], vctr = d.Us[12 * nc + e], ectr = d.Us[18 * nc + e];
+  const double vol = d.vol[e];
+  await_previous();  // the node pass: u*
   double dvdt = 0.0;
 #pragma unroll
   for (int k = 0; k < 8; k++) {
-    const int pn = d.ipq[k * d.nquad + iq];
     double tx, ty;
     mass_flux_weights(L, k, tx, ty);
-    dvdt += d.us_new[pn] * tx + d.vs_new[pn] * ty;
+    dvdt += d.us_new[pn[k]] * tx + d.vs_new[pn[k]] * ty;
   }
   double xp[9][2];
   node_xy(L, xp);
@@ -749,20 +766,18 @@ __host__ __device__ void f_dt_quad(const Dev &d, int iq, double &dtcfl, double &
                       sqrt((b[0] - c[0]) * (b[0] - c[0]) + (b[1] - c[1]) * (b[1] - c[1]));
     if (k == 0 || dl < dlen) dlen = dl;
   }
-  const size_t nc = d.ncell;
-  const double rhomc = d.Us[0 * nc + e];
-  const double uctr = d.Us[6 * nc + e], vctr = d.Us[12 * nc + e], ectr = d.Us[18 * nc + e];
   const double rhoct = 1.0 / rhomc;
   const double pctr = fmax(eps, (g - 1.0) * rhoct * (ectr - 0.5 * (uctr * uctr + vctr * vctr)));
   const double sdctr = sqrt(fmax(eps, g * pctr / rhoct));
   dtcfl = dlen / sdctr;
-  dtvol = d.vol[e] / fabs(dvdt);
+  dtvol = vol / fabs(dvdt);
 }
 
 // Node motion of stage 1, whose dt needs the node velocities first
 __device__ void f_nodes(const Dev &d, int p, double alfa) {
   if (p >= d.npoin) return;
   const int done = d.sc_dev->done;
+  await_previous();  // the time step
   const double dt = d.sc_dev->dtfix;
   const double un = d.us_new[p], vn = d.vs_new[p], xn = d.xn[p], yn = d.yn[p], xs = d.xs[p], ys = d.ys[p];
   if (done) return;
@@ -1689,7 +1704,10 @@ __host__ __device__ void a_centre(const Dev &d, const Adj &a, int p) {
 
 #include "lag2d_tiles.cuh"
 
-__global__ void __launch_bounds__(128, 8) k_persson2(Dev d) { f_persson(d, blockIdx.x * blockDim.x + threadIdx.x); }
+__global__ void __launch_bounds__(128, 8) k_persson2(Dev d) {
+  await_previous();
+  f_persson(d, blockIdx.x * blockDim.x + threadIdx.x);
+}
 __global__ void __launch_bounds__(128, LAG2D_CCORR_MINB) k_corner2_corr(Dev d) {
   f_corner_corr(d, blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -1698,9 +1716,10 @@ template <bool MOVE, int NR>
 __global__ void __launch_bounds__(256) k_node2(Dev d, double alfa) {
   f_node<MOVE, NR>(d, blockIdx.x * blockDim.x + threadIdx.x, alfa);
 }
+template <bool AHEAD>
 __global__ void __launch_bounds__(kRhsBlock, LAG2D_RHS_MINB) k_rhs3(Dev d, int fuse, double alfa) {
   extern __shared__ double rhs_stage[];
-  f_rhs3(d, blockIdx.x * blockDim.x + threadIdx.x, fuse, alfa, rhs_stage + threadIdx.x);
+  f_rhs3<AHEAD>(d, blockIdx.x * blockDim.x + threadIdx.x, fuse, alfa, rhs_stage + threadIdx.x);
 }
 // Block minimum of two values (256 threads); the result is in thread 0
 __device__ __forceinline__ void block_min2(double &a, double &b) {
@@ -1729,9 +1748,9 @@ __device__ __forceinline__ void block_min2(double &a, double &b) {
 // (1024 x 1024: 76 us, as the two launches it replaces; 97 x 61: 12.2 -> 9.9 us.)
 __global__ void __launch_bounds__(256) k_dt2(Dev d, int ndt, int itime) {
   __shared__ int last;
-  if (d.sc_dev->done) return;
   double a, b;
   f_dt_quad(d, blockIdx.x * blockDim.x + threadIdx.x, a, b);
+  if (d.sc_dev->done) return;
   block_min2(a, b);
   if (threadIdx.x == 0) {
     d.dtpart[2 * blockIdx.x] = a;
@@ -1755,7 +1774,9 @@ __global__ void __launch_bounds__(256) k_dt2(Dev d, int ndt, int itime) {
     dt_apply(d, a, b, ndt);
   }
 }
-__global__ void k_nodes2(Dev d, double alfa) { f_nodes(d, blockIdx.x * blockDim.x + threadIdx.x, alfa); }
+__global__ void k_nodes2(Dev d, double alfa) {
+  f_nodes(d, blockIdx.x * blockDim.x + threadIdx.x, alfa);
+}
 __global__ void k_geom2(Dev d, int fix) { f_geom(d, blockIdx.x * blockDim.x + threadIdx.x, fix); }
 __global__ void k_init_wmom(Dev d) { f_init_wmom(d, blockIdx.x * blockDim.x + threadIdx.x); }
 
@@ -1824,7 +1845,9 @@ void launch_adjoint_stage(const Dev &d, const void *adj, cudaStream_t st, double
 int adjoint_stage_launches(const Dev &d) { return d.ntria > 0 ? 10 : 8; }
 
 
-void launch_fast_persson(const Dev &d, cudaStream_t st) { fast::k_persson2<<<fast::nb(d.nquad, 128), 128, 0, st>>>(d); }
+static bool behind(const Dev &d) { return d.nquad <= kBehindMax; }
+
+void launch_fast_persson(const Dev &d, cudaStream_t st) { launch_behind(behind(d), fast::k_persson2, fast::nb(d.nquad, 128), 128, 0, st, d); }
 void launch_fast_corr(const Dev &d, cudaStream_t st) {
   fast::k_corner2_corr<<<fast::nb(d.nquad, 128), 128, 0, st>>>(d);
 }
@@ -1834,50 +1857,56 @@ void launch_fast_corr(const Dev &d, cudaStream_t st) {
 // Faces, us a step with one thread and with four lanes: 16 x 16 88 / 73, 64 x 64
 // 98 / 82, 128 x 128 110 / 100, 256 x 256 206 / 204, 512 x 512 704 / 696,
 // 1024 x 1024 2531 / 2566.
-constexpr int kFaces4Max = 512 * 512;
+constexpr int kFaces4Max = 131072;
 // RHS (255 registers either way): 16 x 16 73 / 69, 64 x 64 82 / 77, 128 x 128
 // 100 / 102, 256 x 256 204 / 236, so one wave of its blocks on 148 SMs.
 constexpr int kRhs4Max = 148 * 4 * (fast::kRhs4Block / 4);
 void launch_fast_faces(const Dev &d, cudaStream_t st) {
   constexpr int smem = fast::kFaceRows * fast::kFaceBlock * sizeof(double);
   if (d.nquad <= kFaces4Max) {
-    fast::k_faces4<<<fast::nb(4 * d.nquad, fast::kFace4Block), fast::kFace4Block, 0, st>>>(d);
+    launch_behind(behind(d), fast::k_faces4, fast::nb(4 * d.nquad, fast::kFace4Block), fast::kFace4Block, 0, st, d);
     return;
   }
-  fast::k_faces<<<fast::nb(d.nquad, fast::kFaceBlock), fast::kFaceBlock, smem, st>>>(d);
+  launch_behind(behind(d), fast::k_faces, fast::nb(d.nquad, fast::kFaceBlock), fast::kFaceBlock, smem, st, d);
 }
 void launch_fast_src(const Dev &d, cudaStream_t st) { fast::k_tgv_src2<<<fast::nb(d.nquad, 128), 128, 0, st>>>(d); }
 void launch_fast_node(const Dev &d, cudaStream_t st, int move, double alfa) {
   const int g = fast::nb(d.npoin, 256);
   if (d.nrow == 3) {
-    if (move) fast::k_node2<true, 3><<<g, 256, 0, st>>>(d, alfa);
-    else fast::k_node2<false, 3><<<g, 256, 0, st>>>(d, alfa);
+    if (move) launch_behind(behind(d), fast::k_node2<true, 3>, g, 256, 0, st, d, alfa);
+    else launch_behind(behind(d), fast::k_node2<false, 3>, g, 256, 0, st, d, alfa);
   } else {
-    if (move) fast::k_node2<true, 5><<<g, 256, 0, st>>>(d, alfa);
-    else fast::k_node2<false, 5><<<g, 256, 0, st>>>(d, alfa);
+    if (move) launch_behind(behind(d), fast::k_node2<true, 5>, g, 256, 0, st, d, alfa);
+    else launch_behind(behind(d), fast::k_node2<false, 5>, g, 256, 0, st, d, alfa);
   }
 }
 void launch_fast_rhs(const Dev &d, cudaStream_t st, int fuse, double alfa) {
   constexpr int smem = fast::kRhsStage * fast::kRhsBlock * sizeof(double);
   if (d.nquad <= kRhs4Max) {
-    fast::k_rhs4<<<fast::nb(4 * d.nquad, fast::kRhs4Block), fast::kRhs4Block, 0, st>>>(d, fuse, alfa);
+    launch_behind(behind(d), fast::k_rhs4, fast::nb(4 * d.nquad, fast::kRhs4Block), fast::kRhs4Block, 0, st, d, fuse, alfa);
     return;
   }
-  fast::k_rhs3<<<fast::nb(d.nquad, fast::kRhsBlock), fast::kRhsBlock, smem, st>>>(d, fuse, alfa);
+  if (behind(d))
+    launch_behind(true, fast::k_rhs3<true>, fast::nb(d.nquad, fast::kRhsBlock), fast::kRhsBlock, smem, st, d, fuse, alfa);
+  else
+    fast::k_rhs3<false><<<fast::nb(d.nquad, fast::kRhsBlock), fast::kRhsBlock, smem, st>>>(d, fuse, alfa);
 }
 // shared-memory limits of the kernels above 48 KB, on the current device
 cudaError_t set_fast_limits() {
   constexpr int smem = fast::kRhsStage * fast::kRhsBlock * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(fast::k_rhs3, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(fast::k_rhs3, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  cudaError_t e = cudaSuccess;
+  for (auto k : {fast::k_rhs3<true>, fast::k_rhs3<false>}) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  }
   if (e == cudaSuccess) e = cudaFuncSetAttribute(fast::k_faces, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   return e;
 }
 void launch_fast_dt(const Dev &d, cudaStream_t st, int ndt, int itime) {
-  fast::k_dt2<<<fast::nb(d.nquad, 256), 256, 0, st>>>(d, ndt, itime);
+  launch_behind(behind(d), fast::k_dt2, fast::nb(d.nquad, 256), 256, 0, st, d, ndt, itime);
 }
 void launch_fast_nodes(const Dev &d, cudaStream_t st, double alfa) {
-  fast::k_nodes2<<<fast::nb(d.npoin, 256), 256, 0, st>>>(d, alfa);
+  launch_behind(behind(d), fast::k_nodes2, fast::nb(d.npoin, 256), 256, 0, st, d, alfa);
 }
 void launch_fast_geom(const Dev &d, cudaStream_t st, int fix) { fast::k_geom2<<<fast::nb(d.nquad, 256), 256, 0, st>>>(d, fix); }
 void launch_init_wmom(const Dev &d, cudaStream_t st) { fast::k_init_wmom<<<fast::nb(d.nquad, 128), 128, 0, st>>>(d); }

@@ -15,6 +15,7 @@
 // Each kernel cites the reference routine it replaces (srccurv-lag/...).
 // Arithmetic keeps the reference's expression order so that a build with
 // --fmad=false reproduces the CPU restatement bit for bit.
+#include "lag2d_launch.cuh"
 #include <cuda_runtime.h>
 #include <math.h>
 #include "lag2d_device.cuh"
@@ -1529,6 +1530,7 @@ __global__ void k_weno_gather(Dev d, double *lamU, double *lamUn, int fold, cons
 }
 
 __global__ void __launch_bounds__(kWenoThreads) k_weno_block(Dev d, int fixcorr) {
+  await_previous();
   extern __shared__ __align__(16) unsigned char wsm[];
   WenoShared &S = *reinterpret_cast<WenoShared *>(wsm);
   if (stopped(d)) return;
@@ -2143,7 +2145,10 @@ __host__ __device__ void b_step_end(const Dev &d, int check_done) {
   if (S->done) return;
   if (check_done && fabs(S->tacru - d.tend) / d.tend <= 1e-11) S->done = 1;
 }
-__global__ void k_step_end(Dev d, int check_done) { b_step_end(d, check_done); }
+__global__ void k_step_end(Dev d, int check_done) {
+  await_previous();
+  b_step_end(d, check_done);
+}
 
 __global__ void k_reset_count(Dev d) {
   *d.wcount = 0;
@@ -3653,7 +3658,7 @@ void launch_weno(const Dev &d, cudaStream_t st) { k_weno<<<nblk(d.nquad, 64), 64
 // one block per troubled quad, a grid of at most 3 blocks per SM looping over the list
 static int weno_grid(const Dev &d) { return d.nquad < 444 ? (d.nquad > 0 ? d.nquad : 1) : 444; }
 void launch_weno_block(const Dev &d, cudaStream_t st, int fixcorr) {
-  k_weno_block<<<weno_grid(d), kWenoThreads, sizeof(WenoShared), st>>>(d, fixcorr);
+  launch_behind(d.nquad <= kBehindMax, k_weno_block, weno_grid(d), kWenoThreads, sizeof(WenoShared), st, d, fixcorr);
 }
 void launch_weno_linear(const Dev &d, cudaStream_t st, int mode, const double *v, double *out, double *wbuf,
                         int *wslot, int cap, int *overflow) {
@@ -3699,7 +3704,7 @@ int launch_energy_seed(const Dev &d, cudaStream_t st, double *lU, double *part) 
 }
 void launch_copyback(const Dev &d, cudaStream_t st) { k_copyback<<<1184, 256, 0, st>>>(d); }
 void launch_step_begin(const Dev &d, cudaStream_t st, int itime) { k_step_begin<<<1, 1, 0, st>>>(d, itime); }
-void launch_step_end(const Dev &d, cudaStream_t st, int check) { k_step_end<<<1, 1, 0, st>>>(d, check); }
+void launch_step_end(const Dev &d, cudaStream_t st, int check) { launch_behind(d.nquad <= kBehindMax, k_step_end, 1, 1, 0, st, d, check); }
 void launch_init_msub(const Dev &d, cudaStream_t st) {
   k_init_msub<<<nblk(d.nquad, 128), 128, 0, st>>>(d);
 }

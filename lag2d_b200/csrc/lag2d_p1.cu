@@ -41,6 +41,7 @@
 //                                 sigma.n A x, y) of corner iv, face f
 //   lim[k*ncell + e]              aflim(1), aflim(4), aflim(5), afvec(1,1),
 //                                 afvec(1,2), afvec(2,1), afvec(2,2)
+#include "lag2d_launch.cuh"
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -1808,22 +1809,24 @@ static void enqueue_rhs(Solver *s, int fuse, double alfa, int stage) {
 }
 
 // the same passes of the optimised stage
+static bool behind(const Dev1 &d) { return d.nquad <= kBehindMax; }
 template <int GEO>
 static void fast_cell(Solver *s, const Dev1 &d, int stage, int itime) {
   launch(s, "cell", [&] {
-    k1f_cell<GEO><<<nb(4 * d.nquad, kCellThreads), kCellThreads, 0, s->st>>>(d, stage, itime);
+    launch_behind(behind(d), k1f_cell<GEO>, nb(4 * d.nquad, kCellThreads), kCellThreads, 0, s->st, d, stage, itime);
   });
 }
 template <int GEO>
 static void fast_node(Solver *s, const Dev1 &d, bool move, double alfa) {
   launch(s, "node", [&] {
-    if (move) k1f_node<GEO, true><<<nb(d.npoin, 64), 64, 0, s->st>>>(d, alfa);
-    else k1f_node<GEO, false><<<nb(d.npoin, 64), 64, 0, s->st>>>(d, alfa);
+    launch_behind(behind(d), move ? k1f_node<GEO, true> : k1f_node<GEO, false>, nb(d.npoin, 64), 64, 0, s->st, d, alfa);
   });
 }
 template <int GEO>
 static void fast_rhs(Solver *s, const Dev1 &d, int fuse, double alfa, int last) {
-  launch(s, "rhs", [&] { k1f_rhs<GEO><<<nb(d.nquad, kRhsThreads), kRhsThreads, 0, s->st>>>(d, fuse, alfa, last); });
+  launch(s, "rhs", [&] {
+    launch_behind(behind(d), k1f_rhs<GEO>, nb(d.nquad, kRhsThreads), kRhsThreads, 0, s->st, d, fuse, alfa, last);
+  });
 }
 // Plane meshes of this many cells and more keep the order of operations of the
 // kernels above (their FAST form) instead of the closed-form moments.  The
@@ -1890,9 +1893,9 @@ static void enqueue_step_fast(Solver *s, int itime) {
       fast_node<GEO>(s, d, istag > 1, alfa);
     }
     if (istag == 1) {
-      launch(s, "dt", [&] { k1f_dt<GEO><<<nb(d.nquad, 256), 256, 0, s->st>>>(d, s->cfg.ndt, itime); });
+      launch(s, "dt", [&] { launch_behind(behind(d), k1f_dt<GEO>, nb(d.nquad, 256), 256, 0, s->st, d, s->cfg.ndt, itime); });
       after(s1, s->st);
-      launch(s, "nodes", [&] { k1f_move<<<nb(d.npoin, 64), 64, 0, s1>>>(d, alfa); });
+      launch(s, "nodes", [&] { launch_behind(behind(d), k1f_move, nb(d.npoin, 64), 64, 0, s1, d, alfa); });
     }
     if (last) {
       after(s1, s->st);

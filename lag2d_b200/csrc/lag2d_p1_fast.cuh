@@ -186,8 +186,14 @@ __global__ void __launch_bounds__(kCellThreads) k1f_cell(Dev1 d, int stage, int 
   const int e = live ? t >> 2 : d.nquad - 1;  // lanes past the end repeat the last cell and store nothing
   const size_t nc = d.ncell, np = d.npoin;
   const Scalars *S = d.sc_dev;
-  const int done = S->done, now = S->itime;
   const int p = d.ipq[iv * nc + e];
+  const int b0 = d.esuv_ptr[p], b1 = d.esuv_ptr[p + 1];
+  const int cls = d.ncase != 1 ? d.wall[p] : 0;
+  int ce[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) ce[j] = b0 + j < b1 ? d.esuv[b0 + j] : e;
+  await_previous();  // the RHS pass before, in a step's first stage its exit test
+  const int done = S->done, now = S->itime;
   double u[4][ND];
 #pragma unroll
   for (int q = 0; q < 4; q++)
@@ -195,12 +201,7 @@ __global__ void __launch_bounds__(kCellThreads) k1f_cell(Dev1 d, int stage, int 
     for (int k = 0; k < ND; k++) u[q][k] = d.Us[(q * ND + k) * nc + e];
   const double pctr_s = d.pbar[e];
   double rc = d.rc[e], sc = d.sc[e];
-  const int b0 = d.esuv_ptr[p], b1 = d.esuv_ptr[p + 1];
   const double x = d.xs[p], y = d.ys[p], us0 = d.us[p], vs0 = d.vs[p];
-  const int cls = d.ncase != 1 ? d.wall[p] : 0;
-  int ce[4];
-#pragma unroll
-  for (int j = 0; j < 4; j++) ce[j] = b0 + j < b1 ? d.esuv[b0 + j] : e;
   // the averages around the vertex; entries past the list repeat the cell itself
   double uj[4], vj[4], mx[5], mn[5];
 #pragma unroll
@@ -386,6 +387,7 @@ __global__ void __launch_bounds__(64) k1f_node(Dev1 d, double alfa) {
   int c[4];
 #pragma unroll
   for (int j = 0; j < 4; j++) c[j] = b + j < en ? d.ncor[b + j] : 0;
+  await_previous();  // the cell pass: corner coefficients
   if (done) return;
   NodeSum n{0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
@@ -450,6 +452,7 @@ __global__ void __launch_bounds__(64) k1f_node(Dev1 d, double alfa) {
 // motion of stage 1
 __global__ void __launch_bounds__(64) k1f_move(Dev1 d, double alfa) {
   const int p = blockIdx.x * 64 + threadIdx.x;
+  await_previous();
   if (p >= d.npoin) return;
   const int done = d.sc_dev->done;
   const double dt = d.sc_dev->dtfix, oma = 1.0 - alfa;
@@ -487,19 +490,22 @@ template <int GEO>
 __global__ void __launch_bounds__(256) k1f_dt(Dev1 d, int ndt, int itime) {
   __shared__ int last;
   const int e = blockIdx.x * 256 + threadIdx.x;
-  if (d.sc_dev->done) return;
   const size_t nc = d.ncell;
+  int ip[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) ip[k] = e < d.nquad ? d.ipq[k * nc + e] : 0;
+  await_previous();  // the node pass: u*
+  if (d.sc_dev->done) return;
   double dtcfl = 1e10, dtvol = 1e10;
   if (e < d.nquad) {
     const double eps = 1.0e-6, g = d.gamlg;
     double x[4], y[4], us[4], vs[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const int p = d.ipq[k * nc + e];
-      x[k] = d.xn[p];
-      y[k] = d.yn[p];
-      us[k] = d.us[p];
-      vs[k] = d.vs[p];
+      x[k] = d.xn[ip[k]];
+      y[k] = d.yn[ip[k]];
+      us[k] = d.us[ip[k]];
+      vs[k] = d.vs[ip[k]];
     }
     const double tau = d.Us[e], uc = d.Us[3 * nc + e], vc = d.Us[6 * nc + e], ec = d.Us[9 * nc + e];
     const Bilin B = bilin(x, y);
@@ -581,26 +587,32 @@ template <int GEO>
 __global__ void __launch_bounds__(kRhsThreads) k1f_rhs(Dev1 d, int fuse, double alfa, int last_stage) {
   const int e = blockIdx.x * kRhsThreads + threadIdx.x;
   const size_t nc = d.ncell;
-  const int done = d.sc_dev->done;
+  const int done = d.sc_dev->done, el = e < d.nquad ? e : d.nquad - 1;
+  // read ahead of the node pass, in stage 1 the time step
+  int ip[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) ip[k] = d.ipq[k * nc + el];
+  double u[4][ND];
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int k = 0; k < ND; k++) u[q][k] = d.Us[(q * ND + k) * nc + el];
+  const double rc = d.rc[el], sc = d.sc[el];
+  const double af1 = d.lim[0 * nc + el], af4 = d.lim[1 * nc + el], af5 = d.lim[2 * nc + el];
+  const double v11 = d.lim[3 * nc + el], v12 = d.lim[4 * nc + el], v22 = d.lim[6 * nc + el];
+  double x[4], y[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    x[k] = d.xs[ip[k]];
+    y[k] = d.ys[ip[k]];
+  }
+  await_previous();
   if (e < d.nquad && !done) {
     const double g = d.gamlg, epsd = 1.0e-6;
     const int md = d.mdegr;
-    int ip[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) ip[k] = d.ipq[k * nc + e];
-    double u[4][ND];
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-#pragma unroll
-      for (int k = 0; k < ND; k++) u[q][k] = d.Us[(q * ND + k) * nc + e];
-    const double rc = d.rc[e], sc = d.sc[e];
-    const double af1 = d.lim[0 * nc + e], af4 = d.lim[1 * nc + e], af5 = d.lim[2 * nc + e];
-    const double v11 = d.lim[3 * nc + e], v12 = d.lim[4 * nc + e], v22 = d.lim[6 * nc + e];
-    double x[4], y[4], us[4], vs[4];
+    double us[4], vs[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      x[k] = d.xs[ip[k]];
-      y[k] = d.ys[ip[k]];
       us[k] = d.us[ip[k]];
       vs[k] = d.vs[ip[k]];
     }

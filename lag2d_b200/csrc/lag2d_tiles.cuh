@@ -73,6 +73,7 @@ __device__ void f_faces(const Dev &d, int iq_in, double *col) {
   const int iq = iq_in, e = iq + d.ntria;
   const size_t nq = d.nquad;
   // all loads in flight before the first use
+  await_previous();
   const int done = d.sc_dev->done;
   int pn[9];
 #pragma unroll
@@ -207,11 +208,12 @@ __global__ void __launch_bounds__(kFace4Block, LAG2D_FACES4_MINB) k_faces4(Dev d
   double u[4][6];
   load_u(d, d.Us, e, u);
   const CellGeo G{d.rc[e], d.sc[e], d.g19[e], d.g20[e], d.g21[e]};
-  const double corr0 = d.corr[v * nq + iq];
-  const int flag = d.flag[e];
   const double cx = d.xs[pc], cy = d.ys[pc], cu = d.us[pc], cv = d.vs[pc];
   const double ex = d.xs[pe], ey = d.ys[pe], eu = d.us[pe], ev = d.vs[pe];
   const double mx = d.xs[pm], my = d.ys[pm], mu = d.us[pm], mv = d.vs[pm];
+  await_previous();  // WENO: corrections, flags, moments
+  const double corr0 = d.corr[v * nq + iq];
+  const int flag = d.flag[e];
   if (flag == 2) {
     // the moments WENO replaced (they are not committed to the stage state)
 #pragma unroll
@@ -329,7 +331,6 @@ __global__ void __launch_bounds__(kRhs4Block, LAG2D_RHS4_MINB) k_rhs4(Dev d, int
   const size_t nq = d.nquad, nc = d.ncell;
   // all loads in flight before the first use
   const int done = d.sc_dev->done;
-  const double dt = d.sc_dev->dtfix;
   int pn[9];
 #pragma unroll
   for (int k = 0; k < 9; k++) pn[k] = d.ipq[k * nq + iq];
@@ -354,7 +355,6 @@ __global__ void __launch_bounds__(kRhs4Block, LAG2D_RHS4_MINB) k_rhs4(Dev d, int
     for (int k = 0; k < 6; k++) stage8(&col[40 + k][0], d.src + k * nq + iq);
   __pipeline_commit();
   const int flag = d.flag[e];
-  const double uc = d.us_new[pc], vc = d.vs_new[pc], ue = d.us_new[pe], ve = d.vs_new[pe];
   Loaded L;
   {
     const int A[9] = {0, 2, 2, 0, 1, 2, 1, 0, 1}, B[9] = {0, 0, 2, 2, 0, 1, 2, 1, 1};
@@ -364,6 +364,9 @@ __global__ void __launch_bounds__(kRhs4Block, LAG2D_RHS4_MINB) k_rhs4(Dev d, int
       L.Y[A[k]][B[k]] = d.ys[pn[k]];
     }
   }
+  await_previous();  // the node pass, in stage 1 the time step
+  const double dt = d.sc_dev->dtfix;
+  const double uc = d.us_new[pc], vc = d.vs_new[pc], ue = d.us_new[pe], ve = d.vs_new[pe];
   if (flag == 2) {
     // the moments WENO replaced (they are not committed to the stage state)
 #pragma unroll
