@@ -1893,7 +1893,7 @@ static void enqueue_step_fast(Solver *s, int itime) {
       fast_node<GEO>(s, d, istag > 1, alfa);
     }
     if (istag == 1) {
-      launch(s, "dt", [&] { launch_behind(behind(d), k1f_dt<GEO>, nb(d.nquad, 256), 256, 0, s->st, d, s->cfg.ndt, itime); });
+      launch(s, "dt", [&] { launch_behind(behind(d), behind(d) ? k1f_dt<GEO, true> : k1f_dt<GEO, false>, nb(d.nquad, 256), 256, 0, s->st, d, s->cfg.ndt, itime); });
       after(s1, s->st);
       launch(s, "nodes", [&] { launch_behind(behind(d), k1f_move, nb(d.npoin, 64), 64, 0, s1, d, alfa); });
     }

@@ -486,28 +486,32 @@ __device__ __forceinline__ void block_min2(double &a, double &b) {
     }
   __syncthreads();
 }
-template <int GEO>
+template <int GEO, bool AHEAD>
 __global__ void __launch_bounds__(256) k1f_dt(Dev1 d, int ndt, int itime) {
   __shared__ int last;
   const int e = blockIdx.x * 256 + threadIdx.x;
   const size_t nc = d.ncell;
+  if (!AHEAD) await_previous();
+  const int el = e < d.nquad ? e : d.nquad - 1;
   int ip[4];
+  double x[4], y[4], us[4], vs[4];
 #pragma unroll
-  for (int k = 0; k < 4; k++) ip[k] = e < d.nquad ? d.ipq[k * nc + e] : 0;
-  await_previous();  // the node pass: u*
+  for (int k = 0; k < 4; k++) {
+    ip[k] = d.ipq[k * nc + el];
+    x[k] = d.xn[ip[k]];
+    y[k] = d.yn[ip[k]];
+  }
+  const double tau = d.Us[el], uc = d.Us[3 * nc + el], vc = d.Us[6 * nc + el], ec = d.Us[9 * nc + el];
+  if (AHEAD) await_previous();  // the node pass: u*
   if (d.sc_dev->done) return;
   double dtcfl = 1e10, dtvol = 1e10;
   if (e < d.nquad) {
     const double eps = 1.0e-6, g = d.gamlg;
-    double x[4], y[4], us[4], vs[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      x[k] = d.xn[ip[k]];
-      y[k] = d.yn[ip[k]];
       us[k] = d.us[ip[k]];
       vs[k] = d.vs[ip[k]];
     }
-    const double tau = d.Us[e], uc = d.Us[3 * nc + e], vc = d.Us[6 * nc + e], ec = d.Us[9 * nc + e];
     const Bilin B = bilin(x, y);
     // the cell-average volume change: the face integral's moment 0 (and the
     // area-weighted form's source); in the plane branch by k1_rhs's expressions
@@ -588,7 +592,7 @@ __global__ void __launch_bounds__(kRhsThreads) k1f_rhs(Dev1 d, int fuse, double 
   const int e = blockIdx.x * kRhsThreads + threadIdx.x;
   const size_t nc = d.ncell;
   const int done = d.sc_dev->done, el = e < d.nquad ? e : d.nquad - 1;
-  // read ahead of the node pass, in stage 1 the time step
+  // ahead of the node pass (in stage 1 of the time step): all but the face integral
   int ip[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) ip[k] = d.ipq[k * nc + el];
@@ -606,17 +610,67 @@ __global__ void __launch_bounds__(kRhsThreads) k1f_rhs(Dev1 d, int fuse, double 
     x[k] = d.xs[ip[k]];
     y[k] = d.ys[ip[k]];
   }
+  const Bilin B = bilin(x, y);
+  const double g = d.gamlg, epsd = 1.0e-6;
+  const int md = d.mdegr;
+  // moments of the limited pressure over the 25 points: M without, Q (nrz = 1)
+  // with the radius weight
+  const double pctr = pressure(g, u[0][0], u[1][0], u[2][0], u[3][0], epsd);
+  double M00 = 0.0, M10 = 0.0, M01 = 0.0, M20 = 0.0, M11 = 0.0, M02 = 0.0;
+  double Q00 = 0.0, Q10 = 0.0, Q01 = 0.0, Q20 = 0.0, Q11 = 0.0, Q02 = 0.0;
+  double c0[4], c1[4], c2[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    c1[q] = md > 1 ? u[q][1] : 0.0;
+    c2[q] = md > 2 ? u[q][2] : 0.0;
+    c0[q] = u[q][0] - c1[q] * rc - c2[q] * sc;
+  }
+#pragma unroll 1
+  for (int i = 0; i < 5; i++) {
+    const double r = g5x(i), wi = g5wt(i);
+    double a[4], t[5], pre[5];
+#pragma unroll
+    for (int q = 0; q < 4; q++) a[q] = c0[q] + c1[q] * r;
+#pragma unroll
+    for (int j = 0; j < 5; j++) {
+      t[j] = a[0] + c2[0] * g5x(j);
+      pre[j] = j == 0 ? t[0] : pre[j - 1] * t[j];
+    }
+    double inv = 1.0 / pre[4], m0 = 0.0, m1 = 0.0, m2 = 0.0, q0 = 0.0, q1 = 0.0, q2 = 0.0;
+    const double yr = B.yc + B.f1 * r, ysl = B.f2 + B.f3 * r;
+#pragma unroll
+    for (int j = 4; j >= 0; j--) {
+      const double rho = j > 0 ? inv * pre[j > 0 ? j - 1 : 0] : inv;
+      inv *= t[j];
+      const double s = g5x(j);
+      const double uu = a[1] + c2[1] * s, vv = a[2] + c2[2] * s, ee = a[3] + c2[3] * s;
+      const double p = pctr + af4 * ((g - 1.0) * rho * (ee - 0.5 * (uu * uu + vv * vv)) - pctr);
+      const double m = g5wt(j) * p;
+      m0 += m;
+      m1 += m * s;
+      m2 += m * s * s;
+      if (GEO == 1) {
+        const double q = m * (yr + ysl * s);
+        q0 += q;
+        q1 += q * s;
+        q2 += q * s * s;
+      }
+    }
+    m0 *= wi; m1 *= wi; m2 *= wi;
+    M00 += m0; M10 += r * m0; M20 += r * r * m0; M01 += m1; M11 += r * m1; M02 += m2;
+    if (GEO == 1) {
+      q0 *= wi; q1 *= wi; q2 *= wi;
+      Q00 += q0; Q10 += r * q0; Q20 += r * r * q0; Q01 += q1; Q11 += r * q1; Q02 += q2;
+    }
+  }
   await_previous();
   if (e < d.nquad && !done) {
-    const double g = d.gamlg, epsd = 1.0e-6;
-    const int md = d.mdegr;
     double us[4], vs[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       us[k] = d.us[ip[k]];
       vs[k] = d.vs[ip[k]];
     }
-    const Bilin B = bilin(x, y);
     // face integral: per corner the two edges with their own and other basis
     double R[ND][4];
 #pragma unroll
@@ -663,56 +717,6 @@ __global__ void __launch_bounds__(kRhsThreads) k1f_rhs(Dev1 d, int fuse, double 
           R[0][0] += w * tw; R[0][1] += w * f0; R[0][2] += w * f1; R[0][3] += w * fe;
           add(ob * br + nn * brn, ob * bs + nn * bsn, tw, f0, f1, fe);
         }
-      }
-    }
-    // moments of the limited pressure over the 25 points: M without, Q (nrz = 1)
-    // with the radius weight
-    const double pctr = pressure(g, u[0][0], u[1][0], u[2][0], u[3][0], epsd);
-    double M00 = 0.0, M10 = 0.0, M01 = 0.0, M20 = 0.0, M11 = 0.0, M02 = 0.0;
-    double Q00 = 0.0, Q10 = 0.0, Q01 = 0.0, Q20 = 0.0, Q11 = 0.0, Q02 = 0.0;
-    double c0[4], c1[4], c2[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      c1[q] = md > 1 ? u[q][1] : 0.0;
-      c2[q] = md > 2 ? u[q][2] : 0.0;
-      c0[q] = u[q][0] - c1[q] * rc - c2[q] * sc;
-    }
-#pragma unroll 1
-    for (int i = 0; i < 5; i++) {
-      const double r = g5x(i), wi = g5wt(i);
-      double a[4], t[5], pre[5];
-#pragma unroll
-      for (int q = 0; q < 4; q++) a[q] = c0[q] + c1[q] * r;
-#pragma unroll
-      for (int j = 0; j < 5; j++) {
-        t[j] = a[0] + c2[0] * g5x(j);
-        pre[j] = j == 0 ? t[0] : pre[j - 1] * t[j];
-      }
-      double inv = 1.0 / pre[4], m0 = 0.0, m1 = 0.0, m2 = 0.0, q0 = 0.0, q1 = 0.0, q2 = 0.0;
-      const double yr = B.yc + B.f1 * r, ysl = B.f2 + B.f3 * r;
-#pragma unroll
-      for (int j = 4; j >= 0; j--) {
-        const double rho = j > 0 ? inv * pre[j > 0 ? j - 1 : 0] : inv;
-        inv *= t[j];
-        const double s = g5x(j);
-        const double uu = a[1] + c2[1] * s, vv = a[2] + c2[2] * s, ee = a[3] + c2[3] * s;
-        const double p = pctr + af4 * ((g - 1.0) * rho * (ee - 0.5 * (uu * uu + vv * vv)) - pctr);
-        const double m = g5wt(j) * p;
-        m0 += m;
-        m1 += m * s;
-        m2 += m * s * s;
-        if (GEO == 1) {
-          const double q = m * (yr + ysl * s);
-          q0 += q;
-          q1 += q * s;
-          q2 += q * s * s;
-        }
-      }
-      m0 *= wi; m1 *= wi; m2 *= wi;
-      M00 += m0; M10 += r * m0; M20 += r * r * m0; M01 += m1; M11 += r * m1; M02 += m2;
-      if (GEO == 1) {
-        q0 *= wi; q1 *= wi; q2 *= wi;
-        Q00 += q0; Q10 += r * q0; Q20 += r * r * q0; Q01 += q1; Q11 += r * q1; Q02 += q2;
       }
     }
     // moments of the weight alone (closed form): 1, or y in nrz = 1

@@ -364,9 +364,6 @@ __global__ void __launch_bounds__(kRhs4Block, LAG2D_RHS4_MINB) k_rhs4(Dev d, int
       L.Y[A[k]][B[k]] = d.ys[pn[k]];
     }
   }
-  await_previous();  // the node pass, in stage 1 the time step
-  const double dt = d.sc_dev->dtfix;
-  const double uc = d.us_new[pc], vc = d.vs_new[pc], ue = d.us_new[pe], ve = d.vs_new[pe];
   if (flag == 2) {
     // the moments WENO replaced (they are not committed to the stage state)
 #pragma unroll
@@ -374,34 +371,12 @@ __global__ void __launch_bounds__(kRhs4Block, LAG2D_RHS4_MINB) k_rhs4(Dev d, int
 #pragma unroll
       for (int k = 1; k < 6; k++) u[q][k] = d.Uw[(q * 5 + k - 1) * nq + iq];
   }
+  // the volume integral ahead of the wait
   double R[4][6];
-  {
-    // the lane's corner c and edge node e, the corners and edge nodes next to them
-    const double xc = v == 1 || v == 2 ? 1.0 : -1.0, yc = v >= 2 ? 1.0 : -1.0;
-    const double xe = v == 1 ? 1.0 : v == 3 ? -1.0 : 0.0, ye = v == 2 ? 1.0 : v == 0 ? -1.0 : 0.0;
-    const double ax = d.xs[pc], ay = d.ys[pc], bx = d.xs[pe], by = d.ys[pe];
-    const int vn = (v + 1) & 3, vp = (v + 3) & 3;
-    const double nx = lane_get(ax, vn), ny = lane_get(ay, vn), px = lane_get(ax, vp), py = lane_get(ay, vp);
-    const double qx = lane_get(bx, vp), qy = lane_get(by, vp);
-    double tx, ty, fc[4], fe[4];
-    corner_flux(px, py, qx, qy, bx, by, nx, ny, tx, ty);
-    fc[0] = uc * tx + vc * ty;
-    fc[1] = uc * c0 - c1;
-    fc[2] = vc * c0 - c2;
-    fc[3] = uc * fc[1] + vc * fc[2];
-    edge_flux(ax, ay, nx, ny, tx, ty);
-    fe[0] = ue * tx + ve * ty;
-    fe[1] = ue * e0 - e1;
-    fe[2] = ve * e0 - e2;
-    fe[3] = ue * fe[1] + ve * fe[2];
-    double bc[6], be[6];
-    basis_at(G, xc, yc, bc);
-    basis_at(G, xe, ye, be);
 #pragma unroll
-    for (int q = 0; q < 4; q++)
+  for (int q = 0; q < 4; q++)
 #pragma unroll
-      for (int k = 0; k < 6; k++) R[q][k] = fc[q] * bc[k] + fe[q] * be[k];
-  }
+    for (int k = 0; k < 6; k++) R[q][k] = 0.0;
   QuadMap m;
   map_coeffs(L.X, m.a);
   map_coeffs(L.Y, m.b);
@@ -468,6 +443,36 @@ __global__ void __launch_bounds__(kRhs4Block, LAG2D_RHS4_MINB) k_rhs4(Dev d, int
       R[q][4] += wi * (S.B1[q] - G.sc * S.B0[q]);
       R[q][5] += wi * (S.A1[q] - G.sc * S.A0[q]) + wr * S.B0[q];
     }
+  }
+  await_previous();  // the node pass, in stage 1 the time step
+  const double dt = d.sc_dev->dtfix;
+  const double uc = d.us_new[pc], vc = d.vs_new[pc], ue = d.us_new[pe], ve = d.vs_new[pe];
+  {
+    // the lane's corner c and edge node e, the corners and edge nodes next to them
+    const double xc = v == 1 || v == 2 ? 1.0 : -1.0, yc = v >= 2 ? 1.0 : -1.0;
+    const double xe = v == 1 ? 1.0 : v == 3 ? -1.0 : 0.0, ye = v == 2 ? 1.0 : v == 0 ? -1.0 : 0.0;
+    const double ax = d.xs[pc], ay = d.ys[pc], bx = d.xs[pe], by = d.ys[pe];
+    const int vn = (v + 1) & 3, vp = (v + 3) & 3;
+    const double nx = lane_get(ax, vn), ny = lane_get(ay, vn), px = lane_get(ax, vp), py = lane_get(ay, vp);
+    const double qx = lane_get(bx, vp), qy = lane_get(by, vp);
+    double tx, ty, fc[4], fe[4];
+    corner_flux(px, py, qx, qy, bx, by, nx, ny, tx, ty);
+    fc[0] = uc * tx + vc * ty;
+    fc[1] = uc * c0 - c1;
+    fc[2] = vc * c0 - c2;
+    fc[3] = uc * fc[1] + vc * fc[2];
+    edge_flux(ax, ay, nx, ny, tx, ty);
+    fe[0] = ue * tx + ve * ty;
+    fe[1] = ue * e0 - e1;
+    fe[2] = ve * e0 - e2;
+    fe[3] = ue * fe[1] + ve * fe[2];
+    double bc[6], be[6];
+    basis_at(G, xc, yc, bc);
+    basis_at(G, xe, ye, be);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+      for (int k = 0; k < 6; k++) R[q][k] += fc[q] * bc[k] + fe[q] * be[k];
   }
   // lane v keeps equation v
   double T[2][6], Rq[6];
