@@ -54,6 +54,7 @@ def build(verbose: bool = False, force: bool = False) -> list:
                   os.path.join(HERE, "csrc", "lag2d_fast_tables.h"), os.path.join(HERE, "csrc", "lag2d_shape9.cuh"),
                   os.path.join(HERE, "csrc", "lag2d_tiles.cuh"), os.path.join(HERE, "csrc", "lag2d_dt.cuh"),
                   os.path.join(HERE, "csrc", "lag2d_cell.cuh"), os.path.join(HERE, "csrc", "lag2d_launch.cuh"),
+                  os.path.join(HERE, "csrc", "lag2d_reverse.cuh"),
                   os.path.join(HERE, "csrc", "lag2d_p1_fast.cuh"), os.path.join(HERE, "csrc", "lag2d_p1.h"),
                   os.path.join(ROOT, "include", "lag2d.h")]
     newest = max(os.path.getmtime(p) for p in deps)

@@ -492,7 +492,11 @@ __host__ __device__ __forceinline__ void mass_flux_weights(const Loaded &L, int 
 // U^n, which is then copied after the rows: 289.
 constexpr int kRhsBlock = 64;
 constexpr int kRhsStage = 64;
-// the rule of the rolled row loop
+// the rules of the rolled row loops
+__constant__ double cG5[5] = {-0.9061798459386639927976269, -0.5384693101056830910363144, 0.0,
+                              0.5384693101056830910363144, 0.9061798459386639927976269};
+__constant__ double cW5[5] = {0.2369268850561890875142640, 0.4786286704993664680412915, 0.5688888888888888888888889,
+                              0.4786286704993664680412915, 0.2369268850561890875142640};
 __constant__ double cL5[5] = {-1.0, -0.6546536707079771437983, 0.0, 0.6546536707079771437983, 1.0};
 __constant__ double cLw[5] = {0.1, 0.544444444444444444444, 0.7111111111111111111111, 0.544444444444444444444, 0.1};
 constexpr double kMassCorner = 1.0 / 3.0, kMassEdge = 2.0 / 3.0;
@@ -1017,7 +1021,7 @@ __host__ __device__ __forceinline__ void vertex_T(const double *b, int mdegr, co
 // into pbuf and the adjoints of the 4 sub-cell density corrections into
 // lcorr.  Without the det J polynomial, sub-cell areas and masses the
 // corrections' transpose needs, it holds far fewer values across its 32
-// unrolled faces.
+// unrolled faces.  (The FP32-mixed adjoint's; the FP64 one runs k_a_faces4.)
 __host__ __device__ void a_corner_faces(const Dev &d, const Adj &a, int iq) {
   if (iq >= d.nquad) return;
   const int e = iq + d.ntria;
@@ -1702,6 +1706,7 @@ __host__ __device__ void a_centre(const Dev &d, const Adj &a, int p) {
 }
 
 #include "lag2d_tiles.cuh"
+#include "lag2d_reverse.cuh"
 
 __global__ void __launch_bounds__(128, 8) k_persson2(Dev d) {
   await_previous();
@@ -1833,10 +1838,11 @@ void launch_adjoint_stage(const Dev &d, const void *adj, cudaStream_t st, double
   fast::k_a_nodes<<<bp, 256, 0, st>>>(d, a, alfa, dtp, fold);
   fast::k_a_update<<<bc, 256, 0, st>>>(d, a, alfa, dtp, fold_u);
   if (mixed) fast::k_a_rhs<float><<<bq, 128, 0, st>>>(d, a);
-  else fast::k_a_rhs<double><<<bq, 128, 0, st>>>(d, a);
+  else fast::k_a_rhs64<<<fast::nb(d.nquad, fast::kRevBlock), fast::kRevBlock, 0, st>>>(d, a);
   launch_tri_adjoint_rhs(d, a, st);
   fast::k_a_gather_solve<<<bp, 256, 0, st>>>(d, a);
-  fast::k_a_corner_faces<<<bq, 128, 0, st>>>(d, a);
+  if (mixed) fast::k_a_corner_faces<<<bq, 128, 0, st>>>(d, a);
+  else fast::k_a_faces4<<<fast::nb(4 * d.nquad, fast::kRevFaceBlock), fast::kRevFaceBlock, 0, st>>>(d, a);
   if (mixed) fast::k_a_corner_corr<float><<<bq, 128, 0, st>>>(d, a);
   else fast::k_a_corner_corr<double><<<bq, 128, 0, st>>>(d, a);
   launch_tri_adjoint_corner(d, a, st);
