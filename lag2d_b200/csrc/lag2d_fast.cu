@@ -1021,7 +1021,8 @@ __host__ __device__ __forceinline__ void vertex_T(const double *b, int mdegr, co
 // into pbuf and the adjoints of the 4 sub-cell density corrections into
 // lcorr.  Without the det J polynomial, sub-cell areas and masses the
 // corrections' transpose needs, it holds far fewer values across its 32
-// unrolled faces.  (The FP32-mixed adjoint's; the FP64 one runs k_a_faces4.)
+// unrolled faces.  (The FP32-mixed adjoint's; the FP64 one runs k_a_faces4 and
+// k_a_corr64.)
 __host__ __device__ void a_corner_faces(const Dev &d, const Adj &a, int iq) {
   if (iq >= d.nquad) return;
   const int e = iq + d.ntria;
@@ -1844,7 +1845,7 @@ void launch_adjoint_stage(const Dev &d, const void *adj, cudaStream_t st, double
   if (mixed) fast::k_a_corner_faces<<<bq, 128, 0, st>>>(d, a);
   else fast::k_a_faces4<<<fast::nb(4 * d.nquad, fast::kRevFaceBlock), fast::kRevFaceBlock, 0, st>>>(d, a);
   if (mixed) fast::k_a_corner_corr<float><<<bq, 128, 0, st>>>(d, a);
-  else fast::k_a_corner_corr<double><<<bq, 128, 0, st>>>(d, a);
+  else fast::k_a_corr64<<<fast::nb(d.nquad, fast::kRevCorrBlock), fast::kRevCorrBlock, 0, st>>>(d, a);
   launch_tri_adjoint_corner(d, a, st);
   fast::k_a_gather<<<bp, 256, 0, st>>>(d, a, 4);
 }

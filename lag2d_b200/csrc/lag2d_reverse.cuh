@@ -526,3 +526,136 @@ __global__ void __launch_bounds__(kRevFaceBlock, 3) k_a_faces4(Dev d, Adj a) {
   }
   a.lcorr[v * nq + iq] = lcr;
 }
+
+// The transpose of f_corner_corr, corr = cdrho (msub - masel) / area with masel = sum
+// w det J / tau, from lcorr: adds into the tau DOF adjoints and the node contributions.
+// One division per row of five points; both halves of a row share its sums; det J
+// hands its adjoint to the map.  256 x 256: 60 -> 33 us a launch
+// (128 registers, 216 bytes of spills; 4 or 6 blocks of 64 an SM 3% slower a sweep).
+constexpr int kRevCorrBlock = 64;
+__global__ void __launch_bounds__(kRevCorrBlock, 8) k_a_corr64(Dev d, Adj a) {
+  const int iq = blockIdx.x * kRevCorrBlock + threadIdx.x;
+  if (iq >= d.nquad) return;
+  const int e = iq + d.ntria;
+  const size_t nq = d.nquad, nc = d.ncell;
+  double u[6], lm[4], la[4];
+#pragma unroll
+  for (int k = 0; k < 6; k++) u[k] = d.Us[k * nc + e];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    lm[k] = a.lcorr[k * nq + iq];
+    la[k] = -lm[k] * d.corr[k * nq + iq];
+  }
+  const CellGeo G{d.rc[e], d.sc[e], d.g19[e], d.g20[e], d.g21[e]};
+  QuadMap m, l;
+  load_map(d, iq, m);
+  double D[4][4], lD[4][4], lq[6] = {0, 0, 0, 0, 0, 0};
+  map_det(m, D);
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int n = 0; n < 4; n++) lD[i][n] = 0.0;
+  const double b3 = 0.5 * G.rc * G.rc - G.g19, b4 = 0.5 * G.sc * G.sc - G.g20, b5 = G.rc * G.sc - G.g21;
+  const double q0 = u[0] - u[1] * G.rc - u[2] * G.sc + u[3] * b3 + u[4] * b4 + u[5] * b5;
+  const double q1 = u[1] - u[3] * G.rc - u[5] * G.sc, q2 = u[2] - u[4] * G.sc - u[5] * G.rc;
+  const double q3 = 0.5 * u[3], t2 = 0.5 * u[4];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const double sg = h == 0 ? -1.0 : 1.0;
+    const int is[2] = {h == 0 ? 0 : 1, h == 0 ? 3 : 2};  // s in [-1, 0], [0, 1]
+    // the areas
+    double F[4], lF[4], lms[2];
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+      F[n] = D[0][n] + (1.0 / 3.0) * D[2][n] + sg * (0.5 * D[1][n] + 0.25 * D[3][n]);
+    const double ev = F[0] + (1.0 / 3.0) * F[2], od = 0.5 * F[1] + 0.25 * F[3];
+    const double r0 = 1.0 / (ev - od), r1 = 1.0 / (ev + od);
+    const double l0 = la[is[0]] * r0, l1 = la[is[1]] * r1;
+    lms[0] = -d.cdrho * lm[is[0]] * r0;
+    lms[1] = -d.cdrho * lm[is[1]] * r1;
+    lF[0] = l0 + l1;
+    lF[2] = (1.0 / 3.0) * lF[0];
+    lF[1] = 0.5 * (l1 - l0);
+    lF[3] = 0.25 * (l1 - l0);
+#pragma unroll
+    for (int n = 0; n < 4; n++) {
+      lD[0][n] += lF[n];
+      lD[1][n] += (0.5 * sg) * lF[n];
+      lD[2][n] += (1.0 / 3.0) * lF[n];
+      lD[3][n] += (0.25 * sg) * lF[n];
+    }
+#pragma unroll 1
+    for (int i = 0; i < 5; i++) {
+      const double r = 0.5 * cG5[i] + 0.5 * sg, wi = 0.25 * cW5[i];
+      double c[4];
+      det_row(D, r, c);
+      const double t0 = q0 + r * (q1 + r * q3), t1 = q2 + r * u[5];
+      double m0 = 0.0, m1 = 0.0, m2 = 0.0, Ls[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const double lw = wi * lms[k];
+        double tau[5], pre[5];
+#pragma unroll
+        for (int j = 0; j < 5; j++) {
+          const double s = 0.5 * g5p(j) + (k == 0 ? -0.5 : 0.5);
+          tau[j] = t0 + s * (t1 + s * t2);
+          pre[j] = j == 0 ? tau[0] : pre[j - 1] * tau[j];
+        }
+        double inv = 1.0 / pre[4];
+#pragma unroll
+        for (int j = 4; j >= 0; j--) {
+          const double s = 0.5 * g5p(j) + (k == 0 ? -0.5 : 0.5);
+          const double it = j > 0 ? inv * pre[j > 0 ? j - 1 : 0] : inv;
+          inv *= tau[j];
+          const double det = c[0] + s * (c[1] + s * (c[2] + s * c[3]));
+          const double ld = (lw * g5w(j)) * it, lt = -(ld * it) * det;
+          m0 += lt;
+          m1 += lt * s;
+          m2 += lt * (s * s);
+          Ls[0] += ld;
+          Ls[1] += ld * s;
+          Ls[2] += ld * (s * s);
+          Ls[3] += ld * (s * s * s);
+        }
+      }
+      lq[0] += m0;
+      lq[1] += r * m0;
+      lq[2] += m1;
+      lq[3] += (r * r) * m0;
+      lq[4] += m2;
+      lq[5] += r * m1;
+      double rp = 1.0;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+#pragma unroll
+        for (int n = 0; n < 4; n++) lD[k][n] += rp * Ls[n];
+        rp *= r;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) l.a[i][j] = l.b[i][j] = 0.0;
+  map_det_T(m, lD, l);
+  double lX[3][3], lY[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) lX[i][j] = lY[i][j] = 0.0;
+  map_coeffs_T(l.a, lX);
+  map_coeffs_T(l.b, lY);
+  const int A[9] = {0, 2, 2, 0, 1, 2, 1, 0, 1}, B[9] = {0, 0, 2, 2, 0, 1, 2, 1, 1};
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    a.pbuf[k * nq + iq] += lX[A[k]][B[k]];
+    a.pbuf[(9 + k) * nq + iq] += lY[A[k]][B[k]];
+  }
+  double *o = a.lU + e;
+  o[0] += lq[0];
+  o[nc] += lq[1] - G.rc * lq[0];
+  o[2 * nc] += lq[2] - G.sc * lq[0];
+  o[3 * nc] += b3 * lq[0] - G.rc * lq[1] + 0.5 * lq[3];
+  o[4 * nc] += b4 * lq[0] - G.sc * lq[2] + 0.5 * lq[4];
+  o[5 * nc] += b5 * lq[0] - G.sc * lq[1] - G.rc * lq[2] + lq[5];
+}

@@ -21,19 +21,18 @@ the step runs (the RHS pass takes the face integral from the corner pass's
 node partial sums):
 
   corner   U^(s), rc/sc/g19..g21, sub-cell masses, connectivity, x^(s),
-           ustar_prev -> 4 sub-cell corrections, 45 node partial sums
-  node     45 partial sums and 9 gather ids per quad, CSR offset, mask,
-           ustar_prev -> ustar
+           ustar_prev -> 4 sub-cell corrections, 27 node partial sums (3 a node)
+  node     27 partial sums and 9 gather ids per quad, CSR offset, mask,
+           ustar_prev -> ustar; after stage 1 the motion with it: x^n, x^(s) -> x^(s+1)
   dt       (stage 1) connectivity, cell averages, volume, x^(s), ustar
            -> two per-block minima
-  rhs      U^(s), U^n, M^-1, geometry, the 40 partial sums of the 8
+  rhs      U^(s), U^n, M^-1, geometry, the 24 partial sums of the 8
            boundary nodes, connectivity, x^(s), ustar (+ the 6 source
            moments on Taylor-Green) -> U^(s+1) (the M^-1 solve and RK
            combine are fused into every stage)
   src      (Taylor-Green) connectivity, geometry, x^(s) -> 6 source moments
-  persson  tau DOFs, mean velocity, geometry, mass, shape moments,
-           connectivity, x^(s) -> flag, physical centre, frame
-  nodes    x^n, x^(s), ustar -> x^(s+1), ustar_prev
+  persson  tau DOFs, geometry, connectivity, x^(s) -> flag
+  nodes    (stage 1) x^n, x^(s), ustar -> x^(s+1)
   geom     connectivity, x^(s) -> volume, centre node
 """
 from __future__ import annotations
@@ -61,13 +60,13 @@ def kernel_bytes(family: str, ncell: int, npoin: int, nstag: int = 3, source: bo
     CONN = 9 * 4          # ipqua row
     XY = 2 * W            # one node pair (x, y) or (u, v)
     fam = {
-        "corner": ncell * (U + GEO + 4 * W + CONN + 4 * W + 45 * W) + npoin * (XY + XY),
-        "node": ncell * (45 * W + 9 * 4) + npoin * (4 + 1 + XY + XY),
+        "corner": ncell * (U + GEO + 4 * W + CONN + 4 * W + 27 * W) + npoin * (XY + XY),
+        "node": ncell * (27 * W + 9 * 4) + npoin * (4 + 1 + XY + XY) + npoin * 3 * XY * (nstag - 1) // nstag,
         "dt": ncell * (CONN + 4 * W + W) + npoin * 2 * XY,
-        "rhs": ncell * (U + U + 16 * W + GEO + 40 * W + CONN + U + (6 * W if source else 0)) + npoin * 2 * XY,
+        "rhs": ncell * (U + U + 16 * W + GEO + 24 * W + CONN + U + (6 * W if source else 0)) + npoin * 2 * XY,
         "src": ncell * (CONN + GEO + 6 * W) + npoin * XY,
-        "persson": ncell * (6 * W + 2 * W + GEO + W + 9 * W + CONN + 4 + 2 * W + 4 * W) + npoin * XY,
-        "nodes": npoin * (3 * XY + 2 * XY),
+        "persson": ncell * (6 * W + GEO + CONN + 4) + npoin * XY,
+        "nodes": npoin * (3 * XY + XY),
         "geom": ncell * (CONN + W + XY) + npoin * XY,
     }
     return fam[family]
