@@ -31,14 +31,19 @@
 // barthlimit_sympre_quadlb writes only geoel(10), which this branch never
 // reads.  With order_exact the kernels keep the reference's expression and
 // summation order, so the build with --fmad=false reproduces the CPU
-// restatement bit for bit; the optimised form (order_exact 0) has its own
-// kernels, described in lag2d_p1_fast.cuh.
+// restatement bit for bit; the optimised plane form (order_exact 0: FAST) sums the
+// two faces of each corner before the node gather and the face integral, takes
+// the volume of the straight quad in closed form, evaluates the limiter function
+// with one division and writes the update from the RHS pass.  The optimised RZ
+// forms have kernels of their own, described in lag2d_p1_fast.cuh.
 //
 // Layout in HBM (0-based, structure of arrays):
 //   U[(q*3 + k)*ncell + e]        P1 DOF k of field q (tau, u, v, e)
 //   ipq[k*nquad + iq]             vertex k (0..3, counter-clockwise) of quad iq
 //   cf[(v*8 + f + 2*iv)*nquad+iq] corner-face coefficient v (m, m u, m v,
 //                                 sigma.n A x, y) of corner iv, face f
+//                                 (FAST: cf[(v*4 + iv)*nquad+iq], the two faces
+//                                 of corner iv summed)
 //   lim[k*ncell + e]              aflim(1), aflim(4), aflim(5), afvec(1,1),
 //                                 afvec(1,2), afvec(2,1), afvec(2,2)
 #include "lag2d_launch.cuh"
@@ -1808,61 +1813,57 @@ static void enqueue_rhs(Solver *s, int fuse, double alfa, int stage) {
   });
 }
 
-// the same passes of the optimised stage
 static bool behind(const Dev1 &d) { return d.nquad <= kBehindMax; }
+// the RZ passes of the optimised stage
 template <int GEO>
-static void fast_cell(Solver *s, const Dev1 &d, int stage, int itime) {
+static void rz_cell(Solver *s, const Dev1 &d, int stage, int itime) {
   launch(s, "cell", [&] {
     launch_behind(behind(d), k1f_cell<GEO>, nb(4 * d.nquad, kCellThreads), kCellThreads, 0, s->st, d, stage, itime);
   });
 }
 template <int GEO>
-static void fast_node(Solver *s, const Dev1 &d, bool move, double alfa) {
+static void rz_node(Solver *s, const Dev1 &d, bool move, double alfa) {
   launch(s, "node", [&] {
     launch_behind(behind(d), move ? k1f_node<GEO, true> : k1f_node<GEO, false>, nb(d.npoin, 64), 64, 0, s->st, d, alfa);
   });
 }
 template <int GEO>
-static void fast_rhs(Solver *s, const Dev1 &d, int fuse, double alfa, int last) {
+static void rz_rhs(Solver *s, const Dev1 &d, int fuse, double alfa, int last) {
   launch(s, "rhs", [&] {
     launch_behind(behind(d), k1f_rhs<GEO>, nb(d.nquad, kRhsThreads), kRhsThreads, 0, s->st, d, fuse, alfa, last);
   });
 }
-// Plane meshes of this many cells and more keep the order of operations of the
-// kernels above (their FAST form) instead of the closed-form moments.  The
-// limiter's absolute thresholds (1e-8 on slopes and on the strain rate) sit in the
-// foot of a wave, where some cells always are within rounding of them: on the
-// 1024 x 512 Sod mesh any change of rounding, an input's last bit included, comes
-// back as 1e-9 of the state within 10 steps (512 x 256: 4e-11), so runs of that
-// size stay comparable to the bit.  Below, the shorter chain of the fused kernels
-// decides (200 x 10: 98 -> 40 us a step with its launches; 1024 x 512: 853 us
-// before, 786 in this form, 670 with them).
-constexpr int kWideCells = 65536;
-static bool wide(const Solver *s) { return s->d.nrz == 0 && s->d.nquad >= kWideCells; }
-
-static void wide_cell(Solver *s, const Dev1 &d, int stage) {
+// The plane branch runs the kernels above in their FAST form on meshes of every size:
+// a limited slope is kept or dropped at absolute thresholds (1e-8 on slopes and on
+// the strain rate), which every cell of a flow that starts at rest crosses, so
+// another order of operations there (closed-form pressure moments, four lanes per
+// cell) comes back as 1e-9 to 1e-7 of the state within 60 steps on 200 x 10 and 30 on
+// 1024 x 512, and no result may depend on which form a mesh's size selects.
+// (200 x 10 83 us a step, in the other form 31; 1024 x 512 785 and 670.)
+static void plane_cell(Solver *s, const Dev1 &d, int stage) {
   launch(s, "bounds", [&] { k1_bounds<<<nb(d.npoin, 256), 256, 0, s->st>>>(d); });
   launch(s, "cell", [&] { launch_cell<0, true>(d, dim3(nb(d.nquad, 128)), dim3(128), s->st, stage); });
 }
-static void wide_node(Solver *s, const Dev1 &d, bool move, double alfa) {
+static void plane_node(Solver *s, const Dev1 &d, bool move, double alfa) {
   launch(s, "node", [&] { k1_node<true, 0><<<nb(d.npoin, 256), 256, 0, s->st>>>(d, move, alfa); });
 }
-static void wide_rhs(Solver *s, const Dev1 &d, int fuse, double alfa) {
+static void plane_rhs(Solver *s, const Dev1 &d, int fuse, double alfa) {
   launch(s, "rhs", [&] { launch_rhs<0, true>(d, dim3(nb(d.nquad, 128)), dim3(128), s->st, fuse, alfa); });
 }
 // the inner seam: RHS written, limiter coefficients in lim, no update
 template <int GEO>
 static void enqueue_rhs_fast(Solver *s) {
-  if (GEO == 0 && wide(s)) {
-    wide_cell(s, s->d, 1);
-    wide_node(s, s->d, false, 0.0);
-    wide_rhs(s, s->d, 0, 0.0);
-    return;
+  const Dev1 &d = s->d;
+  if constexpr (GEO == 0) {
+    plane_cell(s, d, 1);
+    plane_node(s, d, false, 0.0);
+    plane_rhs(s, d, 0, 0.0);
+  } else {
+    launch(s, "cell", [&] { k1f_pbar<<<nb(d.ncell, 128), 128, 0, s->st>>>(d, d.Us); });
+    rz_cell<GEO>(s, d, 1, 1);
+    rz_node<GEO>(s, d, false, 0.0);
+    rz_rhs<GEO>(s, d, 0, 0.0, 0);
   }
-  launch(s, "cell", [&] { k1f_pbar<<<nb(s->d.ncell, 128), 128, 0, s->st>>>(s->d, s->d.Us); });
-  fast_cell<GEO>(s, s->d, 1, 1);
-  fast_node<GEO>(s, s->d, false, 0.0);
-  fast_rhs<GEO>(s, s->d, 0, 0.0, 0);
 }
 template <int GEO>
 static void enqueue_step_fast(Solver *s, int itime) {
@@ -1884,13 +1885,12 @@ static void enqueue_step_fast(Solver *s, int itime) {
     d.Uo = last ? d0.Un : d0.Us;
     d.xo = last ? d0.xn : istag == 1 ? d0.xs : d0.xt;
     d.yo = last ? d0.yn : istag == 1 ? d0.ys : d0.yt;
-    const bool w = GEO == 0 && wide(s);
-    if (w) {
-      wide_cell(s, d, istag);
-      wide_node(s, d, istag > 1, alfa);
+    if constexpr (GEO == 0) {
+      plane_cell(s, d, istag);
+      plane_node(s, d, istag > 1, alfa);
     } else {
-      fast_cell<GEO>(s, d, istag, itime);
-      fast_node<GEO>(s, d, istag > 1, alfa);
+      rz_cell<GEO>(s, d, istag, itime);
+      rz_node<GEO>(s, d, istag > 1, alfa);
     }
     if (istag == 1) {
       launch(s, "dt", [&] { launch_behind(behind(d), behind(d) ? k1f_dt<GEO, true> : k1f_dt<GEO, false>, nb(d.nquad, 256), 256, 0, s->st, d, s->cfg.ndt, itime); });
@@ -1901,10 +1901,10 @@ static void enqueue_step_fast(Solver *s, int itime) {
       after(s1, s->st);
       launch(s, "geom", [&] { launch_geom(s, s1, d.xo, d.yo); });
     }
-    if (w) wide_rhs(s, d, 1, alfa);
-    else fast_rhs<GEO>(s, d, 1, alfa, last);
+    if constexpr (GEO == 0) plane_rhs(s, d, 1, alfa);
+    else rz_rhs<GEO>(s, d, 1, alfa, last);
     if (istag == 1 || last) after(s->st, s1);
-    if (w && last) launch(s, "copy", [&] { k1_step_end<<<1, 1, 0, s->st>>>(d); });
+    if (GEO == 0 && last) launch(s, "copy", [&] { k1_step_end<<<1, 1, 0, s->st>>>(d); });
   }
   s->stale = true;
 }
@@ -2168,7 +2168,7 @@ int init_fields(Solver *s, double *geoel, double *amatr, double *unkno, std::str
   Scalars s0{};
   CK1(cudaMemcpyAsync(d.sc_dev, &s0, sizeof(Scalars), cudaMemcpyHostToDevice, s->st));
   s->stale = false;
-  launch(s, "init", [&] { k1f_pbar<<<nb(ncell, 128), 128, 0, s->st>>>(d, d.Un); });
+  if (d.nrz) launch(s, "init", [&] { k1f_pbar<<<nb(ncell, 128), 128, 0, s->st>>>(d, d.Un); });
   geom(s, d.xn, d.yn);
   int r = read_status(s, err);
   if (r) return r;
@@ -2218,7 +2218,7 @@ int set_state(Solver *s, const double *unkno, const double *coord, const double 
   Scalars s0{};
   CK1(cudaMemcpyAsync(d.sc_dev, &s0, sizeof(Scalars), cudaMemcpyHostToDevice, s->st));
   s->stale = false;
-  launch(s, "copy", [&] { k1f_pbar<<<nb(ncell, 128), 128, 0, s->st>>>(d, d.Un); });
+  if (d.nrz) launch(s, "copy", [&] { k1f_pbar<<<nb(ncell, 128), 128, 0, s->st>>>(d, d.Un); });
   geom(s, d.xs, d.ys);
   return read_status(s, err);
 }

@@ -1,15 +1,16 @@
-// The optimised stage of the linear P1 path (order_exact 0), for the plane
-// branch (GEO 0) and both RZ forms (GEO 1: true volume, 2: area-weighted).
+// The optimised RZ stage of the linear P1 path (order_exact 0; GEO 1: true volume,
+// 2: area-weighted), and the time step, motion and volumes of the plane branch
+// (GEO 0), whose other passes are lag2d_p1.cu's FAST forms.
 // Included by lag2d_p1.cu inside namespace lag2d::p1; the reference-order kernels
 // beside it stay for order_exact.
 //
-// On the meshes this path is run on (2,000 to 10,000 cells) every kernel is one
+// On the meshes this path is run on (about 10,000 cells) every kernel is one
 // wave, so a step's time is launches times the dependent chain of a thread.  A
 // stage is three launches (cell, node, RHS) instead of seven to nine:
 //   cell  four lanes per cell, lane = vertex: node bounds over the cells around
-//         the vertex (no kernel of their own), limiter, corner coefficients; RZ
-//         mass centre and mass matrix with the quadrature rows spread over the
-//         lanes
+//         the vertex (no kernel of their own), limiter, corner coefficients;
+//         area-weighted: mass centre and mass matrix with the quadrature rows
+//         spread over the lanes
 //   node  gather, solve, walls, and the motion once dt is known
 //   RHS   one thread per cell: face and volume integral, M^-1 and the update
 // Stage 1 adds the time step (finished by its last block) and the motion, which
@@ -72,14 +73,12 @@ __device__ __forceinline__ double cell_volume(const Bilin &b) {
 
 // Face weights of corner iv's two edges (a to the previous vertex, b to the
 // next): the share own that weighs the corner's own basis and the share oth that
-// weighs the other end's, of the edge's area vector.  Plane: half each edge, own
-// basis (Limiterlag.f90:708-1033); nrz = 1: the radius weights of the four corner
-// faces (Getrhslagmc.f90:18534-18734); nrz = 2: (2 b_own + b_oth) / 6
+// weighs the other end's, of the edge's area vector.  nrz = 1: the radius weights of
+// the four corner faces (Getrhslagmc.f90:18534-18734); nrz = 2: (2 b_own + b_oth) / 6
 // (Getrhslagrz.f90:1673-1812).
 template <int GEO>
 __device__ __forceinline__ void edge_weights(double ri, double rj, double &own, double &oth) {
-  if (GEO == 0) { own = 0.5; oth = 0.0; }
-  else if (GEO == 1) { own = (1.0 / 12.0) * (3.0 * ri + rj); oth = (1.0 / 12.0) * (ri + rj); }
+  if (GEO == 1) { own = (1.0 / 12.0) * (3.0 * ri + rj); oth = (1.0 / 12.0) * (ri + rj); }
   else { own = 1.0 / 3.0; oth = 1.0 / 6.0; }
 }
 
@@ -88,7 +87,7 @@ __device__ __forceinline__ double pressure(double g, double tau, double u, doubl
 }
 
 // corner coefficients: rows cf[(row*4 + iv)*nquad + iq]; the node pass reads
-// 0-4, the RZ RHS 1-2 and 5-7, the plane RHS 0-4
+// 0-4, the RHS 1-2 and 5-7
 constexpr int CF_P0 = 0, CF_U = 1, CF_V = 2, CF_S1 = 3, CF_S2 = 4, CF_MA = 5, CF_MB = 6, CF_P = 7;
 
 // ---------------------------------------------------------------------------
@@ -184,7 +183,7 @@ __global__ void __launch_bounds__(kCellThreads) k1f_cell(Dev1 d, int stage, int 
   const int t = blockIdx.x * kCellThreads + threadIdx.x, iv = threadIdx.x & 3;
   const bool live = (t >> 2) < d.nquad;
   const int e = live ? t >> 2 : d.nquad - 1;  // lanes past the end repeat the last cell and store nothing
-  const size_t nc = d.ncell, np = d.npoin;
+  const size_t nc = d.ncell;
   const Scalars *S = d.sc_dev;
   const int p = d.ipq[iv * nc + e];
   const int b0 = d.esuv_ptr[p], b1 = d.esuv_ptr[p + 1];
@@ -314,7 +313,7 @@ __global__ void __launch_bounds__(kCellThreads) k1f_cell(Dev1 d, int stage, int 
     }
   }
   // (4) corner coefficients of vertex iv: edges a (from the previous vertex) and b
-  const double floor_ = GEO == 0 ? 1.0e-6 : GEO == 1 ? 1.0e-9 : 1.0e-8;
+  const double floor_ = GEO == 1 ? 1.0e-9 : 1.0e-8;
   const double pctr = pressure(g, tau0, uc, vc, ec, floor_);
   const double snd = sqrt(fmax(floor_, g * pctr * tau0)), rho = 1.0 / tau0;
   const double pl = pctr + af4 * (pressure(g, w[0], w[1], w[2], w[3], floor_) - pctr);
@@ -327,8 +326,7 @@ __global__ void __launch_bounds__(kCellThreads) k1f_cell(Dev1 d, int stage, int 
   const double dx = us0 - ul, dy = vs0 - vl, j2 = dx * dx + dy * dy;
   const double la = sqrt(ax * ax + ay * ay), lb = sqrt(bx * bx + by * by);
   const double da = fabs(dx * ax + dy * ay), db = fabs(dx * bx + dy * by);
-  const double kap = GEO == 0 ? d.cimpd * rho * (0.5 * (g + 1.0)) : 0.0;
-  double ma = rho * snd * la + kap * da, mb = rho * snd * lb + kap * db;
+  double ma = rho * snd * la, mb = rho * snd * lb;
   if (!(j2 < 1.0e24 * snd * snd)) {  // getriecoef_matrixnew's jump direction: times |n . du| / |du|
     const double rj = 1.0 / sqrt(j2);
     ma *= da / la * rj;
@@ -344,12 +342,9 @@ __global__ void __launch_bounds__(kCellThreads) k1f_cell(Dev1 d, int stage, int 
   o[CF_V * 4 * nc] = vl;
   o[CF_S1 * 4 * nc] = -pl * (ax * (oa + na) + bx * (ob + nb_));
   o[CF_S2 * 4 * nc] = -pl * (ay * (oa + na) + by * (ob + nb_));
-  if (GEO != 0) {
-    o[CF_MA * 4 * nc] = ma;
-    o[CF_MB * 4 * nc] = mb;
-    o[CF_P * 4 * nc] = pl;
-  }
-  (void)np;
+  o[CF_MA * 4 * nc] = ma;
+  o[CF_MB * 4 * nc] = mb;
+  o[CF_P * 4 * nc] = pl;
 }
 
 // ---------------------------------------------------------------------------
@@ -394,41 +389,37 @@ __global__ void __launch_bounds__(64) k1f_node(Dev1 d, double alfa) {
   for (int j = 0; j < 4; j++)
     if (b + j < en) corner_add(d, c[j], n);
   for (int i = b + 4; i < en; i++) corner_add(d, d.ncor[i], n);
-  double fx = 0.0, fy = 0.0;
-  if (GEO != 0) {
-    // boundary forces (getbc_lagmaire2, Getrhslag.f90:11269-11491; area-weighted:
-    // GetBClag.f90:57-250): the walls' area vectors (code 22), whose normal
-    // velocity the force removes, and the pressure of code 21 (ncase 3)
-    double bvx = 0.0, bvy = 0.0, bpx = 0.0, bpy = 0.0;
-    bool wall22 = false;
-    for (int i = d.bf_ptr[p]; i < d.bf_ptr[p + 1]; i++) {
-      const int f = d.bf_list[i], q0 = d.bfn[f], q1 = d.bfn[d.nbfac + f], code = d.bfcode[f];
-      const double x0 = d.xs[q0], y0 = d.ys[q0], x1 = d.xs[q1], y1 = d.ys[q1];
-      const double nx = y1 - y0, ny = x0 - x1, len = sqrt(nx * nx + ny * ny);
-      const double r0 = 1.0 - d.alfrz + d.alfrz * y0, r1 = 1.0 - d.alfrz + d.alfrz * y1;
-      const double w = GEO == 2 ? 0.5 : (q0 == p ? 2.0 * r0 + r1 : 2.0 * r1 + r0) / 6.0;
-      if (code / 1000 == 22) {
-        wall22 = true;
-        const int sub = code % 1000;
-        // outward axis of the wall; ncase 1 and 2 know both sides of the unit box
-        if (sub == 221) bvy += (((d.ncase == 1 || d.ncase == 2 || d.ncase == 12) && !(y0 < 1.0e-6 && y1 < 1.0e-6) &&
-                                 fabs(y0 - 1.0) < 1.0e-6 && fabs(y1 - 1.0) < 1.0e-6) ? w : -w) * len;
-        else if (sub == 222) bvx += ((d.ncase == 1 && !(x0 < 1.0e-6 && x1 < 1.0e-6) && fabs(x0 - 1.0) < 1.0e-6 &&
-                                      fabs(x1 - 1.0) < 1.0e-6) ? w : -w) * len;
-      } else if (code / 1000 == 21 && d.ncase == 3) {
-        bpx += 1.0e-6 * w * nx;
-        bpy += 1.0e-6 * w * ny;
-      }
+  // boundary forces (getbc_lagmaire2, Getrhslag.f90:11269-11491; area-weighted:
+  // GetBClag.f90:57-250): the walls' area vectors (code 22), whose normal
+  // velocity the force removes, and the pressure of code 21 (ncase 3)
+  double bvx = 0.0, bvy = 0.0, bpx = 0.0, bpy = 0.0;
+  bool wall22 = false;
+  for (int i = d.bf_ptr[p]; i < d.bf_ptr[p + 1]; i++) {
+    const int f = d.bf_list[i], q0 = d.bfn[f], q1 = d.bfn[d.nbfac + f], code = d.bfcode[f];
+    const double x0 = d.xs[q0], y0 = d.ys[q0], x1 = d.xs[q1], y1 = d.ys[q1];
+    const double nx = y1 - y0, ny = x0 - x1, len = sqrt(nx * nx + ny * ny);
+    const double r0 = 1.0 - d.alfrz + d.alfrz * y0, r1 = 1.0 - d.alfrz + d.alfrz * y1;
+    const double w = GEO == 2 ? 0.5 : (q0 == p ? 2.0 * r0 + r1 : 2.0 * r1 + r0) / 6.0;
+    if (code / 1000 == 22) {
+      wall22 = true;
+      const int sub = code % 1000;
+      // outward axis of the wall; ncase 1 and 2 know both sides of the unit box
+      if (sub == 221) bvy += (((d.ncase == 1 || d.ncase == 2 || d.ncase == 12) && !(y0 < 1.0e-6 && y1 < 1.0e-6) &&
+                               fabs(y0 - 1.0) < 1.0e-6 && fabs(y1 - 1.0) < 1.0e-6) ? w : -w) * len;
+      else if (sub == 222) bvx += ((d.ncase == 1 && !(x0 < 1.0e-6 && x1 < 1.0e-6) && fabs(x0 - 1.0) < 1.0e-6 &&
+                                    fabs(x1 - 1.0) < 1.0e-6) ? w : -w) * len;
+    } else if (code / 1000 == 21 && d.ncase == 3) {
+      bpx += 1.0e-6 * w * nx;
+      bpy += 1.0e-6 * w * ny;
     }
-    fx = bpx;
-    fy = bpy;
-    if (wall22) {
-      const double cl = (bvx * bvx + bvy * bvy) / n.m;
-      const double cr = ((n.a1 - n.s1 - bpx) * bvx + (n.a2 - n.s2 - bpy) * bvy) / n.m;
-      const double k = cr / fmax(1.0e-16, cl);
-      fx += k * bvx;
-      fy += k * bvy;
-    }
+  }
+  double fx = bpx, fy = bpy;
+  if (wall22) {
+    const double cl = (bvx * bvx + bvy * bvy) / n.m;
+    const double cr = ((n.a1 - n.s1 - bpx) * bvx + (n.a2 - n.s2 - bpy) * bvy) / n.m;
+    const double k = cr / fmax(1.0e-16, cl);
+    fx += k * bvx;
+    fy += k * bvy;
   }
   if (!(bc & BC_KEEP)) {
     us = (n.a1 - n.s1 - fx) / n.m;
@@ -522,7 +513,7 @@ __global__ void __launch_bounds__(256) k1f_dt(Dev1 d, int ndt, int itime) {
       const double dl = sqrt((x[k] - x[n]) * (x[k] - x[n]) + (y[k] - y[n]) * (y[k] - y[n]));
       if (k == 0 || dl < dlen) dlen = dl;
     }
-    if (GEO == 0) {
+    if constexpr (GEO == 0) {
       double fn[4][3];
 #pragma unroll
       for (int f = 0; f < 4; f++) {
@@ -541,15 +532,16 @@ __global__ void __launch_bounds__(256) k1f_dt(Dev1 d, int ndt, int itime) {
         const double l2x = c16 * b3 * fn[fb][0] * fn[fb][2], l2y = c16 * b3 * fn[fb][1] * fn[fb][2];
         dv = dv + us[iv] * (l1x + l2x) + vs[iv] * (l1y + l2y);
       }
-    } else
+    } else {
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int n = (k + 1) & 3;
-      const double nx = y[n] - y[k], ny = x[k] - x[n];
-      double o1, t1, o2, t2;
-      edge_weights<GEO>(fabs(y[k]), fabs(y[n]), o1, t1);
-      edge_weights<GEO>(fabs(y[n]), fabs(y[k]), o2, t2);
-      dv += (o1 + t1) * (us[k] * nx + vs[k] * ny) + (o2 + t2) * (us[n] * nx + vs[n] * ny);
+      for (int k = 0; k < 4; k++) {
+        const int n = (k + 1) & 3;
+        const double nx = y[n] - y[k], ny = x[k] - x[n];
+        double o1, t1, o2, t2;
+        edge_weights<GEO>(fabs(y[k]), fabs(y[n]), o1, t1);
+        edge_weights<GEO>(fabs(y[n]), fabs(y[k]), o2, t2);
+        dv += (o1 + t1) * (us[k] * nx + vs[k] * ny) + (o2 + t2) * (us[n] * nx + vs[n] * ny);
+      }
     }
     const double vol = cell_volume<GEO>(B);
     if (GEO == 2) dv = vol / (4.0 * B.j0) * dv + vc * (4.0 * B.j0);
@@ -691,32 +683,24 @@ __global__ void __launch_bounds__(kRhsThreads) k1f_rhs(Dev1 d, int fuse, double 
       const double ul = o[CF_U * 4 * nc], vl = o[CF_V * 4 * nc];
       const double dux = us[iv] - ul, duy = vs[iv] - vl;
       const double ax = y[iv] - y[vp], ay = x[vp] - x[iv], bx = y[vn] - y[iv], by = x[iv] - x[vn];
-      if (GEO == 0) {
-        const double P0 = o[CF_P0 * 4 * nc];
-        const double f0 = o[CF_S1 * 4 * nc] + P0 * dux, f1 = o[CF_S2 * 4 * nc] + P0 * duy;
-        const double tw = 0.5 * (us[iv] * (ax + bx) + vs[iv] * (ay + by)), fe = us[iv] * f0 + vs[iv] * f1;
-        R[0][0] += tw; R[0][1] += f0; R[0][2] += f1; R[0][3] += fe;
-        add(br, bs, tw, f0, f1, fe);
-      } else {
-        const double pl = o[CF_P * 4 * nc], ma = o[CF_MA * 4 * nc], mb = o[CF_MB * 4 * nc];
-        // edge a ends at the previous vertex, edge b at the next one
-        const double brp = bm[(vp == 1 || vp == 2) ? 1 : 0], bsp = cm[vp >= 2 ? 1 : 0];
-        const double brn = bm[(vn == 1 || vn == 2) ? 1 : 0], bsn = cm[vn >= 2 ? 1 : 0];
-        double oa, na, ob, nn;
-        edge_weights<GEO>(fabs(y[iv]), fabs(y[vp]), oa, na);
-        edge_weights<GEO>(fabs(y[iv]), fabs(y[vn]), ob, nn);
-        {
-          const double f0 = ma * dux - pl * ax, f1 = ma * duy - pl * ay;
-          const double tw = us[iv] * ax + vs[iv] * ay, fe = us[iv] * f0 + vs[iv] * f1, w = oa + na;
-          R[0][0] += w * tw; R[0][1] += w * f0; R[0][2] += w * f1; R[0][3] += w * fe;
-          add(oa * br + na * brp, oa * bs + na * bsp, tw, f0, f1, fe);
-        }
-        {
-          const double f0 = mb * dux - pl * bx, f1 = mb * duy - pl * by;
-          const double tw = us[iv] * bx + vs[iv] * by, fe = us[iv] * f0 + vs[iv] * f1, w = ob + nn;
-          R[0][0] += w * tw; R[0][1] += w * f0; R[0][2] += w * f1; R[0][3] += w * fe;
-          add(ob * br + nn * brn, ob * bs + nn * bsn, tw, f0, f1, fe);
-        }
+      const double pl = o[CF_P * 4 * nc], ma = o[CF_MA * 4 * nc], mb = o[CF_MB * 4 * nc];
+      // edge a ends at the previous vertex, edge b at the next one
+      const double brp = bm[(vp == 1 || vp == 2) ? 1 : 0], bsp = cm[vp >= 2 ? 1 : 0];
+      const double brn = bm[(vn == 1 || vn == 2) ? 1 : 0], bsn = cm[vn >= 2 ? 1 : 0];
+      double oa, na, ob, nn;
+      edge_weights<GEO>(fabs(y[iv]), fabs(y[vp]), oa, na);
+      edge_weights<GEO>(fabs(y[iv]), fabs(y[vn]), ob, nn);
+      {
+        const double f0 = ma * dux - pl * ax, f1 = ma * duy - pl * ay;
+        const double tw = us[iv] * ax + vs[iv] * ay, fe = us[iv] * f0 + vs[iv] * f1, w = oa + na;
+        R[0][0] += w * tw; R[0][1] += w * f0; R[0][2] += w * f1; R[0][3] += w * fe;
+        add(oa * br + na * brp, oa * bs + na * bsp, tw, f0, f1, fe);
+      }
+      {
+        const double f0 = mb * dux - pl * bx, f1 = mb * duy - pl * by;
+        const double tw = us[iv] * bx + vs[iv] * by, fe = us[iv] * f0 + vs[iv] * f1, w = ob + nn;
+        R[0][0] += w * tw; R[0][1] += w * f0; R[0][2] += w * f1; R[0][3] += w * fe;
+        add(ob * br + nn * brn, ob * bs + nn * bsn, tw, f0, f1, fe);
       }
     }
     // moments of the weight alone (closed form): 1, or y in nrz = 1
@@ -747,7 +731,7 @@ __global__ void __launch_bounds__(kRhsThreads) k1f_rhs(Dev1 d, int fuse, double 
       R[1][3] += h00 * Q00 + h10 * Q10 + h01 * Q01 + h20 * Q20 + h11 * Q11;
       R[2][3] += k00 * Q00 + k10 * Q10 + k01 * Q01 + k11 * Q11 + k02 * Q02;
     }
-    if (GEO != 0) {
+    {
       // moments of p det J (no radius weight): the sources
       const double d0 = B.j0 * M00 + B.j1 * M10 + B.j2 * M01;
       const double d1 = B.j0 * M10 + B.j1 * M20 + B.j2 * M11 - rc * d0;
