@@ -108,8 +108,8 @@ __device__ __forceinline__ double quad_get(double v, int lane) { return __shfl_s
 // cell-average density, is the area centroid) and M^-1 of the area mass matrix
 // about it over geoel(11) (25 points, :3949-4219).  tau along a row is linear, so
 // a row needs one division; the rows are spread over the cell's lanes.
-__device__ __forceinline__ void area_centre(const Dev1 &d, int e, int iv, const Bilin &B, double t0, double t1, double t2,
-                                            double &rc, double &sc) {
+__device__ __forceinline__ void area_centre(const Dev1 &d, int e, int iv, bool live, const Bilin &B, double t0, double t1,
+                                            double t2, double &rc, double &sc) {
   rc = B.j1 / (3.0 * B.j0);
   sc = B.j2 / (3.0 * B.j0);
   const double scale = t0 / (4.0 * B.j0);  // 1 / masel
@@ -171,6 +171,8 @@ __device__ __forceinline__ void area_centre(const Dev1 &d, int e, int iv, const 
   f1 = quad_sum(f1);
   f2 = quad_sum(f2);
   f3 = quad_sum(f3);
+  // the lanes past the end repeat the last cell, whose centre other warps may still read
+  if (!live) return;
   const double rb = cell_volume<2>(B) / (4.0 * B.j0), det = (f1 * f3 - f2 * f2) * rb;
   d.amatr[iv * (size_t)d.ncell + e] = iv == 0 ? f3 / det : iv == 1 ? -f2 / det : iv == 2 ? f1 / det : 1.0 / (f0 * rb);
   if (iv == 0) d.rc[e] = rc;
@@ -306,7 +308,7 @@ __global__ void __launch_bounds__(kCellThreads) k1f_cell(Dev1 d, int stage, int 
     // the stage's mass centre and mass matrix: every stage but the first of step 1
     if (stage > 1 || (itime < 0 ? now + 1 : itime) > 1) {
       const double t1 = md > 1 ? af1 * u[0][1] : 0.0, t2 = md > 2 ? af1 * u[0][2] : 0.0;
-      area_centre(d, e, iv, B, tau0, t1, t2, rc, sc);
+      area_centre(d, e, iv, live, B, tau0, t1, t2, rc, sc);
 #pragma unroll
       for (int q = 0; q < 4; q++)
         w[q] = u[q][0] + (md > 1 ? u[q][1] * (xi - rc) : 0.0) + (md > 2 ? u[q][2] * (eta - sc) : 0.0);
