@@ -810,6 +810,7 @@ int lag2d_set_rho0(lag2d_handle *h, const double *rho0) {
   if (!h) return fail(LAG2D_EINVAL, "null handle");
   if (h->p1) return fail(LAG2D_EUNSUP, "the initial-density hook is built for the P2 path");
   Dev &d = h->d;
+  const double *before = d.rho0;
   if (rho0) {
     for (int e = 0; e < d.ncell; e++)
       if (!(rho0[e] > 0.0)) return fail(LAG2D_EINVAL, "rho0 must be positive");
@@ -821,6 +822,11 @@ int lag2d_set_rho0(lag2d_handle *h, const double *rho0) {
     d.rho0 = h->rho0_dev;
   } else {
     d.rho0 = nullptr;
+  }
+  // the captured step holds the pointer by value: the next one captures anew
+  if (h->graph && d.rho0 != before) {
+    cudaGraphExecDestroy(h->graph);
+    h->graph = nullptr;
   }
   // the time-invariant reference-configuration masses lag2d_create computed
   // (sub-cell masses, mass-weighted shape moments) follow the new density
