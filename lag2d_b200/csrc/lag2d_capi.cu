@@ -922,7 +922,8 @@ static int get_scalars(lag2d_handle *h, Scalars *s) {
   return LAG2D_OK;
 }
 
-// one step with itime incremented on the device, captured once per handle
+// one step with itime incremented on the device, captured once per handle; not with
+// timing on, whose records cannot be replayed
 static int step_graph(lag2d_handle *h) {
   if (h->graph) return LAG2D_OK;
   cudaGraph_t g;
@@ -1545,13 +1546,18 @@ int lag2d_adjoint(lag2d_handle *h, int itime0, int nsteps, int checkpoint_every,
     return (double)t;
   };
   double t_fwd = 0, t_rec = 0, t_rev = 0;
-  // forward with a checkpoint at every segment start and at the end
+  // forward with a checkpoint at every segment start and at the end; with timing
+  // on launch by launch, as lag2d_step does
   r = put_scalars(h, itime0 - 1, *dtfix, *tacru);
   if (r) return r;
-  if ((r = step_graph(h))) return r;
+  if (!h->timing && (r = step_graph(h))) return r;
   cudaEventRecord(ev[0], h->st);
   for (int n = 0; n < nsteps; n++) {
     if (n % K == 0) ck.save(h, n / K);
+    if (h->timing) {
+      enqueue_step_fast(h, itime0 + n);
+      continue;
+    }
     CK(cudaGraphLaunch(h->graph, h->st));
     h->launches += h->graph_launches;
   }
