@@ -674,7 +674,7 @@ struct WenoShared {
   double unksl[9][4][6];
   double qinvm[4][16], qmat[4][16], os[4][9], wsum[4][4][6], fch[4][4][6], unkf[4][4][6];
   double phy[4][6], rhsuk[4][6], out[4][6];
-  double xt[9][2], csum[4][3];              // target's nodes as they are; sub-cell sums of the corrections
+  double xt[9][2], csum[4][2];              // target's nodes as they are; sub-cell areas and masses of the corrections
   int cell[9], fvalid[4];
 };
 
@@ -765,8 +765,8 @@ __device__ __forceinline__ double weno_hrhs(const WenoShared &S, int is, int km,
 // Reconstructs troubled-list entry t with the whole block; every thread of the
 // block calls it (the early return is block-uniform).  With FACT the factors
 // go to F and nothing is written to the state.  fixcorr: d.corr holds the
-// sub-cell density corrections of the state before WENO; those of the target are
-// moved to its new tau moments.
+// sub-cell density corrections of the state before WENO; the target's are replaced
+// by those of its new moments.
 template <bool FACT>
 __device__ bool weno_block_cell(const Dev &d, int t, WenoShared &S, WenoFactors *F, int fixcorr = 0) {
   const int tid = threadIdx.x;
@@ -1160,8 +1160,8 @@ __device__ bool weno_block_cell(const Dev &d, int t, WenoShared &S, WenoFactors 
   }
   __syncthreads();
   if (fixcorr) {
-    // corr = cdrho (rho0 V0 / V - (sum w det / tau) / V) per sub-cell: only the
-    // harmonic sum depends on the moments (getrhosubg_daverg)
+    // getrhosubg_averg / _daverg of the limited moments, from those alone: the raw tau
+    // of a troubled quad may pass zero at one of the points
     if (tid < 100) {
       const int isg = tid / 25, ig = tid - 25 * isg;
       const double r = 0.5 * (cQ.g25[ig][0] + (isg == 0 || isg == 3 ? -1.0 : 1.0));
@@ -1169,29 +1169,25 @@ __device__ bool weno_block_cell(const Dev &d, int t, WenoShared &S, WenoFactors 
       double dr[9], ds[9];
       shp9d(r, s, dr, ds);
       const Jac j = jac9(S.xt, dr, ds);
-      const double det = cQ.w25[ig] * (j.xr * j.ys - j.yr * j.xs);
+      const double det = 0.25 * cQ.w25[ig] * (j.xr * j.ys - j.yr * j.xs);
       const double b1 = r - S.geo[0][0], b2 = s - S.geo[0][1];
       const double b[6] = {1.0, b1, b2, 0.5 * b1 * b1 - S.geo[0][2], 0.5 * b2 * b2 - S.geo[0][3], b1 * b2 - S.geo[0][4]};
-      double told = S.unkrl[0][0][0], tnew = told;
+      double tau = S.unkrl[0][0][0];
 #pragma unroll
-      for (int k = 1; k < 6; k++) {
-        told += S.unkrl[0][0][k] * b[k];
-        tnew += S.out[0][k] * b[k];
-      }
+      for (int k = 1; k < 6; k++) tau += S.out[0][k] * b[k];
       S.rhodj[tid] = det;
-      S.xl[tid] = det / told;
-      S.yl[tid] = det / tnew;
+      S.xl[tid] = det / tau;
     }
     __syncthreads();
-    if (tid < 12) {
-      const int isg = tid / 3, m = tid - 3 * isg;
-      const double *v = (m == 0 ? S.rhodj : m == 1 ? S.xl : S.yl) + 25 * isg;
+    if (tid < 8) {
+      const int isg = tid >> 1, m = tid & 1;
+      const double *v = (m == 0 ? S.rhodj : S.xl) + 25 * isg;
       double acc = 0.0;
       for (int i = 0; i < 25; i++) acc += v[i];
       S.csum[isg][m] = acc;
     }
     __syncthreads();
-    if (tid < 4) d.corr[tid * nq + iq] += d.cdrho * (S.csum[tid][1] - S.csum[tid][2]) / S.csum[tid][0];
+    if (tid < 4) d.corr[tid * nq + iq] = d.cdrho * (d.msub[tid * nq + iq] - S.csum[tid][1]) / S.csum[tid][0];
     __syncthreads();
   }
   return true;
