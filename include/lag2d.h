@@ -171,10 +171,13 @@ void *lag2d_stream(const lag2d_handle *h);
 /* Number of this library's kernel launches since the handle was created. */
 long long lag2d_kernel_launches(const lag2d_handle *h);
 
-/* Average device time (ms) per launch of the named kernel family over the
- * launches timed since lag2d_timing(h, 1); families: "corner", "node",
- * "rhs", "update", "persson", "weno", "nodes", "geom", "dt".  Returns -1
- * when timing is off or the family is unknown. */
+/* Average device time (ms) per pass of the named kernel family, all kernels of
+ * the pass together (corner: sub-cell corrections and corner faces, of quads and
+ * triangles), over the passes timed since lag2d_timing(h, 1), whose number goes to
+ * launches; families: "corner", "node", "rhs", "update", "persson", "weno",
+ * "nodes", "geom", "dt", "src" and, on the linear path, "bounds" and "cell".  The
+ * optimised step updates in "rhs" and, after stage 1, moves the nodes in "node".
+ * Returns -1 when timing is off or the family is unknown. */
 int lag2d_timing(lag2d_handle *h, int enable);
 double lag2d_kernel_ms(const lag2d_handle *h, const char *family, long long *launches);
 

@@ -102,6 +102,12 @@ struct Family {
   double ms = 0.0;
   long long n = 0;
 };
+// a timed piece of a pass; a pass of several pieces counts once
+struct Record {
+  std::string family;
+  cudaEvent_t a, b;
+  int passes;
+};
 
 struct lag2d_handle {
   Dev d{};
@@ -125,7 +131,7 @@ struct lag2d_handle {
   long long launches = 0;
   bool timing = false;
   std::map<std::string, Family> fam;
-  std::vector<std::pair<std::string, std::pair<cudaEvent_t, cudaEvent_t>>> pending;
+  std::vector<Record> pending;
   p1::Solver *p1 = nullptr;    // the linear P1 path (npoly = 1) when set; Dev d is then unused
   double *errpart = nullptr;   // per-block partial sums of lag2d_error_norms
   double *cellout = nullptr;   // [9][ncell] values of lag2d_cell_output
@@ -257,9 +263,10 @@ static double now_ms_event(cudaEvent_t a, cudaEvent_t b) {
 }
 
 // Launch helper: counts launches and, when timing is on, brackets the
-// launch with events on the handle's stream.
+// launch with events on the handle's stream.  passes = 0: a piece of a pass whose
+// other piece is counted.
 template <typename F>
-static void run(lag2d_handle *h, const char *family, F &&f, int nlaunch = 1) {
+static void run(lag2d_handle *h, const char *family, F &&f, int nlaunch = 1, int passes = 1) {
   cudaEvent_t a = nullptr, b = nullptr;
   if (h->timing) {
     cudaEventCreate(&a);
@@ -270,18 +277,18 @@ static void run(lag2d_handle *h, const char *family, F &&f, int nlaunch = 1) {
   h->launches += nlaunch;
   if (h->timing) {
     cudaEventRecord(b, h->st);
-    h->pending.push_back({family, {a, b}});
+    h->pending.push_back({family, a, b, passes});
   }
 }
 
 static void flush_timing(lag2d_handle *h) {
   for (auto &p : h->pending) {
-    cudaEventSynchronize(p.second.second);
-    Family &f = h->fam[p.first];
-    f.ms += now_ms_event(p.second.first, p.second.second);
-    f.n += 1;
-    cudaEventDestroy(p.second.first);
-    cudaEventDestroy(p.second.second);
+    cudaEventSynchronize(p.b);
+    Family &f = h->fam[p.family];
+    f.ms += now_ms_event(p.a, p.b);
+    f.n += p.passes;
+    cudaEventDestroy(p.a);
+    cudaEventDestroy(p.b);
   }
   h->pending.clear();
 }
@@ -439,17 +446,17 @@ static void enqueue_step_fast(lag2d_handle *h, int itime, const StageRec *rec = 
     }
     if (T) {
       after(s2, s0);
-      run(h, "corner", [&] { launch_fast_tri_corner(d, s2); });
+      run(h, "corner", [&] { launch_fast_tri_corner(d, s2); }, 1, 0);
     }
     if (!mixed) {
       after(s1, s0);
-      run(h, "corner", [&] { launch_fast_corr(d, s1); });
+      run(h, "corner", [&] { launch_fast_corr(d, s1); }, 1, 0);
     }
     run(h, "persson", [&] { launch_fast_persson(d, s0); });
     after(s0, s1);
     run(h, "weno", [&] { launch_weno_block(d, s0, !mixed); });
     if (mixed) {
-      run(h, "weno", [&] { launch_weno_swap(d, s0); });
+      run(h, "weno", [&] { launch_weno_swap(d, s0); }, 1, 0);
       run(h, "corner", [&] { launch_mixed_corner(d, s0); }, 2);
     } else {
       run(h, "corner", [&] { launch_fast_faces(d, s0); });
@@ -471,10 +478,10 @@ static void enqueue_step_fast(lag2d_handle *h, int itime, const StageRec *rec = 
     run(h, "geom", [&] { launch_tri_geom(dx, s2, dx.xs, dx.ys); launch_fast_geom(dx, s2, 1); }, 1 + T);
     if (T) {
       after(s1, s0);
-      run(h, "rhs", [&] { launch_fast_tri_rhs(d, s1, d.us_new, d.vs_new, 1, alfa); });
+      run(h, "rhs", [&] { launch_fast_tri_rhs(d, s1, d.us_new, d.vs_new, 1, alfa); }, 1, 0);
     }
     run(h, "rhs", [&] { launch_rhs_quads(h, d, s0, 1, alfa); });
-    if (mixed && istag == 1) run(h, "weno", [&] { launch_weno_swap(d, s0); });
+    if (mixed && istag == 1) run(h, "weno", [&] { launch_weno_swap(d, s0); }, 1, 0);
     if (T) after(s0, s1);
     after(s0, s2);
     if (has_src(d) && istag < nstag) {
@@ -1618,7 +1625,7 @@ void lag2d_destroy(lag2d_handle *h) {
   if (!h) return;
   if (h->p1) p1::destroy(h->p1);
   if (h->st) cudaStreamSynchronize(h->st);
-  for (auto &p : h->pending) { cudaEventDestroy(p.second.first); cudaEventDestroy(p.second.second); }
+  for (auto &p : h->pending) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
   if (h->graph) cudaGraphExecDestroy(h->graph);
   if (h->fork) cudaEventDestroy(h->fork);
   for (cudaStream_t q : h->side)

@@ -1859,7 +1859,7 @@ static void enqueue_rhs_fast(Solver *s) {
     plane_node(s, d, false, 0.0);
     plane_rhs(s, d, 0, 0.0);
   } else {
-    launch(s, "cell", [&] { k1f_pbar<<<nb(d.ncell, 128), 128, 0, s->st>>>(d, d.Us); });
+    launch(s, "init", [&] { k1f_pbar<<<nb(d.ncell, 128), 128, 0, s->st>>>(d, d.Us); });
     rz_cell<GEO>(s, d, 1, 1);
     rz_node<GEO>(s, d, false, 0.0);
     rz_rhs<GEO>(s, d, 0, 0.0, 0);
@@ -2218,7 +2218,7 @@ int set_state(Solver *s, const double *unkno, const double *coord, const double 
   Scalars s0{};
   CK1(cudaMemcpyAsync(d.sc_dev, &s0, sizeof(Scalars), cudaMemcpyHostToDevice, s->st));
   s->stale = false;
-  if (d.nrz) launch(s, "copy", [&] { k1f_pbar<<<nb(ncell, 128), 128, 0, s->st>>>(d, d.Un); });
+  if (d.nrz) launch(s, "init", [&] { k1f_pbar<<<nb(ncell, 128), 128, 0, s->st>>>(d, d.Un); });
   geom(s, d.xs, d.ys);
   return read_status(s, err);
 }
