@@ -127,6 +127,7 @@ struct lag2d_handle {
   cudaEvent_t fork = nullptr;
   bool forking = false;
   cudaGraphExec_t graph = nullptr;
+  long long direct_steps = 0;  // launched one by one, before the step was captured
   long long graph_launches = 0;
   long long launches = 0;
   bool timing = false;
@@ -633,15 +634,6 @@ int lag2d_create(const lag2d_mesh *m, const lag2d_config *c, lag2d_handle **out)
     lag2d_destroy(h);
     return fail(LAG2D_ECUDA, std::string("kernel attributes: ") + cudaGetErrorString(attr_err));
   }
-  for (cudaStream_t &q : h->side)
-    if (cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) != cudaSuccess) {
-      lag2d_destroy(h);
-      return fail(LAG2D_ECUDA, "cudaStreamCreate failed");
-    }
-  if (cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming) != cudaSuccess) {
-    lag2d_destroy(h);
-    return fail(LAG2D_ECUDA, "cudaEventCreate failed");
-  }
   const int nq = m->nquad, np = m->npoin;
   // ---- connectivity
   std::vector<int> ipq(9 * (size_t)nq), esq(4 * (size_t)nq), sten;
@@ -721,7 +713,8 @@ int lag2d_create(const lag2d_mesh *m, const lag2d_config *c, lag2d_handle **out)
   A(&d.vol, ncell); A(&d.vcx, ncell); A(&d.vcy, ncell); A(&d.msub, 4 * (size_t)nq);
   A(&d.Un, NU * (size_t)ncell); A(&d.Us, NU * (size_t)ncell);
   A(&d.xn, np); A(&d.yn, np); A(&d.xs, np); A(&d.ys, np); A(&d.us, np); A(&d.vs, np);
-  A(&d.amatr, 16 * (size_t)ncell); A(&d.rhs, NU * (size_t)ncell); A(&d.cf, 5 * 32 * (size_t)nq);
+  A(&d.amatr, 16 * (size_t)ncell); A(&d.rhs, NU * (size_t)ncell);
+  if (c->order_exact) A(&d.cf, 5 * 32 * (size_t)nq);
   A(&d.flag, ncell); A(&d.geoph, 2 * (size_t)ncell); A(&d.mapmt, 4 * (size_t)ncell);
   A(&d.Uw, 20 * (size_t)nq); A(&d.wlist, nq); A(&d.wcount, 4); A(&d.xt, np); A(&d.yt, np);
   A(&d.dtpart, 2 * (size_t)dt_blocks(d) + 2); A(&d.sc_dev, 1); A(&h->flags_dev, ncell);
@@ -933,6 +926,9 @@ static int get_scalars(lag2d_handle *h, Scalars *s) {
 // timing on, whose records cannot be replayed
 static int step_graph(lag2d_handle *h) {
   if (h->graph) return LAG2D_OK;
+  for (cudaStream_t &q : h->side)
+    if (!q) CK(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+  if (!h->fork) CK(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
   const long long before = h->launches;
@@ -949,19 +945,35 @@ static int step_graph(lag2d_handle *h) {
   return LAG2D_OK;
 }
 
+// How a call's steps go out: one by one with timing on and for a handle's first
+// kDirectSteps, else as replays of the captured step.  Capturing and instantiating it
+// costs 0.9 ms and releasing it 0.6, which replays gain back at 40 us a step (16 x 16;
+// 1024 x 1024 50 us): a handle of a few steps does not get there.  First step of a
+// handle 0.14 ms (captured at once 0.79), a fresh handle's run of 10 1.1 ms (1.35).
+constexpr long long kDirectSteps = 16;
+static int launch_mode(lag2d_handle *h, int nsteps, bool &direct) {
+  direct = h->timing || (!h->graph && h->direct_steps + nsteps <= kDirectSteps);
+  if (!direct) return step_graph(h);
+  if (!h->timing) h->direct_steps += nsteps;
+  return LAG2D_OK;
+}
+static int launch_step(lag2d_handle *h, int itime, bool direct) {
+  if (direct) {
+    enqueue_step(h, itime);
+    return LAG2D_OK;
+  }
+  CK(cudaGraphLaunch(h->graph, h->st));
+  h->launches += h->graph_launches;
+  return LAG2D_OK;
+}
+
 int lag2d_step(lag2d_handle *h, int itime, double *dtfix, double *tacru) {
   if (!h || !dtfix || !tacru) return fail(LAG2D_EINVAL, "null argument");
   if (h->p1) P1_CALL(p1::step(h->p1, itime, dtfix, tacru, err_));
-  // a replay of the captured step; with timing on, launch by launch
   int r = put_scalars(h, itime - 1, *dtfix, *tacru);
   if (r) return r;
-  if (h->timing) {
-    enqueue_step(h, itime);
-  } else {
-    if ((r = step_graph(h))) return r;
-    CK(cudaGraphLaunch(h->graph, h->st));
-    h->launches += h->graph_launches;
-  }
+  bool direct;
+  if ((r = launch_mode(h, 1, direct)) || (r = launch_step(h, itime, direct))) return r;
   if (!h->cfg.order_exact) h->stale = true;
   Scalars s;
   r = get_scalars(h, &s);
@@ -977,27 +989,18 @@ int lag2d_run(lag2d_handle *h, int itime0, int nsteps, double *dtfix, double *ta
   if (h->p1) P1_CALL(p1::run(h->p1, itime0, nsteps, dtfix, tacru, done, err_));
   int r = put_scalars(h, itime0 - 1, *dtfix, *tacru);
   if (r) return r;
-  int steps = 0;
-  if (h->timing) {
-    // timed path: no graph, events around every kernel family
-    for (int i = 0; i < nsteps; i++) { enqueue_step(h, itime0 + i); steps++; }
-    flush_timing(h);
-  } else {
-    if ((r = step_graph(h))) return r;
-    const long long per_step = h->graph_launches;
-    for (int i = 0; i < nsteps; i++) {
-      CK(cudaGraphLaunch(h->graph, h->st));
-      h->launches += per_step;
-      steps++;
-    }
-  }
-  if (steps && !h->cfg.order_exact) h->stale = true;
+  bool direct;
+  if ((r = launch_mode(h, nsteps, direct))) return r;
+  for (int i = 0; i < nsteps; i++)
+    if ((r = launch_step(h, itime0 + i, direct))) return r;
+  if (h->timing) flush_timing(h);
+  if (nsteps && !h->cfg.order_exact) h->stale = true;
   Scalars s;
   r = get_scalars(h, &s);
   if (r) return r;
   *dtfix = s.dtfix;
   *tacru = s.tacru;
-  if (done) *done = s.done ? std::min(steps, std::max(0, s.itime - itime0 + 1)) : steps;
+  if (done) *done = s.done ? std::min(nsteps, std::max(0, s.itime - itime0 + 1)) : nsteps;
   return status_of(s);
 }
 
@@ -1553,20 +1556,15 @@ int lag2d_adjoint(lag2d_handle *h, int itime0, int nsteps, int checkpoint_every,
     return (double)t;
   };
   double t_fwd = 0, t_rec = 0, t_rev = 0;
-  // forward with a checkpoint at every segment start and at the end; with timing
-  // on launch by launch, as lag2d_step does
+  // forward with a checkpoint at every segment start and at the end
   r = put_scalars(h, itime0 - 1, *dtfix, *tacru);
   if (r) return r;
-  if (!h->timing && (r = step_graph(h))) return r;
+  bool direct;
+  if ((r = launch_mode(h, nsteps, direct))) return r;
   cudaEventRecord(ev[0], h->st);
   for (int n = 0; n < nsteps; n++) {
     if (n % K == 0) ck.save(h, n / K);
-    if (h->timing) {
-      enqueue_step_fast(h, itime0 + n);
-      continue;
-    }
-    CK(cudaGraphLaunch(h->graph, h->st));
-    h->launches += h->graph_launches;
+    if ((r = launch_step(h, itime0 + n, direct))) return r;
   }
   h->stale = true;
   ck.save(h, nseg);

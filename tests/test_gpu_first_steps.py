@@ -1,0 +1,64 @@
+"""A handle's first steps are launched one by one and later ones replayed: the same bits
+whichever way the steps are cut into calls, also across the change, and a first step that
+does not pay for a capture."""
+import time
+
+import numpy as np
+import pytest
+
+from lag2d_b200 import workload
+from lag2d_b200.config import StepConfig
+from lag2d_b200.mesh import hybrid_mesh, quad_mesh
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(kind):
+    c = StepConfig(ncase=1, gamlg=5.0 / 3.0, nstag=3, cfl=0.02, tend=10.0)
+    if kind in ("quads", "mixed", "exact"):
+        return quad_mesh(16, 13, jitter=0.05), c
+    if kind == "hybrid":
+        c.ndt, c.dtfix = 0, 1.0e-4
+        return hybrid_mesh(9, 8), c
+    return workload(kind)
+
+
+@pytest.mark.parametrize("kind", ["quads", "mixed", "exact", "hybrid", "sedov16", "sod40", "noh_rz8", "noh_rzaw8"])
+def test_cuts(kind):
+    from lag2d_b200.api import Lag2DSolver
+    m, c = _case(kind)
+    got = []
+    for cut in ((24,), (1,) * 24, (15, 9), (16, 8), (3, 21)):
+        s = Lag2DSolver(m, c, precision=int(kind == "mixed"), order_exact=kind == "exact")
+        s.init_fields()
+        for n in cut:
+            if n == 1:
+                s.step()
+            else:
+                assert s.run(n) == n
+        got.append(s.get_state() + (s.dtfix, s.tacru))
+        s.close()
+    for g in got[1:]:
+        for a, b in zip(g, got[0]):
+            assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("kind", ["quads", "mixed", "sod40"])
+def test_first_step_is_no_capture(kind):
+    """A captured first step took 4 to 8 later ones, one launched by itself takes 1.2 to
+    1.5: medians over handles, and a limit between."""
+    from lag2d_b200.api import Lag2DSolver
+    m, c = _case(kind)
+    first, later = [], []
+    for _ in range(9):
+        s = Lag2DSolver(m, c, precision=int(kind == "mixed"))
+        s.init_fields()
+        t = time.perf_counter()
+        s.step()
+        first.append(time.perf_counter() - t)
+        s.run(30)
+        t = time.perf_counter()
+        s.step()
+        later.append(time.perf_counter() - t)
+        s.close()
+    assert np.median(first) < 2.5 * np.median(later)
