@@ -8,13 +8,13 @@
 //    36 node cross products x_i y_j - x_j y_i (lag2d_tables.inc);
 //  * det J at fixed points (sub-cell densities, source) comes from its bicubic
 //    coefficients, built from those of the quad's map (lag2d_cell.cuh);
-//  * Jacobians on the 5x5 Gauss-Lobatto grid are sum-factorised on the 3x3
-//    tensor of quad nodes;
+//  * Jacobians on the 5x5 Gauss-Lobatto grid come from the same coefficients,
+//    a polynomial in s along each row;
 //  * the corner pass reduces its 32 corner faces to per-node partial sums
-//    (9 nodes x 5 values) that the node pass gathers in cell order, and the
-//    RHS pass recomputes the cheap corner data instead of reading it back;
-//  * in RK stages 2 and 3 the mass-matrix solve and RK combine are fused into
-//    the RHS pass.
+//    (9 nodes x 3 values) that the node pass gathers in cell order and the RHS
+//    pass reads back in place of the corner data;
+//  * the mass-matrix solve and RK combine are fused into the RHS pass of every
+//    stage.
 #include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 #include "lag2d_launch.cuh"
@@ -406,7 +406,7 @@ __device__ void f_node(const Dev &d, int p, double alfa) {
 
 // ---------------------------------------------------------------------------
 // RHS pass: corner forces + face integral + volume integral (+ source), and
-// in stages 2 and 3 the M^-1 solve and RK combine
+// the M^-1 solve and RK combine of the stage
 // ---------------------------------------------------------------------------
 
 // The momentum and energy face weights of rhsifacedg_lagsubgq2 are 1 on every
@@ -464,7 +464,7 @@ __host__ __device__ __forceinline__ void mass_flux_weights(const Loaded &L, int 
 // affine in u*: sum_f F_f = u* P0 - (P1, P2), where P0..P2 are the node partial
 // sums the corner pass wrote (sum m, sum m u_k - sigma.n A w); the energy
 // term is u* . sum_f F_f; the mass term is u* . t with t the sum of 2 w_mass,f
-// an_f over the node's outer corner faces (node_flux).  So the corner data are
+// an_f over the node's outer corner faces (corner_flux, edge_flux).  So the corner data are
 // not recomputed here: 24 partials and the 8 boundary nodes' velocities replace
 // the 32 corner faces' vertex states, impedances and forces (same sums up to
 // rounding and summation order).  The nodes sit at -1, 0, 1 in r and s, so the
@@ -486,8 +486,8 @@ __host__ __device__ __forceinline__ void mass_flux_weights(const Loaded &L, int 
 // load latency overlaps the face integral and they are read from shared
 // memory where used instead of being held in registers.
 //
-// 1024 x 1024: 341 -> 270 us a launch (65% of the copy rate, FP64 pipe 40%, 8 warps
-// an SM by its 254 registers); 256 x 256 29 -> 24.5.  Rows unrolled, 152 bytes of
+// 1024 x 1024: 341 -> 270 us a launch (68% of the copy rate by what it reads and writes
+// once, 64% by the DRAM counters; 8 warps an SM by its 254 registers); 256 x 256 29 -> 24.5.  Rows unrolled, 152 bytes of
 // spills: 8% slower a step.  The map's coefficients in shared memory in place of
 // U^n, which is then copied after the rows: 289.
 constexpr int kRhsBlock = 64;
@@ -1117,11 +1117,11 @@ __host__ __device__ void a_corner_faces(const Dev &d, const Adj &a, int iq) {
 }
 
 // Second part: the transpose of the sub-cell density corrections
-// corr = cdrho (msub / vsub - masel / volel) from their adjoints in lcorr;
+// corr = cdrho (msub / vsub - masel / volel) from their adjoints in lcorr, its point
+// arithmetic in FP32 (the FP32-mixed adjoint's; the FP64 one runs k_a_corr64);
 // adds into the tau DOF adjoints and the node-coordinate contributions.
 // The corrections come from the forward pass; the sub-cell masses masel
 // are recovered from them and the closed-form volumes volel.
-template <typename R>
 __host__ __device__ void a_corner_corr(const Dev &d, const Adj &a, int iq) {
   if (iq >= d.nquad) return;
   const int e = iq + d.ntria;
@@ -1182,19 +1182,19 @@ __host__ __device__ void a_corner_corr(const Dev &d, const Adj &a, int iq) {
       for (int n = 0; n < 4; n++) ee[n] = D[n] + r * (D[4 + n] + r * (D[8 + n] + r * D[12 + n]));
       const double t0 = u0[0] + u0[1] * dr + u0[3] * (0.5 * dr * dr - G.g19) - u0[4] * G.g20 - u0[5] * G.g21;
       const double t1 = u0[2] + u0[5] * dr, t2 = 0.5 * u0[4];
-      // point arithmetic in R (FP32 in the mixed adjoint), rows added in FP64
-      const R t0r = R(t0), t1r = R(t1), t2r = R(t2), lm = R(lmasel), wi = R(0.25 * g5w(i));
-      const R e0 = R(ee[0]), e1 = R(ee[1]), e2 = R(ee[2]), e3 = R(ee[3]);
-      R m0 = 0, m1 = 0, m2 = 0, Ls[4] = {0, 0, 0, 0};
+      // point arithmetic in float (FP32 in the mixed adjoint), rows added in FP64
+      const float t0r = float(t0), t1r = float(t1), t2r = float(t2), lm = float(lmasel), wi = float(0.25 * g5w(i));
+      const float e0 = float(ee[0]), e1 = float(ee[1]), e2 = float(ee[2]), e3 = float(ee[3]);
+      float m0 = 0, m1 = 0, m2 = 0, Ls[4] = {0, 0, 0, 0};
 #pragma unroll
       for (int j = 0; j < 5; j++) {
         const double sd = (g5p(j) + ofs) / 2.0;
-        const R s = R(sd), ds = R(sd - G.sc);
-        const R tau = t0r + ds * (t1r + t2r * ds);
-        const R det = e0 + s * (e1 + s * (e2 + s * e3));
-        const R itau = R(1) / tau;
-        const R ldet = lm * (wi * R(g5w(j))) * itau;
-        const R ltau = -ldet * det * itau;
+        const float s = float(sd), ds = float(sd - G.sc);
+        const float tau = t0r + ds * (t1r + t2r * ds);
+        const float det = e0 + s * (e1 + s * (e2 + s * e3));
+        const float itau = float(1) / tau;
+        const float ldet = lm * (wi * float(g5w(j))) * itau;
+        const float ltau = -ldet * det * itau;
         m0 += ltau;
         m1 += ltau * ds;
         m2 += ltau * ds * ds;
@@ -1238,10 +1238,8 @@ __host__ __device__ void a_corner_corr(const Dev &d, const Adj &a, int iq) {
 // cofactor form), row by row: the DOFs along a row are a_q + ds (b_q + c_q ds),
 // and the transposed sums over a row collapse to per-row moments (sum l,
 // sum l ds, sum l ds^2 for the DOF adjoints; sum l L_b(s), sum l L_b'(s) for
-// the node adjoints).  R = double for the FP64 adjoint; R = float for the
-// FP32-mixed one, where the point arithmetic and the per-row moments are FP32
-// and the rows are added into the FP64 adjoints.
-template <typename R>
+// the node adjoints).  The point arithmetic and the per-row moments are FP32, the rows
+// are added into the FP64 adjoints.  (The FP64 adjoint runs k_a_rhs64.)
 __host__ __device__ __forceinline__ void vol_T(const Loaded &L, const CellGeo &G, const double u[4][6],
                                                const double lR[4][6], double g, double eps, double lu[4][6],
                                                double lX[3][3], double lY[3][3]) {
@@ -1251,87 +1249,87 @@ __host__ __device__ __forceinline__ void vol_T(const Loaded &L, const CellGeo &G
     double lr[3], dlr[3];
     lag3(r, lr);
     dlag3(r, dlr);
-    R Qx[3], Qy[3], Px[3], Py[3];
+    float Qx[3], Qy[3], Px[3], Py[3];
 #pragma unroll
     for (int bb = 0; bb < 3; bb++) {
-      Qx[bb] = R(dlr[0] * L.X[0][bb] + dlr[1] * L.X[1][bb] + dlr[2] * L.X[2][bb]);
-      Qy[bb] = R(dlr[0] * L.Y[0][bb] + dlr[1] * L.Y[1][bb] + dlr[2] * L.Y[2][bb]);
-      Px[bb] = R(lr[0] * L.X[0][bb] + lr[1] * L.X[1][bb] + lr[2] * L.X[2][bb]);
-      Py[bb] = R(lr[0] * L.Y[0][bb] + lr[1] * L.Y[1][bb] + lr[2] * L.Y[2][bb]);
+      Qx[bb] = float(dlr[0] * L.X[0][bb] + dlr[1] * L.X[1][bb] + dlr[2] * L.X[2][bb]);
+      Qy[bb] = float(dlr[0] * L.Y[0][bb] + dlr[1] * L.Y[1][bb] + dlr[2] * L.Y[2][bb]);
+      Px[bb] = float(lr[0] * L.X[0][bb] + lr[1] * L.X[1][bb] + lr[2] * L.X[2][bb]);
+      Py[bb] = float(lr[0] * L.Y[0][bb] + lr[1] * L.Y[1][bb] + lr[2] * L.Y[2][bb]);
     }
-    R ra[4], rb[4], rc2[4];
+    float ra[4], rb[4], rc2[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      ra[q] = R(u[q][0] + u[q][1] * dr + u[q][3] * (0.5 * dr * dr - G.g19) - u[q][4] * G.g20 - u[q][5] * G.g21);
-      rb[q] = R(u[q][2] + u[q][5] * dr);
-      rc2[q] = R(0.5 * u[q][4]);
+      ra[q] = float(u[q][0] + u[q][1] * dr + u[q][3] * (0.5 * dr * dr - G.g19) - u[q][4] * G.g20 - u[q][5] * G.g21);
+      rb[q] = float(u[q][2] + u[q][5] * dr);
+      rc2[q] = float(0.5 * u[q][4]);
     }
-    R lR1[4][5];
+    float lR1[4][5];
 #pragma unroll
     for (int q = 0; q < 4; q++)
 #pragma unroll
-      for (int kk = 0; kk < 5; kk++) lR1[q][kk] = R(lR[q][kk + 1]);
-    R m0[4] = {0, 0, 0, 0}, m1[4] = {0, 0, 0, 0}, m2[4] = {0, 0, 0, 0};
-    R Mxr[3] = {0, 0, 0}, Mxs[3] = {0, 0, 0}, Myr[3] = {0, 0, 0}, Mys[3] = {0, 0, 0};
-    const R wi = R(l5w(i)), drr = R(dr), gm1 = R(g - 1.0), epsr = R(eps), half = R(0.5), one = R(1);
+      for (int kk = 0; kk < 5; kk++) lR1[q][kk] = float(lR[q][kk + 1]);
+    float m0[4] = {0, 0, 0, 0}, m1[4] = {0, 0, 0, 0}, m2[4] = {0, 0, 0, 0};
+    float Mxr[3] = {0, 0, 0}, Mxs[3] = {0, 0, 0}, Myr[3] = {0, 0, 0}, Mys[3] = {0, 0, 0};
+    const float wi = float(l5w(i)), drr = float(dr), gm1 = float(g - 1.0), epsr = float(eps), half = float(0.5), one = float(1);
 #pragma unroll 1
     for (int j = 0; j < 5; j++) {
-      const R ds = R(l5p(j) - G.sc);
+      const float ds = float(l5p(j) - G.sc);
       double lsd[3], dlsd[3];
       lag3(l5p(j), lsd);
       dlag3(l5p(j), dlsd);
-      const R ls[3] = {R(lsd[0]), R(lsd[1]), R(lsd[2])}, dls[3] = {R(dlsd[0]), R(dlsd[1]), R(dlsd[2])};
-      const R w = wi * R(l5w(j));
-      const R xr = Qx[0] * ls[0] + Qx[1] * ls[1] + Qx[2] * ls[2];
-      const R yr = Qy[0] * ls[0] + Qy[1] * ls[1] + Qy[2] * ls[2];
-      const R xs = Px[0] * dls[0] + Px[1] * dls[1] + Px[2] * dls[2];
-      const R ys = Py[0] * dls[0] + Py[1] * dls[1] + Py[2] * dls[2];
-      R un[4];
+      const float ls[3] = {float(lsd[0]), float(lsd[1]), float(lsd[2])}, dls[3] = {float(dlsd[0]), float(dlsd[1]), float(dlsd[2])};
+      const float w = wi * float(l5w(j));
+      const float xr = Qx[0] * ls[0] + Qx[1] * ls[1] + Qx[2] * ls[2];
+      const float yr = Qy[0] * ls[0] + Qy[1] * ls[1] + Qy[2] * ls[2];
+      const float xs = Px[0] * dls[0] + Px[1] * dls[1] + Px[2] * dls[2];
+      const float ys = Py[0] * dls[0] + Py[1] * dls[1] + Py[2] * dls[2];
+      float un[4];
 #pragma unroll
       for (int q = 0; q < 4; q++) un[q] = ra[q] + ds * (rb[q] + rc2[q] * ds);
-      const R rhoad = one / un[0];
-      const R kin = un[3] - half * (un[1] * un[1] + un[2] * un[2]);
-      const R pe = gm1 * rhoad * kin;
-      const R pres = pe > epsr ? pe : epsr;
-      R gd0[5], gd1[5];
+      const float rhoad = one / un[0];
+      const float kin = un[3] - half * (un[1] * un[1] + un[2] * un[2]);
+      const float pe = gm1 * rhoad * kin;
+      const float pres = pe > epsr ? pe : epsr;
+      float gd0[5], gd1[5];
       gd0[0] = ys;        gd1[0] = -xs;
       gd0[1] = -yr;       gd1[1] = xr;
       gd0[2] = ys * drr;  gd1[2] = -xs * drr;
       gd0[3] = -yr * ds;  gd1[3] = xr * ds;
       gd0[4] = ys * ds - yr * drr;
       gd1[4] = -xs * ds + xr * drr;
-      const R wp = w * pres;
-      R lgd0[5], lgd1[5], lwp = 0, lun1 = 0, lun2 = 0;
+      const float wp = w * pres;
+      float lgd0[5], lgd1[5], lwp = 0, lun1 = 0, lun2 = 0;
 #pragma unroll
       for (int kk = 0; kk < 5; kk++) {
-        const R fv = gd0[kk] * un[1] + gd1[kk] * un[2];
-        const R lfv = -lR1[0][kk] * w + lR1[3][kk] * wp;
+        const float fv = gd0[kk] * un[1] + gd1[kk] * un[2];
+        const float lfv = -lR1[0][kk] * w + lR1[3][kk] * wp;
         lwp += lR1[3][kk] * fv + lR1[1][kk] * gd0[kk] + lR1[2][kk] * gd1[kk];
         lgd0[kk] = lR1[1][kk] * wp + lfv * un[1];
         lgd1[kk] = lR1[2][kk] * wp + lfv * un[2];
         lun1 += lfv * gd0[kk];
         lun2 += lfv * gd1[kk];
       }
-      const R lpres = lwp * w;
-      R lun0 = 0, lun3 = 0;
+      const float lpres = lwp * w;
+      float lun0 = 0, lun3 = 0;
       if (pe > epsr) {
-        const R lrhoad = lpres * gm1 * kin;
+        const float lrhoad = lpres * gm1 * kin;
         lun3 += lpres * gm1 * rhoad;
         lun1 -= lpres * gm1 * rhoad * un[1];
         lun2 -= lpres * gm1 * rhoad * un[2];
         lun0 += -lrhoad * rhoad * rhoad;
       }
-      const R lunq[4] = {lun0, lun1, lun2, lun3};
+      const float lunq[4] = {lun0, lun1, lun2, lun3};
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         m0[q] += lunq[q];
         m1[q] += lunq[q] * ds;
         m2[q] += lunq[q] * ds * ds;
       }
-      const R lys = lgd0[0] + lgd0[2] * drr + lgd0[4] * ds;
-      const R lyr = -lgd0[1] - lgd0[3] * ds - lgd0[4] * drr;
-      const R lxs = -lgd1[0] - lgd1[2] * drr - lgd1[4] * ds;
-      const R lxr = lgd1[1] + lgd1[3] * ds + lgd1[4] * drr;
+      const float lys = lgd0[0] + lgd0[2] * drr + lgd0[4] * ds;
+      const float lyr = -lgd0[1] - lgd0[3] * ds - lgd0[4] * drr;
+      const float lxs = -lgd1[0] - lgd1[2] * drr - lgd1[4] * ds;
+      const float lxr = lgd1[1] + lgd1[3] * ds + lgd1[4] * drr;
 #pragma unroll
       for (int b2 = 0; b2 < 3; b2++) {
         Mxr[b2] += lxr * ls[b2];
@@ -1461,7 +1459,6 @@ __host__ __device__ __forceinline__ void src_T(const Loaded &L, const CellGeo &G
 // from lR adds into lU, writes pbuf (x, y, u*_prev = 0, v*_prev = 0, u*_new,
 // v*_new) and the adjoints of the node partial sums the face integral reads
 // (lP, consumed by a_corner).
-template <typename R>
 __host__ __device__ void a_rhs(const Dev &d, const Adj &a, int iq) {
   if (iq >= d.nquad) return;
   const int e = iq + d.ntria;
@@ -1479,7 +1476,7 @@ __host__ __device__ void a_rhs(const Dev &d, const Adj &a, int iq) {
   for (int q = 0; q < 4; q++) for (int k = 0; k < 6; k++) lu[q][k] = 0.0;
   double lX[3][3], lY[3][3];
   for (int i = 0; i < 3; i++) for (int j = 0; j < 3; j++) { lX[i][j] = 0.0; lY[i][j] = 0.0; }
-  // ---- face integral (f_rhs3): transpose of f = u* P0 - (P1, P2),
+  // ---- face integral: transpose of f = (P3, P4) + u* P0 - (P1, P2),
   // fe = u* . f, tw = u* . t per boundary node; the adjoints of the node
   // partial sums go to a.lP for the corner pass's transpose, those of
   // u* to pbuf, those of the mass-flux weights t to the face vectors
@@ -1497,14 +1494,8 @@ __host__ __device__ void a_rhs(const Dev &d, const Adj &a, int iq) {
     mass_flux_weights(L, k, tx, ty);
     const double P0 = d.npart[(0 * 9 + k) * nq + iq], P1 = d.npart[(1 * 9 + k) * nq + iq];
     const double P2 = d.npart[(2 * 9 + k) * nq + iq];
-    double f0, f1;
-    if (d.nrow == 3) {
-      f0 = un * P0 - P1;
-      f1 = vn * P0 - P2;
-    } else {
-      f0 = d.npart[(3 * 9 + k) * nq + iq] + (un * P0 - P1);
-      f1 = d.npart[(4 * 9 + k) * nq + iq] + (vn * P0 - P2);
-    }
+    const double f0 = d.npart[(3 * 9 + k) * nq + iq] + (un * P0 - P1);
+    const double f1 = d.npart[(4 * 9 + k) * nq + iq] + (vn * P0 - P2);
     double ltw = 0, lf0 = 0, lf1 = 0, lfe = 0;
     for (int kk = 0; kk < 6; kk++) {
       ltw += lR[0][kk] * b[kk];
@@ -1532,7 +1523,7 @@ __host__ __device__ void a_rhs(const Dev &d, const Adj &a, int iq) {
           corner_an_T(isg, ivsg, f, ltx * (2.0 * wmas(isg, ivsg, f)), lty * (2.0 * wmas(isg, ivsg, f)), lX, lY);
     }
   }
-  vol_T<R>(L, G, u, lR, g, eps, lu, lX, lY);
+  vol_T(L, G, u, lR, g, eps, lu, lX, lY);
   // the DOF adjoints are complete: out before the source's transpose
   for (int q = 0; q < 4; q++)
     for (int k = 0; k < 6; k++) a.lU[(q * 6 + k) * nc + e] += lu[q][k];
@@ -1786,21 +1777,16 @@ __global__ void k_nodes2(Dev d, double alfa) {
 __global__ void k_geom2(Dev d, int fix) { f_geom(d, blockIdx.x * blockDim.x + threadIdx.x, fix); }
 __global__ void k_init_wmom(Dev d) { f_init_wmom(d, blockIdx.x * blockDim.x + threadIdx.x); }
 
-// resident blocks of 128 per SM the reverse corner and RHS kernels are
-// compiled for: 3 (168 registers) in the FP32-mixed adjoint (reverse sweep
-// 15.65 -> 15.08 ms per step on the 1024x1024 Taylor-Green mesh), 1 (255)
-// in the FP64 one (3 would cost 12%)
-template <typename R>
-constexpr int arev_minb() { return sizeof(R) == 4 ? LAG2D_AREVF_MINB : 1; }
+// The reverse passes of the FP32-mixed adjoint.  The RHS one is compiled for 3 resident
+// blocks of 128 per SM (168 registers): reverse sweep 15.65 -> 15.08 ms per step on the
+// 1024x1024 Taylor-Green mesh.
 __global__ void __launch_bounds__(128, LAG2D_ACF_MINB) k_a_corner_faces(Dev d, Adj a) {
   a_corner_faces(d, a, blockIdx.x * blockDim.x + threadIdx.x);
 }
-template <typename R>
 __global__ void __launch_bounds__(128, LAG2D_ACC_MINB) k_a_corner_corr(Dev d, Adj a) {
-  a_corner_corr<R>(d, a, blockIdx.x * blockDim.x + threadIdx.x);
+  a_corner_corr(d, a, blockIdx.x * blockDim.x + threadIdx.x);
 }
-template <typename R>
-__global__ void __launch_bounds__(128, arev_minb<R>()) k_a_rhs(Dev d, Adj a) { a_rhs<R>(d, a, blockIdx.x * blockDim.x + threadIdx.x); }
+__global__ void __launch_bounds__(128, LAG2D_AREVF_MINB) k_a_rhs(Dev d, Adj a) { a_rhs(d, a, blockIdx.x * blockDim.x + threadIdx.x); }
 __global__ void k_a_gather(Dev d, Adj a, int nv) { a_gather(d, a, blockIdx.x * blockDim.x + threadIdx.x, nv); }
 __global__ void k_a_gather_solve(Dev d, Adj a) { a_gather_solve(d, a, blockIdx.x * blockDim.x + threadIdx.x); }
 __global__ void k_a_update(Dev d, Adj a, double alfa, const double *dtp, int fold) {
@@ -1838,13 +1824,13 @@ void launch_adjoint_stage(const Dev &d, const void *adj, cudaStream_t st, double
   fast::k_a_centre<<<bp, 256, 0, st>>>(d, a);
   fast::k_a_nodes<<<bp, 256, 0, st>>>(d, a, alfa, dtp, fold);
   fast::k_a_update<<<bc, 256, 0, st>>>(d, a, alfa, dtp, fold_u);
-  if (mixed) fast::k_a_rhs<float><<<bq, 128, 0, st>>>(d, a);
+  if (mixed) fast::k_a_rhs<<<bq, 128, 0, st>>>(d, a);
   else fast::k_a_rhs64<<<fast::nb(d.nquad, fast::kRevBlock), fast::kRevBlock, 0, st>>>(d, a);
   launch_tri_adjoint_rhs(d, a, st);
   fast::k_a_gather_solve<<<bp, 256, 0, st>>>(d, a);
   if (mixed) fast::k_a_corner_faces<<<bq, 128, 0, st>>>(d, a);
   else fast::k_a_faces4<<<fast::nb(4 * d.nquad, fast::kRevFaceBlock), fast::kRevFaceBlock, 0, st>>>(d, a);
-  if (mixed) fast::k_a_corner_corr<float><<<bq, 128, 0, st>>>(d, a);
+  if (mixed) fast::k_a_corner_corr<<<bq, 128, 0, st>>>(d, a);
   else fast::k_a_corr64<<<fast::nb(d.nquad, fast::kRevCorrBlock), fast::kRevCorrBlock, 0, st>>>(d, a);
   launch_tri_adjoint_corner(d, a, st);
   fast::k_a_gather<<<bp, 256, 0, st>>>(d, a, 4);
@@ -1862,9 +1848,10 @@ void launch_fast_corr(const Dev &d, cudaStream_t st) {
 // thread's chain; one thread per quad from where the chip is full several times
 // over and the lanes' repeated loads and centre state count.
 // Faces, us a step with one thread and with four lanes: 16 x 16 88 / 73, 64 x 64
-// 98 / 82, 128 x 128 110 / 100, 256 x 256 206 / 204, 512 x 512 704 / 696,
-// 1024 x 1024 2531 / 2566.
-constexpr int kFaces4Max = 131072;
+// 98 / 82, 128 x 128 110 / 100, 256 x 256 206 / 204; with the present passes 363 x 363
+// 392 / 392, 400 x 400 457 / 452, 512 x 512 696 / 711, 640 x 640 1049 / 1076,
+// 1024 x 1024 2498 / 2606.  The line is that of the passes launched behind one another.
+constexpr int kFaces4Max = kBehindMax;
 // RHS (255 registers either way): 16 x 16 73 / 69, 64 x 64 82 / 77, 128 x 128
 // 100 / 102, 256 x 256 204 / 236, so one wave of its blocks on 148 SMs.
 constexpr int kRhs4Max = 148 * 4 * (fast::kRhs4Block / 4);

@@ -1,5 +1,5 @@
 // The reverse of the FP64 RHS pass, one thread per quad.  Included by lag2d_fast.cu
-// inside namespace lag2d::fast.  (The FP32-mixed adjoint keeps a_rhs<float>, whose
+// inside namespace lag2d::fast.  (The FP32-mixed adjoint keeps a_rhs, whose
 // sums keep their bits.)
 //
 // The transposes of f_rhs3 and f_tgv_src in the same terms: every equation adds
