@@ -13,6 +13,7 @@
 
 #include "lag2d.h"
 #include "lag2d_device.cuh"
+#include "lag2d_launch.cuh"
 #include "lag2d_p1.h"
 
 namespace lag2d {
@@ -945,23 +946,23 @@ static int step_graph(lag2d_handle *h) {
   return LAG2D_OK;
 }
 
-// How a call's steps go out: one by one with timing on and for a handle's first
-// kDirectSteps, else as replays of the captured step.  Capturing and instantiating it
-// costs 0.9 ms and releasing it 0.6, which replays gain back at 40 us a step (16 x 16;
-// 1024 x 1024 50 us): a handle of a few steps does not get there.  First step of a
-// handle 0.14 ms (captured at once 0.79), a fresh handle's run of 10 1.1 ms (1.35).
-constexpr long long kDirectSteps = 16;
-static int launch_mode(lag2d_handle *h, int nsteps, bool &direct) {
-  direct = h->timing || (!h->graph && h->direct_steps + nsteps <= kDirectSteps);
-  if (!direct) return step_graph(h);
-  if (!h->timing) h->direct_steps += nsteps;
-  return LAG2D_OK;
-}
-static int launch_step(lag2d_handle *h, int itime, bool direct) {
-  if (direct) {
+// Step i of a call of nsteps: launched kernel by kernel with timing on and for a handle's
+// first steps, else a replay of the captured step.  Capturing and instantiating it costs
+// 0.9 ms and releasing it 0.6, which replays gain back at 40 us a step (16 x 16; 1024 x
+// 1024 50 us): a handle of a few steps does not get there.  First step of a handle 0.14 ms
+// (captured at once 0.79), a fresh handle's run of 10 1.0 ms (1.35).  A call of several
+// steps that goes past them launches its first one directly too, so that the capture
+// runs while the device works; from kBehindMax quads on one step covers most of it.
+static int launch_step(lag2d_handle *h, int itime, int i, int nsteps) {
+  const long long direct = h->d.nquad > kBehindMax ? 1 : 16;
+  const bool few = h->direct_steps + (nsteps - i) <= direct, cover = i == 0 && nsteps > 1;
+  if (h->timing || (!h->graph && (few || cover))) {
+    if (!h->timing) h->direct_steps++;
     enqueue_step(h, itime);
     return LAG2D_OK;
   }
+  const int r = step_graph(h);
+  if (r) return r;
   CK(cudaGraphLaunch(h->graph, h->st));
   h->launches += h->graph_launches;
   return LAG2D_OK;
@@ -972,8 +973,7 @@ int lag2d_step(lag2d_handle *h, int itime, double *dtfix, double *tacru) {
   if (h->p1) P1_CALL(p1::step(h->p1, itime, dtfix, tacru, err_));
   int r = put_scalars(h, itime - 1, *dtfix, *tacru);
   if (r) return r;
-  bool direct;
-  if ((r = launch_mode(h, 1, direct)) || (r = launch_step(h, itime, direct))) return r;
+  if ((r = launch_step(h, itime, 0, 1))) return r;
   if (!h->cfg.order_exact) h->stale = true;
   Scalars s;
   r = get_scalars(h, &s);
@@ -989,10 +989,8 @@ int lag2d_run(lag2d_handle *h, int itime0, int nsteps, double *dtfix, double *ta
   if (h->p1) P1_CALL(p1::run(h->p1, itime0, nsteps, dtfix, tacru, done, err_));
   int r = put_scalars(h, itime0 - 1, *dtfix, *tacru);
   if (r) return r;
-  bool direct;
-  if ((r = launch_mode(h, nsteps, direct))) return r;
   for (int i = 0; i < nsteps; i++)
-    if ((r = launch_step(h, itime0 + i, direct))) return r;
+    if ((r = launch_step(h, itime0 + i, i, nsteps))) return r;
   if (h->timing) flush_timing(h);
   if (nsteps && !h->cfg.order_exact) h->stale = true;
   Scalars s;
@@ -1559,12 +1557,10 @@ int lag2d_adjoint(lag2d_handle *h, int itime0, int nsteps, int checkpoint_every,
   // forward with a checkpoint at every segment start and at the end
   r = put_scalars(h, itime0 - 1, *dtfix, *tacru);
   if (r) return r;
-  bool direct;
-  if ((r = launch_mode(h, nsteps, direct))) return r;
   cudaEventRecord(ev[0], h->st);
   for (int n = 0; n < nsteps; n++) {
     if (n % K == 0) ck.save(h, n / K);
-    if ((r = launch_step(h, itime0 + n, direct))) return r;
+    if ((r = launch_step(h, itime0 + n, n, nsteps))) return r;
   }
   h->stale = true;
   ck.save(h, nseg);

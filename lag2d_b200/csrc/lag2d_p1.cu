@@ -2239,24 +2239,26 @@ static int step_graph(Solver *s, std::string &err) {
   return LAG2D_OK;
 }
 
-// nsteps steps: one by one with timing on and for a handle's first kDirectSteps, else as
-// replays of the captured step, which costs 0.35 ms to set up and gains 20 us a step
-// (200 x 10, RZ 100 x 100)
+// nsteps steps: kernel by kernel with timing on and for a handle's first kDirectSteps, else
+// as replays of the captured step, which costs 0.35 ms to set up and gains 20 us a step
+// (200 x 10, RZ 100 x 100); a call of several steps that goes past them launches its
+// first one directly too, so that the capture runs while the device works
 constexpr long long kDirectSteps = 16;
 static int advance(Solver *s, int itime0, int nsteps, double *dtfix, double *tacru, Scalars &sc, std::string &err) {
   int r = put_scalars(s, itime0 - 1, *dtfix, *tacru, err);
   if (r) return r;
-  if (s->timing || (!s->graph && s->direct_steps + nsteps <= kDirectSteps)) {
-    for (int i = 0; i < nsteps; i++) enqueue_step(s, itime0 + i);
-    if (s->timing) flush_timing(s);
-    else s->direct_steps += nsteps;
-  } else {
-    if ((r = step_graph(s, err))) return r;
-    for (int i = 0; i < nsteps; i++) {
-      CK1(cudaGraphLaunch(s->graph, s->st));
-      s->launches += s->graph_launches;
+  for (int i = 0; i < nsteps; i++) {
+    const bool few = s->direct_steps + (nsteps - i) <= kDirectSteps, cover = i == 0 && nsteps > 1;
+    if (s->timing || (!s->graph && (few || cover))) {
+      if (!s->timing) s->direct_steps++;
+      enqueue_step(s, itime0 + i);
+      continue;
     }
+    if ((r = step_graph(s, err))) return r;
+    CK1(cudaGraphLaunch(s->graph, s->st));
+    s->launches += s->graph_launches;
   }
+  if (s->timing) flush_timing(s);
   if (nsteps && !s->cfg.order_exact) s->stale = true;
   CK1(cudaMemcpyAsync(&sc, s->d.sc_dev, sizeof(Scalars), cudaMemcpyDeviceToHost, s->st));
   CK1(cudaStreamSynchronize(s->st));
