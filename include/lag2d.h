@@ -58,7 +58,9 @@ typedef struct {
   int ncase;            /* initial-condition / source case               */
   int nlimi, ndens;
   int ngausd, ngausd_geo;
-  int precision;        /* 0: FP64; 1: FP32-mixed corner/RHS arithmetic  */
+  int precision;        /* 0: FP64; 1: FP32-mixed corner/RHS arithmetic
+                           (on B200 not the faster one: 3.24 ms a step
+                           against 2.49 on 1024 x 1024)              */
   int order_exact;      /* 1: kernels that keep the reference's loop and
                            summation order (bit-identical to the CPU
                            restatement in the no-FMA build); 0: optimised */
@@ -109,7 +111,8 @@ int lag2d_step(lag2d_handle *h, int itime, double *dtfix, double *tacru);
 /* nsteps steps of the driver loop (dgflo2d.f90:358-472) with no host
  * synchronisation in between; stops early (on the device) once
  * |tacru - tend| / tend <= 1e-11 as the driver does (dgflo2d.f90:459).
- * *done receives the number of steps taken.  Captured in a CUDA graph. */
+ * *done receives the number of steps taken.  Replays a captured CUDA graph
+ * after a handle's first steps. */
 int lag2d_run(lag2d_handle *h, int itime0, int nsteps, double *dtfix, double *tacru, int *done);
 
 /* Download the state; any pointer may be NULL. geoel(24,nsize) receives the

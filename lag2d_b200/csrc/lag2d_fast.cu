@@ -486,8 +486,8 @@ __host__ __device__ __forceinline__ void mass_flux_weights(const Loaded &L, int 
 // load latency overlaps the face integral and they are read from shared
 // memory where used instead of being held in registers.
 //
-// 1024 x 1024: 341 -> 270 us a launch (68% of the copy rate by what it reads and writes
-// once, 64% by the DRAM counters; 8 warps an SM by its 254 registers); 256 x 256 29 -> 24.5.  Rows unrolled, 152 bytes of
+// 1024 x 1024: 341 -> 270 us a launch (69% of the copy rate by what it reads and writes
+// once, 64% by the DRAM counters; FP64 pipe 41%, 8 warps an SM by its 254 registers); 256 x 256 29 -> 24.5.  Rows unrolled, 152 bytes of
 // spills: 8% slower a step.  The map's coefficients in shared memory in place of
 // U^n, which is then copied after the rows: 289.
 constexpr int kRhsBlock = 64;

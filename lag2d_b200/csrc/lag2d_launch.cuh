@@ -20,8 +20,8 @@ __device__ __forceinline__ void await_previous() {
 
 // Meshes of up to this many cells use it.  us a step without / with: P2 16 x 16
 // 71 / 64, 64 x 64 78 / 71, 128 x 128 102 / 92, 256 x 256 205 / 194, Sedov
-// 128 x 128 149 / 139, linear 200 x 10 37 / 34, RZ 100 x 100 47 / 42; with the
-// integrals that need no u* ahead of the wait 63, 68, 88, 194, 138, 31, 40.  On a mesh that
+// 128 x 128 149 / 139, RZ 100 x 100 47 / 42; with the integrals that need no u* ahead
+// of the wait 63, 68, 88, 194, 138, 40.  On a mesh that
 // fills the chip many times the waiting blocks take room from the side passes
 // (1024 x 1024 2501 / 2555).
 constexpr int kBehindMax = 131072;
